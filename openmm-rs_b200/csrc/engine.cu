@@ -856,6 +856,10 @@ void Engine::setup_gbsa(const GbsaObcDef& g) {
   a.periodic = g.method == 2;
   a.use_cutoff = g.method != 0;
   a.cutoff = g.cutoff;
+  if (a.use_cutoff) {
+    a.block_box = mem_.alloc<float4>(2 * (size_t)blocks);
+    a.skip2 = (float)(g.cutoff * g.cutoff * (1.0 + 1e-4));
+  }
   const size_t rs = dp_ ? 8 : 4;
   a.posq = mem_.alloc_bytes(4 * rs * a.n_slots);
   a.params = mem_.alloc_bytes(2 * rs * a.n_slots);

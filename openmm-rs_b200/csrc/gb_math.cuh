@@ -53,8 +53,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// FP32 form of the integral and its gradient together, with SFU reciprocals and logarithm;
-// inv_r = 1 / r.
+// FP32 forms with SFU reciprocals and logarithm; inv_r = 1 / r.  The integral and its gradient
+// together, and each alone (the compiler drops what a caller does not use).
 __device__ __forceinline__ void descreening_fast(float radius, float scaled, float r, float inv_r,
                                                  float* h, float* grad) {
   if (radius >= r + scaled) {
@@ -73,25 +73,17 @@ __device__ __forceinline__ void descreening_fast(float radius, float scaled, flo
   *grad = (0.125f * (1.f + scaled * scaled * inv_r * inv_r) * l2u2 + 0.25f * lg * inv_r * inv_r) *
           inv_r;
 }
-
-// The pair passes' forms: SFU arithmetic in FP32, the exact expressions in FP64.
-__device__ __forceinline__ float descreening_pair(float radius, float scaled, float r, float inv_r) {
+__device__ __forceinline__ float descreening_fast(float radius, float scaled, float r,
+                                                  float inv_r) {
   float h, g;
   descreening_fast(radius, scaled, r, inv_r, &h, &g);
   return h;
 }
-__device__ __forceinline__ double descreening_pair(double radius, double scaled, double r, double) {
-  return descreening<double>(radius, scaled, r);
-}
-__device__ __forceinline__ float descreening_gradient_pair(float radius, float scaled, float r,
+__device__ __forceinline__ float descreening_gradient_fast(float radius, float scaled, float r,
                                                            float inv_r) {
   float h, g;
   descreening_fast(radius, scaled, r, inv_r, &h, &g);
   return g;
-}
-__device__ __forceinline__ double descreening_gradient_pair(double radius, double scaled, double r,
-                                                            double) {
-  return descreening_gradient<double>(radius, scaled, r);
 }
 
 }  // namespace gb

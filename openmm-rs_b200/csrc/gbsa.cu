@@ -26,13 +26,34 @@ namespace {
 
 using namespace gb;
 
-// kNb (pass 2 only): the NoCutoff NonbondedForce pair terms (bare Coulomb + LJ 12-6 with the
+// Tiles whose blocks' bounding boxes lie farther apart than the cutoff hold no pair (the boxes
+// are gb_pack's, of the same FP32 positions the FP32 passes use; the factor covers rounding).
+// In a periodic box the gap is that of the nearest images, axis by axis, which needs a
+// rectangular box.
+__device__ __forceinline__ bool beyond_cutoff(const GbArgs& a, int I, int J) {
+  const float4 ci = a.block_box[2 * I], hi = a.block_box[2 * I + 1];
+  const float4 cj = a.block_box[2 * J], hj = a.block_box[2 * J + 1];
+  float d[3] = {cj.x - ci.x, cj.y - ci.y, cj.z - ci.z};
+  if (a.periodic) {
+    if (a.boxf.bx != 0.f || a.boxf.cx != 0.f || a.boxf.cy != 0.f) return false;
+    min_image_fast(d[0], d[1], d[2], a.boxf);
+  }
+  return box_gap2f(d, ci, hi, cj, hj) > a.skip2;
+}
+
+// r <= cutoff with r as the FP32 form rounds it (r^2 rsqrt(r^2))
+__device__ __forceinline__ bool within_cutoff(const GbArgs& a, float r2) {
+  return r2 * rsqrt_r(r2) <= (float)a.cutoff;
+}
+
+// The FP64 form of the three passes, one i-particle per lane.  kNb (pass 2 only): the NoCutoff NonbondedForce pair terms (bare Coulomb + LJ 12-6 with the
 // tile's exclusion mask, energy and virial as the nonbonded pair kernel computes them) join the
 // GB pair term, sharing the distance, 1/r and the force rotation.  Pass 2 reads each slot's
 // Born radius with its reciprocal, so r^2 / (4 R_i R_j) needs no division, and needs r itself
 // only for the cutoff (kCutoff) and 1/r only for the nonbonded terms.
-template <class Real, int kPass, bool kEnergy, bool kCutoff, bool kNb = false>
+template <int kPass, bool kEnergy, bool kCutoff, bool kNb = false>
 __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
+  using Real = double;
   if (kPass != 2 && a.use_learned && *a.use_learned) return;  // the network replaces them
   using T4 = typename V4<Real>::T4;
   using T2 = typename V4<Real>::T2;
@@ -50,6 +71,7 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
   for (int t = blockIdx.x * 4 + w; t < a.n_tiles; t += gridDim.x * 4) {
     const int2 tile = a.tiles[t];
     const int I = tile.x, J = tile.y;
+    if (kCutoff && beyond_cutoff(a, I, J)) continue;
     const bool self = I == J;
     const int si = 32 * I + lane, sj = 32 * J + lane;
     const int ai = a.slot_atom[si], aj = a.slot_atom[sj];
@@ -91,32 +113,25 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
       const T4 pj = s_pos[w][jl];
       Real dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
       if (a.periodic) {
-        if constexpr (sizeof(Real) == 4) min_image_fast(dx, dy, dz, a.boxf);
-        else min_image_fast(dx, dy, dz, a.boxd);
+        min_image_fast(dx, dy, dz, a.boxd);
       }
       const Real r2 = dx * dx + dy * dy + dz * dz;
       bool use = ai >= 0 && ((valid_j >> jl) & 1u);
       Real r = Real(1), inv_r = Real(1);
       if (kPass != 2 || kCutoff || kNb) {
-        if constexpr (sizeof(Real) == 4) {  // SFU reciprocal square root in the FP32 kernel
-          inv_r = rsqrt_r(use ? r2 : Real(1));
-          r = (use ? r2 : Real(1)) * inv_r;
-        } else {
-          r = sqrt_r(use ? r2 : Real(1));
-          inv_r = Real(1) / r;
-        }
+        r = sqrt_r(use ? r2 : Real(1));
+        inv_r = Real(1) / r;
       }
       if (kCutoff) use = use && r <= (Real)a.cutoff;  // gbsa_obc.rs:169 (<=)
       Real fo = 0;
       if (kPass == 1) {
         if (use) {
           const T2 qj = s_par[w][jl];
-          acc_i += descreening_pair(qi.x, qj.y, r, inv_r);
-          if (!self) acc_j += descreening_pair(qj.x, qi.y, r, inv_r);
+          acc_i += descreening(qi.x, qj.y, r);
+          if (!self) acc_j += descreening(qj.x, qi.y, r);
         }
       } else if (kPass == 2) {
         if (use) {
-          // SFU forms (ex2, rsqrt) in the FP32 kernel, exact ones in FP64
           const T2 bj = s_born[w][jl];
           const Real product = bi.x * bj.x;
           const Real d = Real(0.25) * r2 * (bi.y * bj.y);
@@ -160,8 +175,8 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
         if (use) {
           const T2 qj = s_par[w][jl];
           const Real rj_aux = s_aux[w][jl];
-          fo = -(ri_aux * descreening_gradient_pair(qi.x, qj.y, r, inv_r) +
-                 rj_aux * descreening_gradient_pair(qj.x, qi.y, r, inv_r));
+          fo = -(ri_aux * descreening_gradient(qi.x, qj.y, r) +
+                 rj_aux * descreening_gradient(qj.x, qi.y, r));
         }
       }
       if (kPass != 1) {
@@ -223,15 +238,15 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
   }
 }
 
-// Pass 2 in FP32 for non-periodic systems without a cutoff (the batched-chain workloads), with
-// two i-particles per lane and packed (f32x2) arithmetic: lane m of each 16-lane half of the
+// Pass 2 in FP32, with two i-particles per lane and packed (f32x2) arithmetic: lane m of each 16-lane half of the
 // warp holds i-slots m and m + 16 of block I and meets the half's 16 entries of block J in 16
 // steps, so a warp evaluates 64 pairs per step; the entry's force and dE/dR rotate within the
 // half and are back at the entry's lane after the 16 steps, and the two halves' partial sums of
 // each i-slot are added at the end (lane ^ 16).  Tiles whose every pair is a valid particle pair
 // without exclusion take a loop without masks; self tiles (each pair seen from both sides, i
-// sums only, half energy), padded and excluded tiles apply bit masks kept in step order.
-template <bool kEnergy, bool kNb>
+// sums only, half energy), padded and excluded tiles apply bit masks kept in step order, and so
+// do all tiles when there is a cutoff (r <= cutoff, gbsa_obc.rs:169).
+template <bool kEnergy, bool kNb, bool kCutoff>
 __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ float4 s_pos[4][32];                // x, y, z, q sqrt|prefactor|
@@ -247,6 +262,7 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
   for (int t = blockIdx.x * 4 + w; t < a.n_tiles; t += gridDim.x * 4) {
     const int2 tile = a.tiles[t];
     const int I = tile.x, J = tile.y;
+    if (kCutoff && beyond_cutoff(a, I, J)) continue;
     const bool self = I == J;
     const int ai = a.slot_atom[32 * I + lane], aj = a.slot_atom[32 * J + lane];
     s_pos[w][lane] = posq[32 * J + lane];
@@ -274,7 +290,7 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
       use_bits = u1 | (u2 << 16);
       if (kNb) ex_bits = rot(__shfl_sync(FULL, excl, i1)) | (rot(__shfl_sync(FULL, excl, i2)) << 16);
     }
-    const bool plain = __all_sync(FULL, use_bits == 0xffffffffu && ex_bits == 0u);
+    const bool plain = !kCutoff && __all_sync(FULL, use_bits == 0xffffffffu && ex_bits == 0u);
     const float4 p1 = posq[32 * I + i1], p2 = posq[32 * I + i2];
     const float2 b1 = born[32 * I + i1], b2 = born[32 * I + i2];
     float4 n1 = make_float4(0.f, 0.f, 0.f, 0.f), n2 = n1;
@@ -302,14 +318,22 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
         const int jl = eb | ((m + k) & 15);
         const float4 pj = s_pos[w][jl];
         const float2 bj = s_born[w][jl];
-        const float2 dx = x2::add(x2::bc(pj.x), npx), dy = x2::add(x2::bc(pj.y), npy),
-                     dz = x2::add(x2::bc(pj.z), npz);
+        float2 dx = x2::add(x2::bc(pj.x), npx), dy = x2::add(x2::bc(pj.y), npy),
+               dz = x2::add(x2::bc(pj.z), npz);
+        if (kCutoff && a.periodic) {
+          min_image_fast(dx.x, dy.x, dz.x, a.boxf);
+          min_image_fast(dx.y, dy.y, dz.y, a.boxf);
+        }
         float2 r2 = x2::fma(dz, dz, x2::fma(dy, dy, x2::mul(dx, dx)));
         bool u1 = true, u2 = true;
         if (kMasked) {
           u1 = (ub & 1u) != 0u;
           u2 = (ub & 0x10000u) != 0u;
           ub >>= 1;
+          if (kCutoff) {
+            u1 = u1 && within_cutoff(a, r2.x);
+            u2 = u2 && within_cutoff(a, r2.y);
+          }
           r2 = x2::select(u1, u2, r2, 1.f);
         }
         // GB pair (gbsa_obc.rs:239-260): pe = -qn q_j / sqrt(r^2 + R_i R_j exp(-d)), d = r^2 / (4 R_i R_j)
@@ -323,8 +347,10 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
         float2 bd = x2::mul(x2::mul(pi2, ex), x2::fma(d, x2::bc(0.5f), x2::bc(0.5f)));
         if (kEnergy) {
           const double sc = self ? 0.5 : 1.0;
-          if (u1) e_gb -= sc * (double)pen.x;
-          if (u2) e_gb -= sc * (double)pen.y;
+          // with a cutoff the pair energy is shifted by -prefactor q_i q_j / cutoff
+          const double inv_rc = kCutoff ? 1.0 / a.cutoff : 0.0;
+          if (u1) e_gb -= sc * ((double)pen.x - (kCutoff ? (double)(qn.x * pj.w) * inv_rc : 0.0));
+          if (u2) e_gb -= sc * ((double)pen.y - (kCutoff ? (double)(qn.y * pj.w) * inv_rc : 0.0));
         }
         if constexpr (kNb) {
           bool x1 = true, x2v = true;  // not excluded
@@ -439,6 +465,199 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
   }
 }
 
+// The descreening integral of a sphere of scaled radius s at distance r outside radius rho
+// (rho = rho_i - 0.009) and its gradient, for pairs far enough apart that the sphere lies wholly
+// outside rho (r - s >= rho).  There the reference's expression (gbsa_obc.rs:278-309) equals
+//   H = s / (r^2 - s^2) - atanh(s / r) / r = (s^3 / r^4) sum_{k>=1} 2k / (2k+1) t^(k-1),
+//   g = (x (1 + x^2) / (1 - x^2)^2 - atanh x) / (2 r^3)
+//     = (s^3 / r^6) sum_{k>=1} 2k (k+1) / (2k+1) t^(k-1),   x = s / r, t = x^2
+// (the power series of atanh and of the geometric sums): one reciprocal and no logarithm, and no
+// difference of nearly equal terms.  Seven terms of either series leave a relative error below
+// 3e-8 for t <= kFarX^2.
+constexpr float kFarX = 0.25f;  // the series serves |s| <= 0.25 r and rho <= 0.75 r
+__device__ __forceinline__ float2 far_integral(float2 t) {
+  float2 p = x2::bc(14.f / 15.f);
+  p = x2::fma(p, t, x2::bc(12.f / 13.f));
+  p = x2::fma(p, t, x2::bc(10.f / 11.f));
+  p = x2::fma(p, t, x2::bc(8.f / 9.f));
+  p = x2::fma(p, t, x2::bc(6.f / 7.f));
+  p = x2::fma(p, t, x2::bc(4.f / 5.f));
+  return x2::fma(p, t, x2::bc(2.f / 3.f));
+}
+__device__ __forceinline__ float2 far_gradient(float2 t) {
+  float2 p = x2::bc(112.f / 15.f);
+  p = x2::fma(p, t, x2::bc(84.f / 13.f));
+  p = x2::fma(p, t, x2::bc(60.f / 11.f));
+  p = x2::fma(p, t, x2::bc(40.f / 9.f));
+  p = x2::fma(p, t, x2::bc(24.f / 7.f));
+  p = x2::fma(p, t, x2::bc(12.f / 5.f));
+  return x2::fma(p, t, x2::bc(4.f / 3.f));
+}
+
+// Passes 1 and 3 in FP32: two i-particles per lane and packed arithmetic as in pass 2, both
+// directions of a pair from one distance.  Pairs of which either particle is closer than the
+// series above allows (r^2 below the larger of the two particles' bounds, max(|s| / kFarX,
+// rho / (1 - kFarX))^2) take the general expressions, lane by lane; in a chain of 2,000 particles
+// that is a few per cent of the pairs, in few tiles.  Bound by the FP32 pipe.  The general
+// expressions for every pair, one pair per lane (7 SFU operations and about 100 FP32 instructions
+// for both directions), took 114 us (pass 1) and 118 us (pass 3) on 48 chains of 200 to 2,000
+// particles (35.6 M pairs); this form takes 68 and 81 us, and the forces' error against 64 bits
+// falls too (4,999-particle chain, 2 nm cutoff: 1.8e-6 to 1.4e-6).
+template <int kPass, bool kCutoff>
+__global__ void __launch_bounds__(128) gb_descreen_x2(const GbArgs a) {
+  if (a.use_learned && *a.use_learned) return;  // the network replaces them
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ float4 s_pos[4][32];  // x, y, z, the particle's squared near bound
+  __shared__ float4 s_par[4][32];  // rho, s, s^2, s^3
+  __shared__ float s_dedr[kPass == 3 ? 4 : 1][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float4* posq = reinterpret_cast<const float4*>(a.posq);
+  const float2* par = reinterpret_cast<const float2*>(a.params);
+  const float* dedr = reinterpret_cast<const float*>(a.dedr_slot);
+  const int m = lane & 15, eb = lane & 16, i1 = m, i2 = m + 16;
+  const int src = eb | ((m + 1) & 15);
+  auto near2 = [](float2 q) {
+    const float b = fmaxf(fabsf(q.y) * (1.f / kFarX), q.x * (1.f / (1.f - kFarX)));
+    return b * b;
+  };
+  for (int t = blockIdx.x * 4 + w; t < a.n_tiles; t += gridDim.x * 4) {
+    const int2 tile = a.tiles[t];
+    const int I = tile.x, J = tile.y;
+    if (kCutoff && beyond_cutoff(a, I, J)) continue;
+    const bool self = I == J;
+    const int ai = a.slot_atom[32 * I + lane], aj = a.slot_atom[32 * J + lane];
+    {
+      const float4 p = posq[32 * J + lane];
+      const float2 q = par[32 * J + lane];
+      const float ss = q.y * q.y;
+      s_pos[w][lane] = make_float4(p.x, p.y, p.z, near2(q));
+      s_par[w][lane] = make_float4(q.x, q.y, ss, ss * q.y);
+      if (kPass == 3) s_dedr[w][lane] = dedr[32 * J + lane];
+    }
+    const unsigned valid_i = __ballot_sync(FULL, ai >= 0), valid_j = __ballot_sync(FULL, aj >= 0);
+    // step-ordered masks: bit k (i1) and 16 + k (i2) stand for entry eb + ((m + k) mod 16)
+    uint32_t use_bits;
+    {
+      const uint32_t x = (valid_j >> eb) & 0xffffu;
+      const uint32_t vj = ((x >> m) | (x << (16 - m))) & 0xffffu;
+      uint32_t u1 = ((valid_i >> i1) & 1u) ? vj : 0u, u2 = ((valid_i >> i2) & 1u) ? vj : 0u;
+      if (self) {  // the diagonal: entry eb + m at step 0 is i1 (eb = 0) or i2 (eb = 16)
+        u1 &= eb == 0 ? ~1u : ~0u;
+        u2 &= eb == 16 ? ~1u : ~0u;
+      }
+      use_bits = u1 | (u2 << 16);
+    }
+    const float4 p1 = posq[32 * I + i1], p2 = posq[32 * I + i2];
+    const float2 q1 = par[32 * I + i1], q2 = par[32 * I + i2];
+    const float2 npx = make_float2(-p1.x, -p2.x), npy = make_float2(-p1.y, -p2.y),
+                 npz = make_float2(-p1.z, -p2.z);
+    const float2 si = make_float2(q1.y, q2.y), s2i = x2::mul(si, si), s3i = x2::mul(s2i, si);
+    const float n1 = near2(q1), n2 = near2(q2);
+    float2 di = x2::bc(0.f);
+    if (kPass == 3) di = make_float2(dedr[32 * I + i1], dedr[32 * I + i2]);
+    __syncwarp();
+    float2 acc_i = x2::bc(0.f), fx = x2::bc(0.f), fy = x2::bc(0.f), fz = x2::bc(0.f);
+    float acc_j = 0.f, fjx = 0.f, fjy = 0.f, fjz = 0.f;
+    uint32_t ub = use_bits;
+#pragma unroll 2
+    for (int k = 0; k < 16; ++k) {
+      const int jl = eb | ((m + k) & 15);
+      const float4 pj = s_pos[w][jl], qj = s_par[w][jl];
+      float2 dx = x2::add(x2::bc(pj.x), npx), dy = x2::add(x2::bc(pj.y), npy),
+             dz = x2::add(x2::bc(pj.z), npz);
+      if (kCutoff && a.periodic) {
+        min_image_fast(dx.x, dy.x, dz.x, a.boxf);
+        min_image_fast(dx.y, dy.y, dz.y, a.boxf);
+      }
+      float2 r2 = x2::fma(dz, dz, x2::fma(dy, dy, x2::mul(dx, dx)));
+      bool u1 = (ub & 1u) != 0u, u2 = (ub & 0x10000u) != 0u;
+      ub >>= 1;
+      if (kCutoff) {
+        u1 = u1 && within_cutoff(a, r2.x);
+        u2 = u2 && within_cutoff(a, r2.y);
+      }
+      const bool near1 = u1 && r2.x < fmaxf(n1, pj.w), near_2 = u2 && r2.y < fmaxf(n2, pj.w);
+      const float2 u = x2::rcp_approx(r2), uu = x2::mul(u, u);
+      const float2 ti = x2::mul(u, x2::bc(qj.z)), tj = x2::mul(u, s2i);
+      if (kPass == 1) {
+        float2 hi = x2::mul(x2::mul(uu, x2::bc(qj.w)), far_integral(ti));  // adds to I_i
+        float2 hj = x2::mul(x2::mul(uu, s3i), far_integral(tj));           // adds to I_j
+        if (near1) {
+          const float inv = rsqrt_r(r2.x), r = r2.x * inv;
+          hi.x = descreening_fast(q1.x, qj.y, r, inv);
+          hj.x = descreening_fast(qj.x, q1.y, r, inv);
+        }
+        if (near_2) {
+          const float inv = rsqrt_r(r2.y), r = r2.y * inv;
+          hi.y = descreening_fast(q2.x, qj.y, r, inv);
+          hj.y = descreening_fast(qj.x, q2.y, r, inv);
+        }
+        acc_i = x2::add(acc_i, x2::select(u1, u2, hi, 0.f));
+        if (!self) {
+          acc_j += (u1 ? hj.x : 0.f) + (u2 ? hj.y : 0.f);
+          acc_j = __shfl_sync(FULL, acc_j, src);
+        }
+      } else {
+        const float dj = s_dedr[w][jl];
+        // minus the radial force: D_i g(rho_i, s_j) + D_j g(rho_j, s_i)
+        float2 fo = x2::mul(x2::mul(x2::mul(di, x2::bc(qj.w)), far_gradient(ti)), uu);
+        fo = x2::mul(x2::fma(x2::mul(x2::mul(s3i, x2::bc(dj)), far_gradient(tj)), uu, fo), u);
+        if (near1) {
+          const float inv = rsqrt_r(r2.x), r = r2.x * inv;
+          fo.x = di.x * descreening_gradient_fast(q1.x, qj.y, r, inv) +
+                 dj * descreening_gradient_fast(qj.x, q1.y, r, inv);
+        }
+        if (near_2) {
+          const float inv = rsqrt_r(r2.y), r = r2.y * inv;
+          fo.y = di.y * descreening_gradient_fast(q2.x, qj.y, r, inv) +
+                 dj * descreening_gradient_fast(qj.x, q2.y, r, inv);
+        }
+        fo = x2::select(u1, u2, fo, 0.f);
+        const float2 gx = x2::mul(fo, dx), gy = x2::mul(fo, dy), gz = x2::mul(fo, dz);
+        fx = x2::sub(fx, gx);
+        fy = x2::sub(fy, gy);
+        fz = x2::sub(fz, gz);
+        if (!self) {
+          fjx += gx.x + gx.y;
+          fjy += gy.x + gy.y;
+          fjz += gz.x + gz.y;
+          fjx = __shfl_sync(FULL, fjx, src);
+          fjy = __shfl_sync(FULL, fjy, src);
+          fjz = __shfl_sync(FULL, fjz, src);
+        }
+      }
+    }
+    // the two halves' sums of this lane's i-slots; the lane commits i-slot `lane`
+    const bool second = eb != 0;
+    if (kPass == 1) {
+      acc_i.x += __shfl_xor_sync(FULL, acc_i.x, 16);
+      acc_i.y += __shfl_xor_sync(FULL, acc_i.y, 16);
+      if (ai >= 0)
+        add_fixed(a.born_sum + ai, to_fixed((double)(second ? acc_i.y : acc_i.x), kBornScale));
+      if (!self && aj >= 0) add_fixed(a.born_sum + aj, to_fixed((double)acc_j, kBornScale));
+    } else {
+      fx.x += __shfl_xor_sync(FULL, fx.x, 16);
+      fx.y += __shfl_xor_sync(FULL, fx.y, 16);
+      fy.x += __shfl_xor_sync(FULL, fy.x, 16);
+      fy.y += __shfl_xor_sync(FULL, fy.y, 16);
+      fz.x += __shfl_xor_sync(FULL, fz.x, 16);
+      fz.y += __shfl_xor_sync(FULL, fz.y, 16);
+      const float fs = float(kForceScale);
+      if (ai >= 0) {
+        add_fixed(a.force + ai, to_fixed(second ? fx.y : fx.x, fs));
+        add_fixed(a.force + a.n_atoms + ai, to_fixed(second ? fy.y : fy.x, fs));
+        add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(second ? fz.y : fz.x, fs));
+      }
+      if (!self && aj >= 0) {
+        add_fixed(a.force + aj, to_fixed(fjx, fs));
+        add_fixed(a.force + a.n_atoms + aj, to_fixed(fjy, fs));
+        add_fixed(a.force + 2 * a.n_atoms + aj, to_fixed(fjz, fs));
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // gbsa_obc.rs:214-237: radii, chain factor, self + ACE energies, dE/dR from them.
 template <class Real, bool kEnergy>
 __global__ void gb_radii(const GbArgs a) {
@@ -497,7 +716,7 @@ __global__ void gb_chain(const GbArgs a) {
 template <class Real>
 __global__ void gb_pack(const GbArgs a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n_slots) return;
+  if (s >= a.n_slots) return;  // whole warps: n_slots is a multiple of 32
   const int atom = a.slot_atom[s];
   typename V4<Real>::T4 p;
   typename V4<Real>::T2 q;
@@ -517,6 +736,20 @@ __global__ void gb_pack(const GbArgs a) {
   }
   reinterpret_cast<typename V4<Real>::T4*>(a.posq)[s] = p;
   reinterpret_cast<typename V4<Real>::T2*>(a.params)[s] = q;
+  if (a.use_cutoff) {  // the block's bounding box, for the tiles the cutoff leaves empty
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (atom >= 0) {
+      lo[0] = hi[0] = (float)p.x;
+      lo[1] = hi[1] = (float)p.y;
+      lo[2] = hi[2] = (float)p.z;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+    if ((s & 31) == 0) store_box(a.block_box, s >> 5, lo, hi);
+  }
   if (a.nb_params) {
     typename V4<Real>::T4 nb;
     nb.x = nb.y = nb.z = nb.w = Real(0);
@@ -531,12 +764,26 @@ __global__ void gb_pack(const GbArgs a) {
 
 }  // namespace
 
-template <class Real, int kPass, bool kEnergy, bool kNb = false>
+// Pass `kPass` in the form for Real: FP32 packed, FP64 one pair per lane.
+template <class Real, int kPass, bool kEnergy, bool kNb, bool kCutoff>
 void launch_gb_pass(const GbArgs& a, int grid, cudaStream_t s) {
-  if (a.use_cutoff)
-    gb_pass<Real, kPass, kEnergy, true, kNb><<<grid, 128, 0, s>>>(a);
+  if constexpr (sizeof(Real) == 8)
+    gb_pass<kPass, kEnergy, kCutoff, kNb><<<grid, 128, 0, s>>>(a);
+  else if constexpr (kPass == 2)
+    gb_pairs_x2<kEnergy, kNb, kCutoff><<<grid, 128, 0, s>>>(a);
   else
-    gb_pass<Real, kPass, kEnergy, false, kNb><<<grid, 128, 0, s>>>(a);
+    gb_descreen_x2<kPass, kCutoff><<<grid, 128, 0, s>>>(a);
+}
+
+// `fuse`: the NoCutoff nonbonded terms join pass 2 (never with a cutoff).
+template <class Real, int kPass, bool kEnergy>
+void launch_gb_pass(const GbArgs& a, bool fuse, int grid, cudaStream_t s) {
+  if (a.use_cutoff)
+    launch_gb_pass<Real, kPass, kEnergy, false, true>(a, grid, s);
+  else if (kPass == 2 && fuse)
+    launch_gb_pass<Real, kPass, kEnergy, kPass == 2, false>(a, grid, s);
+  else
+    launch_gb_pass<Real, kPass, kEnergy, false, false>(a, grid, s);
 }
 
 template <class Real>
@@ -549,7 +796,7 @@ void launch_gbsa_phase(const GbArgs& a, int phase, bool energy, int sm_count, cu
       gb_pack<Real><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass1:
-      launch_gb_pass<Real, 1, false>(a, gt, s);
+      launch_gb_pass<Real, 1, false>(a, false, gt, s);
       break;
     case kGbRadii:
       if (energy)
@@ -558,33 +805,16 @@ void launch_gbsa_phase(const GbArgs& a, int phase, bool energy, int sm_count, cu
         gb_radii<Real, false><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass2:
-      if (sizeof(Real) == 4 && !a.use_cutoff && !a.periodic) {
-        if (a.fuse_nonbonded) {
-          if (energy)
-            gb_pairs_x2<true, true><<<gt, 128, 0, s>>>(a);
-          else
-            gb_pairs_x2<false, true><<<gt, 128, 0, s>>>(a);
-        } else if (energy) {
-          gb_pairs_x2<true, false><<<gt, 128, 0, s>>>(a);
-        } else {
-          gb_pairs_x2<false, false><<<gt, 128, 0, s>>>(a);
-        }
-      } else if (a.fuse_nonbonded) {
-        if (energy)
-          launch_gb_pass<Real, 2, true, true>(a, gt, s);
-        else
-          launch_gb_pass<Real, 2, false, true>(a, gt, s);
-      } else if (energy) {
-        launch_gb_pass<Real, 2, true>(a, gt, s);
-      } else {
-        launch_gb_pass<Real, 2, false>(a, gt, s);
-      }
+      if (energy)
+        launch_gb_pass<Real, 2, true>(a, a.fuse_nonbonded != 0, gt, s);
+      else
+        launch_gb_pass<Real, 2, false>(a, a.fuse_nonbonded != 0, gt, s);
       break;
     case kGbChain:
       gb_chain<Real><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass3:
-      launch_gb_pass<Real, 3, false>(a, gt, s);
+      launch_gb_pass<Real, 3, false>(a, false, gt, s);
       break;
   }
 }

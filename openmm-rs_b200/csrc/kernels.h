@@ -262,6 +262,8 @@ struct GbArgs {
   double cutoff;
   Box<double> boxd;
   Box<float> boxf;
+  float4* block_box;          // [n_slots / 32][2] centre, half extents (with a cutoff)
+  float skip2;                // cutoff^2 with a margin for rounding: box gaps beyond hold no pair
   void* posq;                 // [n_slots] Real4: x, y, z, q sqrt|prefactor|
   void* params;               // [n_slots] Real2: rho - 0.009, s (rho - 0.009)
   void* born_slot;            // [n_slots] Real2: Born radius and its reciprocal

@@ -7,6 +7,34 @@
 #include "kernels.h"
 
 namespace ommb200 {
+
+// Bounding boxes of 32-slot blocks, centre and half extents, of FP32 positions; a block without
+// particles gets an infinitely distant one.
+__device__ __forceinline__ void store_box(float4* boxes, int blk, const float lo[3],
+                                          const float hi[3]) {
+  const bool empty = lo[0] > hi[0];
+  boxes[2 * blk] = empty ? make_float4(3e18f, 3e18f, 3e18f, 0.f)
+                         : make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]),
+                                       0.5f * (lo[2] + hi[2]), 0.f);
+  boxes[2 * blk + 1] = empty ? make_float4(0.f, 0.f, 0.f, 0.f)
+                             : make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]),
+                                           0.5f * (hi[2] - lo[2]), 0.f);
+}
+// Squared gap between two boxes, less the rounding of coordinates of their size; d: the centres'
+// difference.
+__device__ __forceinline__ float box_gap2f(const float d[3], const float4& ci, const float4& hi,
+                                           const float4& cj, const float4& hj) {
+  const float gx = fabsf(d[0]) - hi.x - hj.x - 5e-7f * (fabsf(ci.x) + fabsf(cj.x) + hi.x + hj.x);
+  const float gy = fabsf(d[1]) - hi.y - hj.y - 5e-7f * (fabsf(ci.y) + fabsf(cj.y) + hi.y + hj.y);
+  const float gz = fabsf(d[2]) - hi.z - hj.z - 5e-7f * (fabsf(ci.z) + fabsf(cj.z) + hi.z + hj.z);
+  const float x = fmaxf(gx, 0.f), y = fmaxf(gy, 0.f), z = fmaxf(gz, 0.f);
+  return x * x + y * y + z * z;
+}
+__device__ __forceinline__ bool boxes_apart(const float4* boxes, int I, int J, float limit2) {
+  const float4 ci = boxes[2 * I], hi = boxes[2 * I + 1], cj = boxes[2 * J], hj = boxes[2 * J + 1];
+  const float d[3] = {cj.x - ci.x, cj.y - ci.y, cj.z - ci.z};
+  return box_gap2f(d, ci, hi, cj, hj) > limit2;
+}
 namespace {
 
 template <class Real>

@@ -2,6 +2,7 @@
 #include "engine.h"
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -226,6 +227,12 @@ Engine::Engine(std::unique_ptr<SystemDef> system, std::unique_ptr<IntegratorDef>
   status_ = mem_.alloc<int>(1);
   rebuild_ = mem_.alloc<int>(1);
   rng_step_ = mem_.alloc<unsigned long long>(1);
+  mass_ = mem_.alloc<double>(n_);
+  kinetic_ = mem_.alloc<double>(kKineticParts);
+  OMMB200_CK(cudaMemcpy(mass_, host_masses_.data(), sizeof(double) * n_, cudaMemcpyHostToDevice));
+  void* hr = nullptr;
+  OMMB200_CK(cudaHostAlloc(&hr, sizeof(HostResults), cudaHostAllocDefault));
+  host_.reset(new (hr) HostResults());
   std::vector<double> im(n_);
   for (int i = 0; i < n_; ++i) im[i] = host_masses_[i] == 0.0 ? 0.0 : 1.0 / host_masses_[i];
   OMMB200_CK(cudaMemcpy(inv_mass_, im.data(), sizeof(double) * n_, cudaMemcpyHostToDevice));
@@ -1218,11 +1225,10 @@ void Engine::destroy_graph() {
 void Engine::sync() { OMMB200_CK(cudaStreamSynchronize(stream_)); }
 
 int Engine::take_status() {
-  int st = 0;
-  OMMB200_CK(cudaMemcpy(&st, status_, sizeof(int), cudaMemcpyDeviceToHost));
-  if (st == 0) return 0;
-  const int zero = 0;
-  OMMB200_CK(cudaMemcpy(status_, &zero, sizeof(int), cudaMemcpyHostToDevice));
+  OMMB200_CK(cudaMemcpyAsync(&host_->status, status_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  sync();
+  const int st = host_->status;
+  if (st != 0) OMMB200_CK(cudaMemsetAsync(status_, 0, sizeof(int), stream_));
   return st;
 }
 
@@ -1844,9 +1850,8 @@ void Engine::run_steps(int steps) {
       launch_advance_counter(rng_step_, 1, stream_);
     }
     OMMB200_CK(cudaGetLastError());
-    sync();
-    harvest_profile();
     const int st = take_status();
+    harvest_profile();
     if (st == kStatusTileOverflow && guarded && grow_neighbor_capacity()) {
       restore_dynamic_state(step_snapshot_);
       continue;
@@ -1859,13 +1864,16 @@ void Engine::run_steps(int steps) {
 }
 
 void Engine::set_positions(const double* xyz) {
-  for (size_t i = 0; i < 3 * (size_t)n_; ++i)
-    require(std::isfinite(xyz[i]), "particle positions must be finite");  // neighbors.rs:107-110
+  bool finite = true;  // branch-free, so that it runs at memory speed
+  for (size_t i = 0; i < 3 * (size_t)n_; ++i) finite &= std::fabs(xyz[i]) <= DBL_MAX;
+  require(finite, "particle positions must be finite");  // neighbors.rs:107-110
   OMMB200_CK(cudaMemcpyAsync(pos_, xyz, sizeof(double) * 3 * (size_t)n_, cudaMemcpyHostToDevice, stream_));
-  const int one = 1;
-  OMMB200_CK(cudaMemcpyAsync(rebuild_, &one, sizeof(int), cudaMemcpyHostToDevice, stream_));
+  request_rebuild();
   sync();
 }
+
+// The flag is 0 or 1, so its lowest byte says all.
+void Engine::request_rebuild() { OMMB200_CK(cudaMemsetAsync(rebuild_, 1, 1, stream_)); }
 
 void Engine::set_velocities(const double* v) {
   OMMB200_CK(cudaMemcpyAsync(vel_, v, sizeof(double) * 3 * (size_t)n_, cudaMemcpyHostToDevice, stream_));
@@ -1939,15 +1947,15 @@ void Engine::apply_velocity_constraints(double tolerance) {
   check_status();
 }
 
-// Forces (into `forces`, may be null) and, with `energy`, the fixed-point energy/virial
-// terms of every segment: [8 * segment + (energy, virial xx yy zz xy xz yz)].
-// compute_forces with the energy sums zeroed first, synchronised, and run again after the
-// neighbour list grew when it overflowed; any other device error is raised.
-void Engine::compute_forces_checked(bool energy, uint32_t groups) {
+// compute_forces with the energy sums zeroed first and `outputs` enqueued behind it,
+// synchronised, and run again after the neighbour list grew when it overflowed; any other device
+// error is raised.
+void Engine::compute_forces_checked(bool energy, uint32_t groups,
+                                    const std::function<void()>& outputs) {
   for (;;) {
     OMMB200_CK(cudaMemsetAsync(energy_, 0, 8 * segments_.size() * sizeof(long long), stream_));
     compute_forces(energy, groups);
-    sync();
+    if (outputs) outputs();
     const int st = take_status();
     if (st == kStatusTileOverflow && grow_neighbor_capacity()) continue;
     raise_status(st);
@@ -1955,21 +1963,21 @@ void Engine::compute_forces_checked(bool energy, uint32_t groups) {
   }
 }
 
-std::vector<long long> Engine::evaluate(bool energy, uint32_t groups, double* forces) {
-  const size_t nterms = 8 * segments_.size();
-  compute_forces_checked(energy, groups);
-  if (forces) {
-    std::vector<long long> f(3 * (size_t)n_);
-    OMMB200_CK(cudaMemcpyAsync(f.data(), force_, 8 * f.size(), cudaMemcpyDeviceToHost, stream_));
-    sync();
-    for (int i = 0; i < n_; ++i)
-      for (int c = 0; c < 3; ++c) forces[3 * i + c] = (double)f[(size_t)c * n_ + i] * kForceScaleInv;
-  }
-  std::vector<long long> terms(nterms);
-  OMMB200_CK(cudaMemcpyAsync(terms.data(), energy_, 8 * nterms, cudaMemcpyDeviceToHost, stream_));
-  sync();
+// Forces (into `forces`, may be null) and, with `energy`, the fixed-point energy/virial
+// terms of every segment: [8 * segment + (energy, virial xx yy zz xy xz yz)].  `outputs`:
+// further device-to-host copies of the same call.
+std::vector<long long> Engine::evaluate(bool energy, uint32_t groups, double* forces,
+                                        const std::function<void()>& outputs) {
+  std::vector<long long> terms(8 * segments_.size());
+  compute_forces_checked(energy, groups, [&] {
+    if (forces) {
+      launch_state_forces(n_, force_, scratch3_, stream_);
+      OMMB200_CK(cudaMemcpyAsync(forces, scratch3_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+    }
+    OMMB200_CK(cudaMemcpyAsync(terms.data(), energy_, 8 * terms.size(), cudaMemcpyDeviceToHost, stream_));
+    if (outputs) outputs();
+  });
   harvest_profile();
-  check_status();
   return terms;
 }
 
@@ -2003,27 +2011,29 @@ void Engine::get_state(int flags, uint32_t groups, double* pos, double* vel, dou
                        ommb200_state_info* info) {
   const bool need_forces = flags & (OMMB200_STATE_FORCES | OMMB200_STATE_ENERGY | OMMB200_STATE_VIRIAL);
   const bool need_energy = flags & (OMMB200_STATE_ENERGY | OMMB200_STATE_VIRIAL);
+  auto outputs = [&] {
+    if (info) {
+      launch_kinetic_energy(n_, mass_, vel_, kinetic_, stream_);
+      OMMB200_CK(cudaMemcpyAsync(host_->kinetic, kinetic_, sizeof(host_->kinetic),
+                                 cudaMemcpyDeviceToHost, stream_));
+    }
+    if (pos) OMMB200_CK(cudaMemcpyAsync(pos, pos_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+    if (vel) OMMB200_CK(cudaMemcpyAsync(vel, vel_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+  };
   long long e[8] = {0};
   if (need_forces) {
-    std::vector<long long> terms = evaluate(need_energy, groups, forces);
+    std::vector<long long> terms = evaluate(need_energy, groups, forces, outputs);
     for (size_t k = 0; k < terms.size(); ++k) e[k % 8] += terms[k];
+  } else {
+    outputs();
+    sync();
   }
-  std::vector<double> vtmp;
-  double* vout = vel;
-  if (!vout && info) {
-    vtmp.resize(3 * (size_t)n_);
-    vout = vtmp.data();
-  }
-  if (pos) OMMB200_CK(cudaMemcpyAsync(pos, pos_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
-  if (vout) OMMB200_CK(cudaMemcpyAsync(vout, vel_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
-  sync();
   if (!info) return;
   info->time = time_;
   info->step_count = step_count_;
   std::copy(box_, box_ + 9, info->box);
   double ke = 0.0;
-  for (int i = 0; i < n_; ++i)
-    ke += host_masses_[i] * (vout[3 * i] * vout[3 * i] + vout[3 * i + 1] * vout[3 * i + 1] + vout[3 * i + 2] * vout[3 * i + 2]);
+  for (double part : host_->kinetic) ke += part;
   info->kinetic_energy = 0.5 * ke;
   double w[6];
   const double pe = assemble_energy(e, need_energy ? groups : 0u, w);
@@ -2260,11 +2270,15 @@ void Engine::save_dynamic_state(DynamicSnapshot& snap) {
   if (!snap.x) {
     snap.x = mem_.alloc<double>(3 * (size_t)n_);
     snap.v = mem_.alloc<double>(3 * (size_t)n_);
-    if (learned_) snap.lr = mem_.alloc<float>(kRadiiMlpParams + 2 * kRadiiMlpTrainable + 1 + segments_.size());
+    snap.rng = mem_.alloc<unsigned long long>(1);
+    if (learned_) {
+      snap.lr = mem_.alloc<float>(kRadiiMlpParams + 2 * kRadiiMlpTrainable + 1 + segments_.size());
+      snap.state = mem_.alloc<LearnedState>(1);
+    }
   }
   OMMB200_CK(cudaMemcpyAsync(snap.x, pos_, bytes, cudaMemcpyDeviceToDevice, stream_));
   OMMB200_CK(cudaMemcpyAsync(snap.v, vel_, bytes, cudaMemcpyDeviceToDevice, stream_));
-  OMMB200_CK(cudaMemcpyAsync(&snap.rng, rng_step_, 8, cudaMemcpyDeviceToHost, stream_));
+  OMMB200_CK(cudaMemcpyAsync(snap.rng, rng_step_, 8, cudaMemcpyDeviceToDevice, stream_));
   if (learned_) {
     const size_t at = kRadiiMlpParams + 2 * kRadiiMlpTrainable;
     OMMB200_CK(cudaMemcpyAsync(snap.lr, lr_.params, 4 * kRadiiMlpParams, cudaMemcpyDeviceToDevice, stream_));
@@ -2273,10 +2287,9 @@ void Engine::save_dynamic_state(DynamicSnapshot& snap) {
     OMMB200_CK(cudaMemcpyAsync(snap.lr + at, lr_.adam_t, 4, cudaMemcpyDeviceToDevice, stream_));
     OMMB200_CK(cudaMemcpyAsync(snap.lr + at + 1, lr_.seg_offset, 4 * segments_.size(),
                                cudaMemcpyDeviceToDevice, stream_));
-    OMMB200_CK(cudaMemcpyAsync(&snap.state, lr_.state, sizeof(snap.state), cudaMemcpyDeviceToHost,
-                               stream_));
+    OMMB200_CK(cudaMemcpyAsync(snap.state, lr_.state, sizeof(LearnedState),
+                               cudaMemcpyDeviceToDevice, stream_));
   }
-  sync();
 }
 
 // Puts the saved state back and requests a neighbour-list rebuild from it.
@@ -2284,7 +2297,7 @@ void Engine::restore_dynamic_state(const DynamicSnapshot& snap) {
   const size_t bytes = 24 * (size_t)n_;
   OMMB200_CK(cudaMemcpyAsync(pos_, snap.x, bytes, cudaMemcpyDeviceToDevice, stream_));
   OMMB200_CK(cudaMemcpyAsync(vel_, snap.v, bytes, cudaMemcpyDeviceToDevice, stream_));
-  OMMB200_CK(cudaMemcpyAsync(rng_step_, &snap.rng, 8, cudaMemcpyHostToDevice, stream_));
+  OMMB200_CK(cudaMemcpyAsync(rng_step_, snap.rng, 8, cudaMemcpyDeviceToDevice, stream_));
   const int one = 1;
   OMMB200_CK(cudaMemcpyAsync(rebuild_, &one, sizeof(int), cudaMemcpyHostToDevice, stream_));
   if (learned_) {
@@ -2295,8 +2308,8 @@ void Engine::restore_dynamic_state(const DynamicSnapshot& snap) {
     OMMB200_CK(cudaMemcpyAsync(lr_.adam_t, snap.lr + at, 4, cudaMemcpyDeviceToDevice, stream_));
     OMMB200_CK(cudaMemcpyAsync(lr_.seg_offset, snap.lr + at + 1, 4 * segments_.size(),
                                cudaMemcpyDeviceToDevice, stream_));
-    OMMB200_CK(cudaMemcpyAsync(lr_.state, &snap.state, sizeof(snap.state), cudaMemcpyHostToDevice,
-                               stream_));
+    OMMB200_CK(cudaMemcpyAsync(lr_.state, snap.state, sizeof(LearnedState),
+                               cudaMemcpyDeviceToDevice, stream_));
   }
   sync();
 }

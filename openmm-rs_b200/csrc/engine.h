@@ -72,8 +72,18 @@ struct DynamicSnapshot {
   double* x = nullptr;
   double* v = nullptr;
   float* lr = nullptr;  // learned radii: network, optimiser moments and step, system offsets
-  unsigned long long rng = 0;
-  LearnedState state{};
+  unsigned long long* rng = nullptr;
+  LearnedState* state = nullptr;
+};
+
+// Small results of a call, in pinned memory, so that reading them back waits for nothing but
+// the stream: the device status word and the kinetic energy's partial sums.
+struct HostResults {
+  int status = 0;
+  double kinetic[kKineticParts] = {};
+};
+struct PinnedFree {
+  void operator()(HostResults* p) const { cudaFreeHost(p); }
 };
 
 class Engine {
@@ -175,10 +185,13 @@ class Engine {
   // `in_step`: an MD step's evaluation (the learned radii may judge and train there);
   // `step_offset`: its position inside the captured group of steps.
   void compute_forces(bool energy, uint32_t groups, bool in_step = false, int step_offset = 0);
-  void compute_forces_checked(bool energy, uint32_t groups);
+  void compute_forces_checked(bool energy, uint32_t groups,
+                              const std::function<void()>& outputs = {});
+  void request_rebuild();
   void setup_learned(const LearnedRadiiDef& def);
   void upload_nonbonded_parameters(const NonbondedDef& nb);
-  std::vector<long long> evaluate(bool energy, uint32_t groups, double* forces);
+  std::vector<long long> evaluate(bool energy, uint32_t groups, double* forces,
+                                  const std::function<void()>& outputs = {});
   void enqueue_step(int step_offset);
   void run_steps(int steps);
   void run_graph_steps(int graph_launches);
@@ -192,7 +205,8 @@ class Engine {
   // long-range corrections added to the fixed-point sums e[8] (energy, virial) of `groups`
   double assemble_energy(const long long e[8], uint32_t groups, double w[6]) const;
   void check_status();
-  // Reads and clears the device status word; raise_status throws its error (0: none).
+  // Waits for the stream, reads and clears the device status word; raise_status throws its
+  // error (0: none).
   int take_status();
   void raise_status(int status);
   // After a neighbour-list overflow: larger tile and mask arrays and per-column sort, and a
@@ -245,6 +259,9 @@ class Engine {
   double* pos_ = nullptr;
   double* vel_ = nullptr;
   double* inv_mass_ = nullptr;
+  double* mass_ = nullptr;
+  double* kinetic_ = nullptr;  // [kKineticParts]
+  std::unique_ptr<HostResults, PinnedFree> host_;
   double* scratch3_ = nullptr;
   long long* force_ = nullptr;
   long long* energy_ = nullptr;  // [8 * segments]: energy, virial (6), unused

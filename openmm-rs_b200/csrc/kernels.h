@@ -241,6 +241,14 @@ void launch_pme_convolve(const PmeArgs<Real>& a, bool energy, cudaStream_t s);
 template <class Real>
 void launch_pme_gather(const PmeArgs<Real>& a, cudaStream_t s);
 
+// ---- getState outputs (state.cu) ------------------------------------------------------------
+constexpr int kKineticParts = 64;  // partial sums of the kinetic energy
+// fixed-point forces [3][n] -> kJ/mol/nm [n][3]
+void launch_state_forces(int n, const long long* force, double* out, cudaStream_t s);
+// parts[k]: sum of m v^2 over the particles k takes, in an order fixed by n
+void launch_kinetic_energy(int n, const double* mass, const double* vel, double* parts,
+                           cudaStream_t s);
+
 // ---- GBSAOBCForce --------------------------------------------------------------------------
 // Particles in segment-padded slot order (one segment per independent system); tiles pair
 // 32-slot blocks of the same segment.  energy[8 * segment] receives each segment's energy.

@@ -841,6 +841,9 @@ void Engine::setup_gbsa(const GbsaObcDef& g) {
                         cudaMemcpyHostToDevice));
   a.tiles = dt;
   a.slot_atom = dsa;
+  int* das = mem_.alloc<int>(n_);
+  OMMB200_CK(cudaMemcpy(das, static_atom_slot_.data(), 4 * (size_t)n_, cudaMemcpyHostToDevice));
+  a.atom_slot = das;
   a.block_segment = d_block_segment_;
   a.atom_segment = d_atom_segment_;
   double* q = mem_.alloc<double>(n_);
@@ -1215,11 +1218,12 @@ void Engine::update_bricks() {
 }
 
 void Engine::destroy_graph() {
-  if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-  if (graph_) cudaGraphDestroy(graph_);
-  graph_exec_ = nullptr;
-  graph_ = nullptr;
-  graph_steps_ = 0;
+  for (StepGraph* g : {&group_graph_, &step_graph_}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    if (g->graph) cudaGraphDestroy(g->graph);
+    *g = StepGraph{};
+  }
+  steps_since_capture_ = 0;
 }
 
 void Engine::sync() { OMMB200_CK(cudaStreamSynchronize(stream_)); }
@@ -1346,13 +1350,23 @@ void Engine::set_profiling(bool enabled) {
 // In a captured step the neighbour-list rebuild is the body of an IF node whose condition a
 // one-thread kernel copies from the rebuild flag, so steps without a rebuild skip its nine
 // launches instead of running them as early-exit kernels.
-void Engine::enqueue_conditional_rebuild() {
+cudaGraphConditionalHandle Engine::new_condition() {
   cudaStreamCaptureStatus st;
   cudaGraph_t cap = nullptr;
   OMMB200_CK(cudaStreamGetCaptureInfo(stream_, &st, nullptr, &cap, nullptr, nullptr));
   cudaGraphConditionalHandle handle;
   OMMB200_CK(cudaGraphConditionalHandleCreate(&handle, cap, 0, cudaGraphCondAssignDefault));
-  launch_nlist_condition(nl_, handle, stream_);
+  return handle;
+}
+
+// The rebuild's condition: the first step of a captured group reads the rebuild flag; later
+// steps have theirs set by the integrator before them, in the launch that raises the flag.
+void Engine::enqueue_conditional_rebuild(bool first) {
+  cudaGraphConditionalHandle handle = rebuild_condition_;
+  if (first) {
+    handle = new_condition();
+    launch_nlist_condition(nl_, handle, stream_);
+  }
   enqueue_conditional_body(handle, [&](cudaStream_t s) {
     launch_nlist_rebuild(nl_, dp_, s, with_new_list(nl_));
   });
@@ -1447,12 +1461,13 @@ PruneArgs Engine::prune_args() const {
 }
 
 template <class Real>
-void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs) {
+void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
+                               int step_offset, cudaStream_t direct_stream) {
   const NonbondedDef& nb = *nb_;
   if (nb_periodic_) {
     prof_begin("nlist_rebuild");
     if (capturing_)
-      enqueue_conditional_rebuild();
+      enqueue_conditional_rebuild(step_offset == 0);
     else
       launch_nlist_rebuild(nl_, dp_, stream_, with_new_list(nl_));
     prof_end();
@@ -1542,14 +1557,14 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     e.alpha = alpha_;
     e.n_atoms_for_force = n_;
     prof_begin("exceptions");
-    launch_exceptions(e, energy, stream_);
+    launch_exceptions(e, energy, direct_stream);
     prof_end();
   }
   if (direct && pairs) {
     if (!packed_by_integrator()) {
       prof_begin("pack");
       launch_pack<Real>(n_slots_, nl_.sorted_atom, pos_, nl_.image, nl_.block_center, qscaled_,
-                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, stream_);
+                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, direct_stream);
       prof_end();
     }
     const bool pruned = pruning();
@@ -1628,7 +1643,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
       p.cull_rounds = cull_rounds_;
     }
     prof_begin("pair");
-    launch_pair<Real>(p, elec_, energy, dump, pair_grid_, stream_);
+    launch_pair<Real>(p, elec_, energy, dump, pair_grid_, direct_stream);
     prof_end();
   }
   if (ps != stream_) {  // join
@@ -1645,21 +1660,30 @@ void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step
     prof_end();
   }
   gb_.fuse_nonbonded = 0;
+  const bool gb_on = gb_def_ && ((groups >> gb_def_->force_group) & 1u);
+  // the GB passes are a serial chain of small launches; without a periodic list the direct
+  // nonbonded and bonded kernels need nothing of it and run beside it on their own stream (with
+  // the packing left to the integrator, a 603-particle chain's step takes 31 us against 39)
+  cudaStream_t side = stream_;
+  if (gb_on && !nb_periodic_ && !profiling_) {
+    side = pme_stream_;
+    OMMB200_CK(cudaEventRecord(fork_ev_, stream_));
+    OMMB200_CK(cudaStreamWaitEvent(side, fork_ev_, 0));
+  }
   if (nb_) {
     const int g = nb_->force_group;
     const int rg = nb_->reciprocal_force_group < 0 ? g : nb_->reciprocal_force_group;
     const bool direct = nb_->include_direct_space && ((groups >> g) & 1u);
     const bool recip = nb_pme_ && ((groups >> rg) & 1u);
     // the pair terms go to GB pass 2 when both forces are evaluated (not while dumping pairs)
-    const bool fuse = nb_gb_fusable_ && direct && !dump_mode_ &&
-                      ((groups >> gb_def_->force_group) & 1u);
+    const bool fuse = nb_gb_fusable_ && direct && !dump_mode_ && gb_on;
     gb_.fuse_nonbonded = fuse ? 1 : 0;
     if (dp_)
-      enqueue_nonbonded<double>(energy, direct, recip, dump_mode_, !fuse);
+      enqueue_nonbonded<double>(energy, direct, recip, dump_mode_, !fuse, step_offset, side);
     else
-      enqueue_nonbonded<float>(energy, direct, recip, dump_mode_, !fuse);
+      enqueue_nonbonded<float>(energy, direct, recip, dump_mode_, !fuse, step_offset, side);
   }
-  if (gb_def_ && ((groups >> gb_def_->force_group) & 1u)) {
+  if (gb_on) {
     auto gb = [&](int phase, const char* name) {
       prof_begin(name);
       if (dp_)
@@ -1682,7 +1706,9 @@ void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step
       launch_learned_control(lr_, in_step, step_offset, stream_);
       prof_end();
     }
-    gb(kGbPack, "gb_pack");
+    // inside a captured group the previous step's integrator wrote the packed coordinates
+    if (!(in_step && capturing_ && step_offset > 0 && gb_packed_by_integrator()))
+      gb(kGbPack, "gb_pack");
     lr(kLrLists, "lr_lists");
     lr(kLrFeatures, "lr_features");
     lr(kLrInfer, "lr_infer");
@@ -1699,10 +1725,18 @@ void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step
   for (auto& L : bonded_) {
     if (!((groups >> L.group) & 1u)) continue;
     prof_begin("bonded");
-    launch_bonded(L.args, energy, stream_);
+    launch_bonded(L.args, energy, side);
     prof_end();
   }
+  if (side != stream_) {
+    OMMB200_CK(cudaEventRecord(join_ev_, side));
+    OMMB200_CK(cudaStreamWaitEvent(stream_, join_ev_, 0));
+  }
 }
+
+// The exact GB path without a cutoff (with one, gb_pack also makes the blocks' boxes; the
+// learned radii's judge reads the sums that gb_pack clears).
+bool Engine::gb_packed_by_integrator() const { return gb_def_ && !learned_ && !gb_.use_cutoff; }
 
 IntegrateArgs Engine::integrate_args(int step_offset) const {
   IntegrateArgs a{};
@@ -1742,7 +1776,7 @@ IntegrateArgs Engine::integrate_args(int step_offset) const {
   return a;
 }
 
-void Engine::enqueue_step(int step_offset) {
+void Engine::enqueue_step(int step_offset, int group) {
   compute_forces(false, integ_->integration_force_groups, true, step_offset);
   IntegrateArgs a = integrate_args(step_offset);
   a.zero_force = 1;
@@ -1754,6 +1788,16 @@ void Engine::enqueue_step(int step_offset) {
     a.block_center = nl_.block_center;
     a.qscaled = qscaled_;
     a.pbox = nl_.box;
+  }
+  if (gb_packed_by_integrator()) {
+    a.gb_posq = gb_.posq;
+    a.gb_posq_double = dp_ ? 1 : 0;
+    a.gb_slot = gb_.atom_slot;
+  }
+  if (capturing_ && nb_periodic_ && step_offset + 1 < group) {  // the next step's rebuild condition
+    rebuild_condition_ = new_condition();
+    a.has_condition = 1;
+    a.condition = rebuild_condition_;
   }
   prof_begin("integrate");
   launch_integrate(a, stream_);
@@ -1781,26 +1825,26 @@ void Engine::pack_slots(const double* pos, cudaStream_t s, const int* only_after
                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, s, only_after_rebuild);
 }
 
-void Engine::run_graph_steps(int launches) {
-  const int k = graph_steps_;
-  if (!graph_exec_) {
+void Engine::run_graph_steps(StepGraph& g, int k, int launches) {
+  if (!g.exec) {
     OMMB200_CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     capturing_ = true;
     try {
-      for (int s = 0; s < k; ++s) enqueue_step(s);
+      for (int s = 0; s < k; ++s) enqueue_step(s, k);
       launch_advance_counter(rng_step_, k, stream_);
     } catch (...) {
       capturing_ = false;
-      cudaGraph_t g = nullptr;
-      cudaStreamEndCapture(stream_, &g);
-      if (g) cudaGraphDestroy(g);
+      cudaGraph_t broken = nullptr;
+      cudaStreamEndCapture(stream_, &broken);
+      if (broken) cudaGraphDestroy(broken);
       throw;
     }
     capturing_ = false;
-    OMMB200_CK(cudaStreamEndCapture(stream_, &graph_));
-    OMMB200_CK(cudaGraphInstantiate(&graph_exec_, graph_, cudaGraphInstantiateFlagUseNodePriority));
+    OMMB200_CK(cudaStreamEndCapture(stream_, &g.graph));
+    OMMB200_CK(cudaGraphInstantiate(&g.exec, g.graph, cudaGraphInstantiateFlagUseNodePriority));
+    g.steps = k;
   }
-  for (int i = 0; i < launches; ++i) OMMB200_CK(cudaGraphLaunch(graph_exec_, stream_));
+  for (int i = 0; i < launches; ++i) OMMB200_CK(cudaGraphLaunch(g.exec, stream_));
 }
 
 void Engine::step(int steps) {
@@ -1839,14 +1883,29 @@ void Engine::run_steps(int steps) {
     const bool guarded = nb_periodic_;
     if (guarded) save_dynamic_state(step_snapshot_);
     int remaining = steps;
-    if (opt_.use_graph && !profiling_ && steps >= k) {
-      if (graph_steps_ != k) destroy_graph();
-      graph_steps_ = k;
-      run_graph_steps(steps / k);
-      remaining = steps % k;
+    if (opt_.use_graph && !profiling_) {
+      // Groups of k steps, and single steps for the rest, each from its own graph.  A group's
+      // graph takes about k times as long to capture and instantiate as a step's, which an
+      // accepted barostat move throws away again (the launches carry the box): under a barostat
+      // it is captured once the box has held for kStepsBeforeGroup steps (8,217 particles, a move
+      // every 25 steps: 50 steps and a state 8.4 -> 5.9 ms).
+      if (group_graph_.exec && group_graph_.steps != k) destroy_graph();
+      if (bar_def_ && !group_graph_.exec) {
+        const int singles =
+            (int)std::min<int64_t>(remaining, std::max<int64_t>(0, kStepsBeforeGroup - steps_since_capture_));
+        if (singles > 0) run_graph_steps(step_graph_, 1, singles);
+        remaining -= singles;
+      }
+      if (remaining >= k) {
+        run_graph_steps(group_graph_, k, remaining / k);
+        remaining %= k;
+      }
+      if (remaining > 0) run_graph_steps(step_graph_, 1, remaining);
+      remaining = 0;
+      steps_since_capture_ += steps;
     }
     for (int s = 0; s < remaining; ++s) {
-      enqueue_step(0);
+      enqueue_step(0, 1);
       launch_advance_counter(rng_step_, 1, stream_);
     }
     OMMB200_CK(cudaGetLastError());

@@ -43,6 +43,9 @@ constexpr int kDefaultCullTiles = 64;
 constexpr double kCullMinTilesPerWarp = 40.0;
 constexpr int kTunedCullTiles[] = {0, 4, 8, 16, 32, 64};
 
+// Under a barostat, steps with an unchanged box before a group of steps is captured.
+constexpr int kStepsBeforeGroup = 100;
+
 class DeviceArena {
  public:
   ~DeviceArena();
@@ -168,7 +171,8 @@ class Engine {
   std::function<void(cudaStream_t)> with_new_list(const NlistArgs& list);
   void pack_slots(const double* pos, cudaStream_t s, const int* only_after_rebuild = nullptr);
   void build_static_tiles();
-  void enqueue_conditional_rebuild();
+  cudaGraphConditionalHandle new_condition();  // of the graph being captured
+  void enqueue_conditional_rebuild(bool first);
   void enqueue_conditional_body(cudaGraphConditionalHandle handle,
                                 const std::function<void(cudaStream_t)>& body);
   // The pair kernel runs on the pruned list: periodic rectangular boxes whose rebuild packs 16
@@ -192,9 +196,16 @@ class Engine {
   void upload_nonbonded_parameters(const NonbondedDef& nb);
   std::vector<long long> evaluate(bool energy, uint32_t groups, double* forces,
                                   const std::function<void()>& outputs = {});
-  void enqueue_step(int step_offset);
+  // One step of a group of `group` (1 outside a captured group).
+  void enqueue_step(int step_offset, int group);
   void run_steps(int steps);
-  void run_graph_steps(int graph_launches);
+  struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    int steps = 0;
+  };
+  // Launches the graph of k steps `launches` times, capturing it first where needed.
+  void run_graph_steps(StepGraph& g, int k, int launches);
   // MonteCarloBarostat (forces/barostat.rs, context/program.rs:5-47)
   void setup_barostat(BarostatDef& def);
   void barostat_move();
@@ -217,7 +228,9 @@ class Engine {
   void sync();
   void destroy_graph();
   template <class Real>
-  void enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs);
+  void enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
+                         int step_offset, cudaStream_t direct_stream);
+  bool gb_packed_by_integrator() const;
   void prof_begin(const char* name);
   void prof_end();
   void harvest_profile();
@@ -370,9 +383,9 @@ class Engine {
   int regrows_ = 0;                 // neighbour-list capacity increases so far
 
   // graph
-  cudaGraph_t graph_ = nullptr;
-  cudaGraphExec_t graph_exec_ = nullptr;
-  int graph_steps_ = 0;
+  StepGraph group_graph_, step_graph_;
+  int64_t steps_since_capture_ = 0;  // steps run since the graphs were last dropped
+  cudaGraphConditionalHandle rebuild_condition_{};  // of the next step being captured
 
   // profiling
   bool profiling_ = false;

@@ -675,6 +675,7 @@ __global__ void gb_radii(const GbArgs a) {
                               ? (double)a.short_sum[atom] * kBornScaleInv + (double)a.tail[atom] +
                                     (double)a.seg_offset[a.atom_segment[atom]]
                               : (double)a.born_sum[atom] * kBornScaleInv;
+  if (!a.use_learned) a.born_sum[atom] = 0;  // for the next step; learned radii judge by it
   const double psi = 0.5 * offset * integral;
   const double t = tanh(psi - 0.8 * psi * psi + 4.85 * psi * psi * psi);
   const double R = 1.0 / (1.0 / offset - t / rho);
@@ -710,6 +711,7 @@ __global__ void gb_chain(const GbArgs a) {
   }
   const double R = a.born_radius[atom];
   const double total = a.dedr_self[atom] + (double)a.dedr_sum[atom] * kForceScaleInv;
+  a.dedr_sum[atom] = 0;  // for the next step
   dedr[s] = (Real)(total * R * R * a.chain[atom]);
 }
 

@@ -186,7 +186,10 @@ __device__ __forceinline__ void check_rebuild(const IntegrateArgs& a, const Step
                                               const double x[3]) {
   if (!a.pos_ref) return;
   const double dx = x[0] - t.ref[0], dy = x[1] - t.ref[1], dz = x[2] - t.ref[2];
-  if (dx * dx + dy * dy + dz * dz > a.half_skin2) *a.rebuild = 1;
+  if (dx * dx + dy * dy + dz * dz > a.half_skin2) {
+    *a.rebuild = 1;
+    if (a.has_condition) cudaGraphSetConditional(a.condition, 1u);
+  }
   if (!a.pos_prune) return;
   const double px = x[0] - t.prune_ref[0], py = x[1] - t.prune_ref[1], pz = x[2] - t.prune_ref[2];
   if (px * px + py * py + pz * pz > a.half_margin2) *a.prune = 1;
@@ -204,6 +207,21 @@ __device__ __forceinline__ void write_packed(const IntegrateArgs& a, const StepT
   else
     reinterpret_cast<float4*>(a.posq)[t.slot] =
         make_float4((float)r[0], (float)r[1], (float)r[2], (float)q);
+}
+
+// The GB passes' packed coordinates of `atom` at its new position (gb_pack's conversion); the
+// charge beside them stays.
+__device__ __forceinline__ void write_gb_packed(const IntegrateArgs& a, int atom,
+                                                const double x[3]) {
+  if (!a.gb_posq) return;
+  const int slot = a.gb_slot[atom];
+  if (a.gb_posq_double) {
+    st3(reinterpret_cast<double*>(a.gb_posq) + slot, slot, x);  // 4 slot + 0, 1, 2
+  } else {
+    float* p = reinterpret_cast<float*>(a.gb_posq) + 4 * slot;
+    *reinterpret_cast<float2*>(p) = make_float2((float)x[0], (float)x[1]);
+    p[2] = (float)x[2];
+  }
 }
 
 // drift / thermostat / drift for one particle (langevin.rs:121-134 without the kick)
@@ -277,6 +295,7 @@ __device__ void water_step_lanes(const IntegrateArgs& a, int w, int k, uint64_t 
   st3(a.pos, atom, xo);
   st3(a.vel, atom, wk);
   write_packed(a, tail, qk, xo);
+  write_gb_packed(a, atom, xo);
   check_rebuild(a, tail, xo);
 }
 
@@ -295,6 +314,7 @@ __device__ void free_step(const IntegrateArgs& a, int atom, uint64_t step, int n
   st3(a.pos, atom, x);
   st3(a.vel, atom, v);
   write_packed(a, tail, q, x);
+  write_gb_packed(a, atom, x);
   check_rebuild(a, tail, x);
 }
 
@@ -381,6 +401,7 @@ __device__ void cluster_step(const IntegrateArgs& a, int c, uint64_t step, int n
     StepTail tail{};
     load_tail(a, atom, tail);
     write_packed(a, tail, a.posq ? a.qscaled[atom] : 0.0, x);
+    write_gb_packed(a, atom, x);
     check_rebuild(a, tail, x);
   }
 }

@@ -256,6 +256,7 @@ struct GbArgs {
   int n_atoms, n_slots, n_tiles;
   const int2* tiles;          // (I, J), I <= J
   const int* slot_atom;       // [n_slots], -1 = padding
+  const int* atom_slot;       // [n_atoms]
   const int* block_segment;   // [n_slots / 32]
   const int* atom_segment;    // [n_atoms]
   const double* pos;
@@ -443,6 +444,14 @@ struct IntegrateArgs {
   const double* block_center;
   const double* qscaled;
   Box<double> pbox;
+  // GBSA without a cutoff: the next step's packed GB coordinates (x, y, z of each slot)
+  void* gb_posq;                  // float4 or double4 per slot (may be null)
+  int gb_posq_double;
+  const int* gb_slot;             // slot of each particle
+  // inside a captured group of steps: the next step's conditional neighbour-list rebuild, set
+  // together with `rebuild`
+  int has_condition;
+  cudaGraphConditionalHandle condition;
 };
 void launch_integrate(const IntegrateArgs& a, cudaStream_t s);
 // Barostat volume move: positions scaled, per particle or per molecule (CSR lists of atoms)

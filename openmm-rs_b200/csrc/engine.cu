@@ -480,11 +480,23 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
     pme_k_ = mem_.alloc_bytes(2 * rs * gk);
     influence_ = mem_.alloc_bytes(rs * gk);
     moduli_ = mem_.alloc<double>(grid_[0] + grid_[1] + grid_[2]);
-    // own transform while every axis factors into radices 2, 3, 4, 5, 7, 8 and the
-    // plane kernels' buffers fit in shared memory; cuFFT otherwise
+    // own transform while every axis factors into radices 2, 3, 4, 5, 7, 8 and at most one larger
+    // prime (the first stage) and the plane kernels' buffers fit in shared memory; cuFFT otherwise
     own_fft_ = true;
     for (int d = 0; d < 3; ++d) {
       int m = grid_[d], k = 0;
+      int prime = m;
+      for (int r : {2, 3, 5, 7})
+        while (prime % r == 0) prime /= r;
+      bool one = prime > 1;
+      for (int r = 11; r * r <= prime; ++r) one = one && prime % r != 0;
+      // where the direct sums beat cuFFT (three cubes of each size measured): cuFFT's own radices
+      // end at 11, and its way round larger primes is slow except for some even sizes past 65
+      // (39^3: 58 us against 23; 65^3: 65, 38; 95^3: 94, 65; but 68^3: 31, 44 and 104^3: 42, 86)
+      if (one && prime >= kMinFftPrime && prime <= kMaxFftPrime && (m <= 65 || (m <= 96 && m % 2))) {
+        fft_.rad[d][k++] = prime;
+        m /= prime;
+      }
       for (int r : {8, 4, 2, 3, 5, 7})
         while (m % r == 0 && k < 16) {
           fft_.rad[d][k++] = r;
@@ -498,7 +510,10 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
       const int ny = grid_[1], nz = grid_[2], nzh = nz / 2 + 1, nyp = (ny + 1) / 2;
       auto items = [&](int d, int pencils) {  // most butterflies of one stage of axis d
         int most = 0;
-        for (int k = 0; k < fft_.nrad[d]; ++k) most = std::max(most, pencils * grid_[d] / fft_.rad[d][k]);
+        for (int k = 0; k < fft_.nrad[d]; ++k) {
+          const int r = fft_.rad[d][k];  // a prime stage gives half a sub-transform's outputs each
+          most = std::max(most, pencils * grid_[d] / r * (r > 8 ? (r + 1) / 2 : 1));
+        }
         return most;
       };
       auto block = [](int want, int lo, int hi) { return std::min(hi, std::max(lo, (want + 31) / 32 * 32)); };

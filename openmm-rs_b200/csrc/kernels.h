@@ -221,6 +221,9 @@ void launch_pme_influence(Real* out, const double* moduli, int nx, int ny, int n
 // and the convolution kernel): per axis the radices of the Stockham stages and
 // the twiddle table W_n^m = exp(-2 pi i m / n), m < n (Real2 elements); block sizes of the
 // forward-plane, x-pass and inverse-plane kernels; kz pencils per x-pass CTA.
+// The prime factors above 7 an axis of the own transform may have, one of them, as a direct-sum
+// stage.
+constexpr int kMinFftPrime = 13, kMaxFftPrime = 31;
 struct PmeFft {
   int nrad[3];
   int rad[3][16];

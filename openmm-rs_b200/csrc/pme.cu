@@ -362,9 +362,9 @@ __global__ void gather_kernel(const PmeArgs<Real> a) {
 //   planes_inverse  one CTA per x plane: inverse y transform, inverse z transform of two
 //                   Hermitian rows at once, real rows -> potential grid for the gather
 // Every 1-D transform is a mixed-radix Stockham FFT in shared memory (radices 2, 3, 4, 5, 7,
-// 8; one radix-R butterfly per thread and stage), forward sign exp(-2 pi i jk/n) and
-// unnormalised like cuFFT; the inverse is conj(F(conj(x))).  Sizes with other prime factors
-// use cuFFT.
+// 8; one radix-R butterfly per thread and stage; one larger prime as the first stage, by direct
+// sums), forward sign exp(-2 pi i jk/n) and unnormalised like cuFFT; the inverse is
+// conj(F(conj(x))).  Sizes with other prime factors use cuFFT.
 template <class C2>
 __device__ __forceinline__ C2 cmul(C2 a, C2 w) {
   C2 r;
@@ -478,6 +478,42 @@ __device__ __noinline__ void stockham_stage(const C2* in, C2* out, const C2* tw,
   }
 }
 
+// First stage (ns = 1) for a prime radix R > 7: outputs m and R - m of a sub-transform are the
+// sum and difference of the same four real sums over its R inputs, so a thread that owns both
+// spends 4 multiply-adds and two shared loads (one of them a broadcast: the lanes of a warp
+// mostly share their inputs) per input instead of 8 and four.
+template <class C2>
+__device__ __noinline__ void stockham_prime(const C2* in, C2* out, const C2* tw, int n, int R, int P) {
+  using S = decltype(in->x);
+  const int nr = n / R, nh = (R + 1) / 2, items = P * nr * nh;
+  for (int t = threadIdx.x; t < items; t += blockDim.x) {
+    const int pj = t / nh, m = t - pj * nh, p = pj / nr, j = pj - p * nr;
+    const C2* src = in + p * n + j;
+    C2* dst = out + p * n + j * R;
+    const C2 v0 = src[0];
+    S xc = v0.x, yc = v0.y, xs = 0, ys = 0;  // sums of x cos, y cos, x sin, y sin
+    const int step = m * nr;
+    int w = 0;
+#pragma unroll 4
+    for (int r = 1; r < R; ++r) {
+      w += step;
+      w -= w >= n ? n : 0;
+      const C2 v = src[r * nr], e = tw[w];  // e = (cos, -sin)
+      xc += v.x * e.x;
+      yc += v.y * e.x;
+      xs += v.x * e.y;
+      ys += v.y * e.y;
+    }
+    C2 a, b;
+    a.x = xc - ys;
+    a.y = yc + xs;
+    b.x = xc + ys;
+    b.y = yc - xs;
+    dst[m] = a;
+    if (m) dst[R - m] = b;
+  }
+}
+
 // Forward transform of P pencils held in a (b: scratch of the same size); returns the buffer
 // that holds the result.  The callers synchronise before and after.
 template <class C2>
@@ -491,7 +527,8 @@ __device__ C2* stockham(C2* a, C2* b, const C2* tw, const PmeFft& f, int axis, i
       case 4: stockham_stage<4>(a, b, tw, n, ns, P); break;
       case 5: stockham_stage<5>(a, b, tw, n, ns, P); break;
       case 7: stockham_stage<7>(a, b, tw, n, ns, P); break;
-      default: stockham_stage<8>(a, b, tw, n, ns, P); break;
+      case 8: stockham_stage<8>(a, b, tw, n, ns, P); break;
+      default: stockham_prime(a, b, tw, n, R, P); break;  // always the first stage
     }
     __syncthreads();
     C2* t = a;

@@ -1,0 +1,66 @@
+"""PME on grids whose axes hold one larger prime factor (the direct-sum first stage of the own
+transform) against the f64 oracle (pme.rs:141-425)."""
+import numpy as np
+import pytest
+
+import oracle as O
+import ommb200
+from ommb200 import systems
+
+pytestmark = pytest.mark.gpu
+
+ALPHA = 3.0
+
+
+def ions(n, box, seed):
+    """Alternating unit charges, jittered about a lattice, with a weak LJ core."""
+    rng = np.random.default_rng(seed)
+    k = int(np.ceil(n ** (1.0 / 3.0)))
+    site = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    pos = (site + 0.5 + rng.uniform(-0.2, 0.2, site.shape)) / k * box
+    pos += rng.integers(-1, 2, site.shape) * box  # any lattice image is a position
+    q = np.where(np.arange(n) % 2 == 0, 1.0, -1.0) * rng.uniform(0.2, 1.0, n)
+    return pos, q
+
+
+def system(n, q, box, grid, exceptions=()):
+    s = ommb200.System()
+    s.set_default_periodic_box_vectors(*np.diag(box))
+    nb = ommb200.NonbondedForce()
+    nb.set_nonbonded_method("PME")
+    nb.set_cutoff_distance(0.8)
+    nb.set_pme_parameters(ALPHA, *grid)
+    nb.set_use_dispersion_correction(False)
+    nb.set_reciprocal_space_force_group(1)
+    for i in range(n):
+        s.add_particle(20.0)
+        nb.add_particle(float(q[i]), 0.2, 0.1)
+    s.add_force(nb)
+    return s
+
+
+def check(n, box, grid, precision, **options):
+    box = np.asarray(box)
+    pos, q = ions(n, box, seed=n + grid[0])
+    ctx = ommb200.Context(system(n, q, box, grid), systems.langevin(seed=3), precision=precision,
+                          **options)
+    ctx.set_positions(pos)
+    st = ctx.get_state(forces=True, energy=True, groups=1 << 1)
+    f_ref, e_ref = O.nonbonded(pos, q, np.full(n, 0.2), np.zeros(n), method="PME", cutoff=0.8,
+                               box=np.diag(box), pme=(ALPHA, grid), include_direct=False,
+                               use_dispersion_correction=False)
+    err = np.sqrt(((st.forces - f_ref) ** 2).sum() / (f_ref ** 2).sum())
+    bound = 5e-6 if precision == "mixed" else 1e-9
+    assert err < bound
+    assert abs(st.potential_energy - e_ref) < bound * max(abs(e_ref), 1.0)
+    ctx.close()
+    return st
+
+
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+@pytest.mark.parametrize("grid", [(11, 13, 17), (22, 26, 33), (19, 23, 29), (31, 24, 39), (62, 58, 46),
+                                  (37, 22, 25)])
+@pytest.mark.parametrize("bricks", [-1, 0])
+def test_prime_grids(grid, precision, bricks):
+    # 11 and 37 are outside the own transform's primes
+    check(350, (1.7, 2.1, 1.9), grid, precision, pme_bricks=bricks)

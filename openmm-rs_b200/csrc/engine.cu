@@ -390,9 +390,9 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
     a.zkey = mem_.alloc<float>(n_);
     a.col_count = mem_.alloc<int>(a.n_cols);
     a.col_start = mem_.alloc<int>(a.n_cols + 1);
-    a.col_scatter = mem_.alloc<int>(a.n_cols + 1);
-    a.col_cursor = mem_.alloc<int>(a.n_cols);
-    a.scratch_atoms = mem_.alloc<int>(n_);
+    a.col_size = mem_.alloc<int>(a.n_cols);
+    a.bins = mem_.alloc<int>((size_t)a.n_cols * a.col_max);
+    a.done = mem_.alloc<unsigned>(2);
     const long long blocks = a.slot_capacity / 32;
     // sized for the largest skin the autotuner may pick
     const double reach = nb.cutoff + std::max(skin_, kMaxTunedSkin);
@@ -430,6 +430,8 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
   a.slot_wpos = mem_.alloc<double4>(n_slots_);
   a.block_center = mem_.alloc<double>(3 * (size_t)n_blocks_);
   a.block_half = mem_.alloc<double>(3 * (size_t)n_blocks_);
+  a.block_radius = mem_.alloc<double>(n_blocks_);
+  a.slot_local = mem_.alloc<float4>(n_slots_);
   if (nb_periodic_) {  // replaced by the first rebuild
     std::vector<int> sorted(n_slots_, -1);
     for (int i = 0; i < n_; ++i) sorted[i] = i;
@@ -460,6 +462,11 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
   }
   posq_ = mem_.alloc_bytes((dp_ ? 32 : 16) * (size_t)n_slots_);
   ljp_ = mem_.alloc_bytes((dp_ ? 16 : 8) * (size_t)n_slots_);
+  a.qscaled = qscaled_;
+  a.half_sigma = half_sigma_;
+  a.two_sqrt_eps = sqrt_eps_;
+  a.posq = posq_;
+  a.ljp = ljp_;
   if (!nb_periodic_) build_static_tiles();
   int dev_sms = 148;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, opt_.device);
@@ -1176,6 +1183,12 @@ void Engine::update_box_dependents() {
     const long long expected = (long long)std::ceil(2.0 * cand_scale_ * cols * per_column);
     const long long cand = std::min(bound, expected);
     if (cand * 48 <= 200 * 1024) nl_.max_cand = (int)cand;
+    // the CTA builder gives every tile the mask slot of its own index (a box that was triclinic
+    // at creation has fewer)
+    if (nl_.mask_capacity < nl_.tile_capacity) {
+      nl_.mask_capacity = nl_.tile_capacity;
+      nl_.masks = mem_.alloc<uint32_t>(32 * (size_t)nl_.mask_capacity);
+    }
   }
   for (auto& L : bonded_) L.args.box = make_box(box_);
   gb_.boxd = make_box(box_);
@@ -1281,6 +1294,7 @@ bool Engine::grow_neighbor_capacity() {
   // per-column sort: the keys of one column live in shared memory, at most 4096
   if (a.col_max < 4096) {
     a.col_max = std::min(4096, 2 * a.col_max);
+    a.bins = mem_.alloc<int>((size_t)a.n_cols * a.col_max);
     grew = true;
   }
   // tiles and masks: half again as many as the failed build asked for (it counts its whole
@@ -1295,8 +1309,12 @@ bool Engine::grow_neighbor_capacity() {
     a.entries = mem_.alloc_bytes((size_t)(dp_ ? 32 : 16) * 32 * (size_t)a.tile_capacity);
     grew = true;
   }
-  const long long want_masks = std::min<long long>(
-      a.tile_capacity, std::max<long long>(3LL * demand_masks / 2, 3LL * a.mask_capacity / 2));
+  // rectangular boxes: one mask slot per tile
+  const bool rectangular = box_[3] == 0.0 && box_[6] == 0.0 && box_[7] == 0.0;
+  const long long want_masks =
+      rectangular ? a.tile_capacity
+                  : std::min<long long>(a.tile_capacity, std::max<long long>(3LL * demand_masks / 2,
+                                                                             3LL * a.mask_capacity / 2));
   if (want_masks > a.mask_capacity) {
     a.mask_capacity = (int)want_masks;
     a.masks = mem_.alloc<uint32_t>(32 * (size_t)a.mask_capacity);
@@ -1827,17 +1845,16 @@ bool Engine::packed_by_integrator() const { return nb_ && nb_periodic_ && segmen
 std::function<void(cudaStream_t)> Engine::with_new_list(const NlistArgs& list) {
   return [this, list](cudaStream_t s) {
     if (use_bricks_) launch_pme_brick_ranges(list, bricks_, s);
-    if (packed_by_integrator()) pack_slots(list.pos, s, list.rebuild);
   };
 }
 
-void Engine::pack_slots(const double* pos, cudaStream_t s, const int* only_after_rebuild) {
+void Engine::pack_slots(const double* pos, cudaStream_t s) {
   if (dp_)
     launch_pack<double>(n_slots_, nl_.sorted_atom, pos, nl_.image, nl_.block_center, qscaled_,
-                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, s, only_after_rebuild);
+                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, s);
   else
     launch_pack<float>(n_slots_, nl_.sorted_atom, pos, nl_.image, nl_.block_center, qscaled_,
-                       half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, s, only_after_rebuild);
+                       half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, s);
 }
 
 void Engine::run_graph_steps(StepGraph& g, int k, int launches) {

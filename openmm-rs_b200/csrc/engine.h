@@ -167,9 +167,9 @@ class Engine {
   void update_box_dependents();
   void update_bricks();
   bool packed_by_integrator() const;
-  // the launches that follow a neighbour-list build of `list` (brick ranges, gated pack)
+  // the launches that join a neighbour-list build of `list` (brick ranges)
   std::function<void(cudaStream_t)> with_new_list(const NlistArgs& list);
-  void pack_slots(const double* pos, cudaStream_t s, const int* only_after_rebuild = nullptr);
+  void pack_slots(const double* pos, cudaStream_t s);
   void build_static_tiles();
   cudaGraphConditionalHandle new_condition();  // of the graph being captured
   void enqueue_conditional_rebuild(bool first);

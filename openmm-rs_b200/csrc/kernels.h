@@ -32,16 +32,23 @@ struct NlistArgs {
   int* column;        // [N] x-y column of each particle
   float* zkey;        // [N] wrapped z of each particle
   int* col_count;     // [n_cols] particles per column (zero between rebuilds)
+  int* col_size;      // [n_cols] particles per column at the last rebuild
   int* col_start;     // [n_cols + 1] first slot of each column (columns padded to blocks)
-  int* col_scatter;   // [n_cols + 1] unpadded prefix, for the scatter
-  int* col_cursor;    // [n_cols] scatter cursor (zero between rebuilds)
-  int* scratch_atoms; // [N] unordered scatter
+  int* bins;          // [n_cols * col_max] particles of each column, unordered
+  unsigned* done;     // [2] CTAs done of the column and list kernels (zero between launches)
   int* n_blocks;      // device: blocks in use after the last rebuild
   int* sorted_atom;   // [slot_capacity] particle in each slot, -1 for padding
   int* atom_slot;     // [N] inverse of sorted_atom
   double4* slot_wpos;    // [slot_capacity] wrapped rebuild position of each slot (w = 0)
   double* block_center;  // [3 * slot_capacity / 32]
   double* block_half;    // [3 * slot_capacity / 32] half extents of the bounding box
+  double* block_radius;  // [slot_capacity / 32] their norm
+  float4* slot_local;    // [slot_capacity] rebuild position relative to the block's centre
+  const double* qscaled; // [N] parameters of the pair kernel's packed particles
+  const double* half_sigma;
+  const double* two_sqrt_eps;
+  void* posq;            // [slot_capacity] float4/double4: packed by every rebuild
+  void* ljp;             // [slot_capacity] float2/double2
   int4* tiles;           // [tile_capacity] (I, flags, mask_slot, 0)
   void* entries;         // [32 * tile_capacity] float4/double4: shift xyz, slot (as int bits
                          //   for float4, as a double for double4); slot -1 = padding
@@ -87,11 +94,11 @@ struct PruneArgs {
   unsigned long long* prune_count;
 };
 
-// `with_list` (may be empty) enqueues launches that need the new list and must run only on a
-// rebuild: it is called after the list is built and before the rebuild flag clears, so its
-// kernels can gate on the flag (the brick gather's slot ranges, the pack of the new slots).
+// `with_columns` (may be empty) enqueues launches that need the new columns and slots and must
+// run only on a rebuild: it is called after the sort and before the list kernel, which clears the
+// rebuild flag, so its kernels can gate on the flag (the brick gather's slot ranges).
 void launch_nlist_rebuild(const NlistArgs& a, bool double_entries, cudaStream_t s,
-                          const std::function<void(cudaStream_t)>& with_list = {});
+                          const std::function<void(cudaStream_t)>& with_columns = {});
 void launch_nlist_prune(const NlistArgs& a, const PruneArgs& p, bool double_entries,
                         cudaStream_t s);
 // Sets `handle` to whether a prune is pending (the graph form of the early-exit prune kernels).
@@ -149,14 +156,12 @@ template <class Real>
 void launch_pair(const PairArgs<Real>& a, int elec, bool energy, bool dump, int grid,
                  cudaStream_t s);
 
-// Packing of block-local coordinates and LJ parameters into the sorted slots; with
-// `only_after_rebuild` set, only when that rebuild flag is set (between rebuilds of a periodic
-// list the integrator writes the packed coordinates).
+// Packing of block-local coordinates and LJ parameters into the sorted slots.
 template <class Real>
 void launch_pack(int n_slots, const int* sorted_atom, const double* pos, const int* image,
                  const double* block_center, const double* qscaled, const double* half_sigma,
                  const double* two_sqrt_eps, void* posq, void* ljp, const Box<double>& box,
-                 cudaStream_t s, const int* only_after_rebuild = nullptr);
+                 cudaStream_t s);
 
 // ---- PME -------------------------------------------------------------------------------
 template <class Real>

@@ -42,101 +42,115 @@ __device__ __forceinline__ int aggregated_add(int* counter, int key) {
   return base + __popc(peers & ((1u << lane) - 1u));
 }
 
-__global__ void nl_columns(NlistArgs a) {
+// A rebuild is three launches (plus the brick gather's slot ranges on large grids): columns and
+// their scan, the per-column sort with everything that follows from one column alone, and the
+// list.  Between them they replace ten (counting, scan, scatter, sort, bounds, list, pack,
+// clean-up, flag), each of which took 2-4 us of a small box's step for its launch and its first
+// loads.  With the FP32 particle tests of the list kernel, a rebuild's share of a step (one in four
+// or five rebuilds): 1,524 particles 28 -> 12 us with the launches of an idle rebuild, 8,217
+// particles 37 -> 17 us, 23,958 particles 37 -> 18 us; 255,477 particles 125 -> 92 us.
+
+// True in every thread of the last CTA of the launch to get here; `counter` is left at zero.
+__device__ __forceinline__ bool last_cta(unsigned* counter) {
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1 : 0;
+    if (s_last) *counter = 0u;
+  }
+  __syncthreads();
+  __threadfence();
+  return s_last != 0;
+}
+
+// Bins the particles into columns (in any order: the sort orders them), then, in the last CTA to
+// finish, the scan over the columns: block-padded slot starts, column sizes, block count.
+__global__ void __launch_bounds__(256) nl_columns(NlistArgs a) {
   if (*a.rebuild == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * 256 + threadIdx.x;
   if (i == 0) {
     *a.n_tiles = 0;
     *a.n_masks = 0;
   }
-  if (i >= a.n_atoms) return;
-  double x = a.pos[3 * i], y = a.pos[3 * i + 1], z = a.pos[3 * i + 2];
-  a.pos_ref[3 * i] = x;
-  a.pos_ref[3 * i + 1] = y;
-  a.pos_ref[3 * i + 2] = z;
-  const Box<double>& b = a.box;
-  const double n2 = floor(z * b.inv_cz);
-  z -= n2 * b.cz;
-  y -= n2 * b.cy;
-  x -= n2 * b.cx;
-  const double n1 = floor(y * b.inv_by);
-  y -= n1 * b.by;
-  x -= n1 * b.bx;
-  const double n0 = floor(x * b.inv_ax);
-  x -= n0 * b.ax;
-  a.image[3 * i] = (int)n0;
-  a.image[3 * i + 1] = (int)n1;
-  a.image[3 * i + 2] = (int)n2;
-  const int cx = min(max((int)(x * b.inv_ax * a.n_col[0]), 0), a.n_col[0] - 1);
-  const int cy = min(max((int)(y * b.inv_by * a.n_col[1]), 0), a.n_col[1] - 1);
-  const int col = cy * a.n_col[0] + cx;
-  a.column[i] = col;
-  a.zkey[i] = fmaxf((float)z, 0.0f);
-  aggregated_add(&a.col_count[col], col);
-}
-
-// Single-CTA scan over the columns: padded slot starts, unpadded scatter starts, block count.
-__global__ void __launch_bounds__(1024) nl_col_scan(NlistArgs a) {
-  if (*a.rebuild == 0) return;
-  __shared__ int ps[1024], pu[1024];
-  const int t = threadIdx.x;
-  const int chunk = (a.n_cols + 1023) / 1024;
+  if (i < a.n_atoms) {
+    double x = a.pos[3 * i], y = a.pos[3 * i + 1], z = a.pos[3 * i + 2];
+    a.pos_ref[3 * i] = x;
+    a.pos_ref[3 * i + 1] = y;
+    a.pos_ref[3 * i + 2] = z;
+    const Box<double>& b = a.box;
+    const double n2 = floor(z * b.inv_cz);
+    z -= n2 * b.cz;
+    y -= n2 * b.cy;
+    x -= n2 * b.cx;
+    const double n1 = floor(y * b.inv_by);
+    y -= n1 * b.by;
+    x -= n1 * b.bx;
+    const double n0 = floor(x * b.inv_ax);
+    x -= n0 * b.ax;
+    a.image[3 * i] = (int)n0;
+    a.image[3 * i + 1] = (int)n1;
+    a.image[3 * i + 2] = (int)n2;
+    const int cx = min(max((int)(x * b.inv_ax * a.n_col[0]), 0), a.n_col[0] - 1);
+    const int cy = min(max((int)(y * b.inv_by * a.n_col[1]), 0), a.n_col[1] - 1);
+    const int col = cy * a.n_col[0] + cx;
+    a.column[i] = col;
+    a.zkey[i] = fmaxf((float)z, 0.0f);
+    const int at = aggregated_add(&a.col_count[col], col);
+    if (at < a.col_max) a.bins[(size_t)col * a.col_max + at] = i;
+  }
+  if (!last_cta(a.done)) return;
+  __shared__ int s_warp[8];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int chunk = (a.n_cols + 255) / 256;
   const int lo = min(t * chunk, a.n_cols), hi = min(lo + chunk, a.n_cols);
-  int sp = 0, su = 0;
+  int sum = 0;
   for (int c = lo; c < hi; ++c) {
-    const int n = a.col_count[c];
+    const int n = __ldcg(a.col_count + c);
     if (n > a.col_max) report_status(a.status, kStatusTileOverflow);
-    sp += (n + 31) & ~31;
-    su += n;
+    a.col_size[c] = n;
+    a.col_count[c] = 0;  // for the next rebuild
+    sum += (n + 31) & ~31;
   }
-  ps[t] = sp;
-  pu[t] = su;
+  int incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[w] = incl;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const int vp = t >= off ? ps[t - off] : 0, vu = t >= off ? pu[t - off] : 0;
-    __syncthreads();
-    ps[t] += vp;
-    pu[t] += vu;
-    __syncthreads();
-  }
-  int rp = ps[t] - sp, ru = pu[t] - su;
+  int start = incl - sum;
+  for (int u = 0; u < w; ++u) start += s_warp[u];
   for (int c = lo; c < hi; ++c) {
-    a.col_start[c] = rp;
-    a.col_scatter[c] = ru;
-    const int n = a.col_count[c];
-    rp += (n + 31) & ~31;
-    ru += n;
+    a.col_start[c] = start;
+    start += (a.col_size[c] + 31) & ~31;
   }
-  const int total = min(ps[1023], a.slot_capacity);
-  if (t == 0) {
+  if (t == 255) {
+    const int total = min(start, a.slot_capacity);
     a.col_start[a.n_cols] = total;
-    a.col_scatter[a.n_cols] = pu[1023];
     *a.n_blocks = total / 32;
   }
-  for (int s = total + t; s < a.slot_capacity; s += 1024) a.sorted_atom[s] = -1;
 }
 
-__global__ void nl_col_scatter(NlistArgs a) {
-  if (*a.rebuild == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n_atoms) return;
-  const int c = a.column[i];
-  a.scratch_atoms[a.col_scatter[c] + aggregated_add(&a.col_cursor[c], c)] = i;
-}
-
-// One CTA per column: bitonic sort of (z, particle) keys in shared memory.
+// One CTA per column: bitonic sort of (z, particle) keys in shared memory, then one warp per
+// 32-slot block of the column: its slots, the bounding box of its particles' wrapped positions,
+// their positions relative to the box's centre, and the pair kernel's packed particles.
+template <bool kDouble>
 __global__ void __launch_bounds__(256) nl_col_sort(NlistArgs a) {
   if (*a.rebuild == 0) return;
   extern __shared__ unsigned long long keys[];
   const int c = blockIdx.x;
-  const int n = a.col_count[c];
+  // the slots past the last column's, shared out over the CTAs
+  for (int s = a.col_start[a.n_cols] + c * 256 + threadIdx.x; s < a.slot_capacity;
+       s += gridDim.x * 256)
+    a.sorted_atom[s] = -1;
+  const int n = a.col_size[c];
   if (n > a.col_max || n == 0) return;
   int m = 1;
   while (m < n) m <<= 1;
-  const int s0 = a.col_scatter[c];
   for (int k = threadIdx.x; k < m; k += blockDim.x) {
     if (k < n) {
-      const int atom = a.scratch_atoms[s0 + k];
+      const int atom = a.bins[(size_t)c * a.col_max + k];
       keys[k] = ((unsigned long long)__float_as_uint(a.zkey[atom]) << 32) | (unsigned)atom;
     } else {
       keys[k] = ~0ull;
@@ -158,48 +172,65 @@ __global__ void __launch_bounds__(256) nl_col_sort(NlistArgs a) {
       }
       __syncthreads();
     }
-  const int base = a.col_start[c];
-  const int padded = (n + 31) & ~31;
-  for (int k = threadIdx.x; k < padded; k += blockDim.x) {
-    if (base + k >= a.slot_capacity) break;
-    if (k < n) {
-      const int atom = (int)(keys[k] & 0xffffffffu);
-      a.sorted_atom[base + k] = atom;
-      a.atom_slot[atom] = base + k;
+  const int base = a.col_start[c], lane = threadIdx.x & 31;
+  for (int k0 = 32 * (threadIdx.x >> 5); k0 < n; k0 += 256) {
+    if (base + k0 + 32 > a.slot_capacity) break;
+    const int slot = base + k0 + lane, blk = (base + k0) >> 5;
+    const int atom = k0 + lane < n ? (int)(keys[k0 + lane] & 0xffffffffu) : -1;
+    a.sorted_atom[slot] = atom;
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    double x[3] = {0.0, 0.0, 0.0}, im[3] = {0.0, 0.0, 0.0}, wp[3] = {0.0, 0.0, 0.0};
+    if (atom >= 0) {
+      a.atom_slot[atom] = slot;
+      const Box<double>& b = a.box;
+      for (int d = 0; d < 3; ++d) {
+        im[d] = a.image[3 * atom + d];
+        x[d] = a.pos_ref[3 * atom + d];
+      }
+      wp[0] = x[0] - (im[0] * b.ax + im[1] * b.bx + im[2] * b.cx);
+      wp[1] = x[1] - (im[1] * b.by + im[2] * b.cy);
+      wp[2] = x[2] - im[2] * b.cz;
+      for (int d = 0; d < 3; ++d) lo[d] = hi[d] = wp[d];
+      a.slot_wpos[slot] = make_double4(wp[0], wp[1], wp[2], 0.0);
+    }
+    for (int off = 16; off > 0; off >>= 1)
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], off));
+        hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], off));
+      }
+    double cen[3], half[3];
+    for (int d = 0; d < 3; ++d) {
+      cen[d] = 0.5 * (lo[d] + hi[d]);
+      half[d] = 0.5 * (hi[d] - lo[d]);
+    }
+    if (lane == 0) {
+      for (int d = 0; d < 3; ++d) {
+        a.block_center[3 * blk + d] = cen[d];
+        a.block_half[3 * blk + d] = half[d];
+      }
+      a.block_radius[blk] = sqrt(half[0] * half[0] + half[1] * half[1] + half[2] * half[2]);
+    }
+    a.slot_local[slot] =
+        atom >= 0 ? make_float4((float)(wp[0] - cen[0]), (float)(wp[1] - cen[1]),
+                                (float)(wp[2] - cen[2]), 0.f)
+                  : make_float4(0.f, 0.f, 0.f, 0.f);
+    // the pack kernel's arithmetic
+    double r[3] = {0.0, 0.0, 0.0}, q = 0.0, hs = 0.0, se = 0.0;
+    if (atom >= 0) {
+      block_local(x, im[0], im[1], im[2], cen, a.box, r);
+      q = a.qscaled[atom];
+      hs = a.half_sigma[atom];
+      se = a.two_sqrt_eps[atom];
+    }
+    if (kDouble) {
+      reinterpret_cast<double4*>(a.posq)[slot] = make_double4(r[0], r[1], r[2], q);
+      reinterpret_cast<double2*>(a.ljp)[slot] = make_double2(hs, se);
     } else {
-      a.sorted_atom[base + k] = -1;
+      reinterpret_cast<float4*>(a.posq)[slot] =
+          make_float4((float)r[0], (float)r[1], (float)r[2], (float)q);
+      reinterpret_cast<float2*>(a.ljp)[slot] = make_float2((float)hs, (float)se);
     }
   }
-}
-
-// One warp per block: bounding box of the wrapped rebuild positions.
-__global__ void nl_bounds(NlistArgs a) {
-  if (*a.rebuild == 0) return;
-  const int lane = threadIdx.x & 31;
-  const int blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (blk >= *a.n_blocks) return;
-  const int atom = a.sorted_atom[32 * blk + lane];
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  if (atom >= 0) {
-    const Box<double>& b = a.box;
-    const double n0 = a.image[3 * atom], n1 = a.image[3 * atom + 1], n2 = a.image[3 * atom + 2];
-    const double w[3] = {a.pos_ref[3 * atom] - (n0 * b.ax + n1 * b.bx + n2 * b.cx),
-                         a.pos_ref[3 * atom + 1] - (n1 * b.by + n2 * b.cy),
-                         a.pos_ref[3 * atom + 2] - n2 * b.cz};
-    for (int d = 0; d < 3; ++d) lo[d] = hi[d] = w[d];
-    a.slot_wpos[32 * blk + lane] = make_double4(w[0], w[1], w[2], 0.0);
-  }
-  for (int off = 16; off > 0; off >>= 1)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], off));
-      hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], off));
-    }
-  if (lane == 0)
-    for (int d = 0; d < 3; ++d) {
-      const bool empty = lo[d] > hi[d];
-      a.block_center[3 * blk + d] = empty ? 0.0 : 0.5 * (lo[d] + hi[d]);
-      a.block_half[3 * blk + d] = empty ? 0.0 : 0.5 * (hi[d] - lo[d]);
-    }
 }
 
 __device__ __forceinline__ double box_gap2(const double d[3], const double* hi, const double* hj) {
@@ -533,9 +564,15 @@ __global__ void __launch_bounds__(32 * kListWarps) nl_lists(NlistArgs a) {
   }
 }
 
+// The rebuild is done: the flag clears, and the pruned list must be made from the new tiles.
+__device__ __forceinline__ void close_rebuild(const NlistArgs& a) {
+  *a.rebuild = 0;
+  *a.rebuild_count += 1;
+  if (a.prune) *a.prune = 1;
+}
+
 // Rectangular boxes: one CTA of kCtaWarps warps per block I, in four phases.
-//   A  candidate blocks J > I of I's column neighbourhood whose boxes come within reach (the
-//      warps split the columns; two passes place every warp's candidates at fixed offsets)
+//   A  candidate blocks J > I of I's column neighbourhood whose boxes come within reach
 //   B  per candidate, the 32-bit masks of its particles within reach of each half of I (slots
 //      0-15 and 16-31; one warp per candidate; the conservative sphere test for blocks near a
 //      periodic image of I)
@@ -544,13 +581,17 @@ __global__ void __launch_bounds__(32 * kListWarps) nl_lists(NlistArgs a) {
 //   D  each warp fills whole tiles: entries, flags, and exclusion masks
 // Candidates, masks and prefix sums live in shared memory; I's tiles are reserved with one
 // atomic, so they are contiguous.  The selected particles and their order are a function of
-// the rebuild positions alone, so the tile contents are deterministic.
+// the rebuild positions alone, so the tile contents are deterministic.  The particle tests of
+// phase B run in FP32 on block-local coordinates with the reach widened by their rounding (a
+// pair's membership is decided by the pair kernel, so a list may hold more than it needs), half
+// the bytes and, on this path, a third of the arithmetic of the f64 form; tile t's masks are slot
+// t, which takes an atomic and its round trip out of every masked tile.  The last CTA to finish
+// closes the rebuild.
 constexpr int kCtaWarps = 8;
-constexpr int kStageRegs = 2;  // staged candidates per lane when phase A packs its regions
+constexpr int kCtaThreads = 32 * kCtaWarps;
 
 template <bool kDouble>
-__global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
-  if (*a.rebuild == 0) return;
+__device__ __forceinline__ void build_block_list(const NlistArgs& a, int I) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int cap = a.max_cand;
   double* c_d = reinterpret_cast<double*>(smem);                    // [3][cap]
@@ -558,45 +599,48 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
   int* c_un = c_J + cap;                                             // [cap]
   uint32_t* c_mask = reinterpret_cast<uint32_t*>(c_un + cap);        // [2][cap] per half of I
   int* c_pre = reinterpret_cast<int*>(c_mask + 2 * (size_t)cap);     // [2][cap + 1]
-  __shared__ int s_wcount[kCtaWarps], s_wbase[kCtaWarps + 1];
-  __shared__ int s_tile0, s_ntiles, s_spill;
+  __shared__ int s_wcount[kCtaWarps];
+  __shared__ int s_first[kCtaThreads], s_start[kCtaThreads + 1];
+  __shared__ int s_tile0, s_ntiles;
   __shared__ int s_slots[kCtaWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int nb = *a.n_blocks;
-  const int I = blockIdx.x;
-  if (I >= nb) return;
   const double reach = a.cutoff + a.skin;
   const double reach2 = reach * reach;
   const double ci[3] = {a.block_center[3 * I], a.block_center[3 * I + 1], a.block_center[3 * I + 2]};
   const double hi[3] = {a.block_half[3 * I], a.block_half[3 * I + 1], a.block_half[3 * I + 2]};
-  const double ri = sqrt(hi[0] * hi[0] + hi[1] * hi[1] + hi[2] * hi[2]);
+  const double ri = a.block_radius[I];
   const Box<double>& bx = a.box;
   // boxes of the two halves of I (slots 0-15 and 16-31), relative to I's centre
-  double hc[3], hh[3];
+  float hc[3], hh[3];
   {
     const int ai0 = a.sorted_atom[32 * I + lane];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, up[3] = {-INFINITY, -INFINITY, -INFINITY};
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, up[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (ai0 >= 0) {
-      const double4 wp = a.slot_wpos[32 * I + lane];
-      lo[0] = up[0] = wp.x - ci[0];
-      lo[1] = up[1] = wp.y - ci[1];
-      lo[2] = up[2] = wp.z - ci[2];
+      const float4 p = a.slot_local[32 * I + lane];
+      lo[0] = up[0] = p.x;
+      lo[1] = up[1] = p.y;
+      lo[2] = up[2] = p.z;
     }
     for (int o = 8; o > 0; o >>= 1)
       for (int d = 0; d < 3; ++d) {
-        lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], o));
-        up[d] = fmax(up[d], __shfl_xor_sync(kFull, up[d], o));
+        lo[d] = fminf(lo[d], __shfl_xor_sync(kFull, lo[d], o));
+        up[d] = fmaxf(up[d], __shfl_xor_sync(kFull, up[d], o));
       }
     for (int d = 0; d < 3; ++d) {
       const bool empty = lo[d] > up[d];
-      hc[d] = empty ? 0.0 : 0.5 * (lo[d] + up[d]);
-      hh[d] = empty ? -1.0 : 0.5 * (up[d] - lo[d]);  // negative: the half holds no particle
+      hc[d] = empty ? 0.f : 0.5f * (lo[d] + up[d]);
+      hh[d] = empty ? -1.f : 0.5f * (up[d] - lo[d]);  // negative: the half holds no particle
     }
   }
-  const double hcA[3] = {__shfl_sync(kFull, hc[0], 0), __shfl_sync(kFull, hc[1], 0), __shfl_sync(kFull, hc[2], 0)};
-  const double hhA[3] = {__shfl_sync(kFull, hh[0], 0), __shfl_sync(kFull, hh[1], 0), __shfl_sync(kFull, hh[2], 0)};
-  const double hcB[3] = {__shfl_sync(kFull, hc[0], 16), __shfl_sync(kFull, hc[1], 16), __shfl_sync(kFull, hc[2], 16)};
-  const double hhB[3] = {__shfl_sync(kFull, hh[0], 16), __shfl_sync(kFull, hh[1], 16), __shfl_sync(kFull, hh[2], 16)};
+  const float hcA[3] = {__shfl_sync(kFull, hc[0], 0), __shfl_sync(kFull, hc[1], 0), __shfl_sync(kFull, hc[2], 0)};
+  const float hhA[3] = {__shfl_sync(kFull, hh[0], 0), __shfl_sync(kFull, hh[1], 0), __shfl_sync(kFull, hh[2], 0)};
+  const float hcB[3] = {__shfl_sync(kFull, hc[0], 16), __shfl_sync(kFull, hc[1], 16), __shfl_sync(kFull, hc[2], 16)};
+  const float hhB[3] = {__shfl_sync(kFull, hh[0], 16), __shfl_sync(kFull, hh[1], 16), __shfl_sync(kFull, hh[2], 16)};
+  // phase B's reach: widened by the FP32 rounding of coordinates of this size
+  const float reach_f = (float)(reach + 2e-6 * (1.0 + 2.0 * reach + 4.0 * ri));
+  const Box<float> bxf = {(float)bx.ax, (float)bx.bx, (float)bx.by, (float)bx.cx, (float)bx.cy,
+                          (float)bx.cz, (float)bx.inv_ax, (float)bx.inv_by, (float)bx.inv_cz};
   const int first = a.sorted_atom[32 * I];
   const int col = first >= 0 ? a.column[first] : 0;
   const int nx = a.n_col[0], ny = a.n_col[1];
@@ -606,7 +650,8 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
   const int x0 = col % nx, y0 = col / nx;
   const int ny_iter = all_y ? ny : 2 * ky + 1, nx_iter = all_x ? nx : 2 * kx + 1;
   const int n_colq = nx_iter * ny_iter;
-  // candidate test of block J (same arithmetic as the warp-per-block kernel)
+  // candidate test of block J: the nearest image's gap is the smallest in a rectangular box;
+  // `unsafe` where another image could come within reach too
   auto test = [&](int J, double d[3], bool* unsafe) {
     const double* cj = a.block_center + 3 * J;
     const double* hj = a.block_half + 3 * J;
@@ -614,146 +659,116 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
     d[1] = cj[1] - ci[1];
     d[2] = cj[2] - ci[2];
     min_image_fast(d[0], d[1], d[2], bx);
-    const double rj = sqrt(hj[0] * hj[0] + hj[1] * hj[1] + hj[2] * hj[2]);
-    const double dist = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    *unsafe = a.min_width - dist < reach + ri + rj;
-    double gap2 = box_gap2(d, hi, hj);
-    if (*unsafe) {
-      for (int m0 = -1; m0 <= 1; ++m0)
-        for (int m1 = -1; m1 <= 1; ++m1)
-          for (int m2 = -1; m2 <= 1; ++m2) {
-            const double e[3] = {d[0] + m0 * bx.ax + m1 * bx.bx + m2 * bx.cx,
-                                 d[1] + m1 * bx.by + m2 * bx.cy, d[2] + m2 * bx.cz};
-            gap2 = fmin(gap2, box_gap2(e, hi, hj));
-          }
-    }
-    return gap2 < reach2;
+    const double room = a.min_width - (reach + ri + a.block_radius[J]);
+    *unsafe = room < 0.0 || d[0] * d[0] + d[1] * d[1] + d[2] * d[2] > room * room;
+    return box_gap2(d, hi, hj) < reach2;
   };
-  // phase A: the warps split I's columns.  In one pass each warp stages its candidates, in
-  // test order, in its own region of the candidate arrays; the regions are then packed in
-  // warp order (through registers, so no region is overwritten before it is read).  A warp
-  // with more candidates than its region holds makes the CTA test again, placing every
-  // candidate at its final offset.  Either way candidate c of warp w lands at
-  // s_wbase[w] + c, the same order whichever way it was placed.
-  const int region = min(cap / kCtaWarps, 32 * kStageRegs);
-  auto scan_columns = [&](bool staged) {
-    int n = 0;
-    for (int q = w; q < n_colq; q += kCtaWarps) {
-      const int oy = q / nx_iter, ox = q % nx_iter;
+  // phase A: the blocks of the columns in reach, one per thread, whatever column each is of (a
+  // column holds eight or so blocks of a 6 nm box, too few for a warp of its own): the columns'
+  // block counts are scanned, each thread finds its column by bisection, and the candidates are
+  // packed in (column, block) order
+  int n_cand = 0;
+  for (int q0 = 0; q0 < n_colq; q0 += kCtaThreads) {
+    const int q = q0 + threadIdx.x;
+    int j0 = 0, count = 0;
+    if (q < n_colq) {
+      const int oy = q / nx_iter, ox = q - oy * nx_iter;
       const int cy = all_y ? oy : (y0 + oy - ky + ny) % ny;
       const int cx = all_x ? ox : (x0 + ox - kx + nx) % nx;
       const int c = cy * nx + cx;
-      const int j0 = max(a.col_start[c] / 32, I + 1), j1 = min(a.col_start[c + 1] / 32, nb);
-      for (int base = j0; base < j1; base += 32) {
-        const int J = base + lane;
-        double d[3] = {0.0, 0.0, 0.0};
-        bool unsafe = false, cand = false;
-        if (J < j1) cand = test(J, d, &unsafe);
-        const unsigned m = __ballot_sync(kFull, cand);
-        if (cand) {
-          const int r = n + __popc(m & ((1u << lane) - 1u));
-          const int k = staged ? (r < region ? w * region + r : cap) : s_wbase[w] + r;
-          if (k < cap) {
-            c_J[k] = J;
-            c_un[k] = unsafe ? 1 : 0;
-            c_d[k] = d[0];
-            c_d[cap + k] = d[1];
-            c_d[2 * cap + k] = d[2];
-          }
-        }
-        n += __popc(m);
-      }
+      j0 = max(a.col_start[c] / 32, I + 1);
+      count = max(0, min(a.col_start[c + 1] / 32, nb) - j0);
     }
-    return n;
-  };
-  if (threadIdx.x == 0) s_spill = 0;
-  __syncthreads();
-  {
-    const int n = scan_columns(true);
-    if (lane == 0) {
-      s_wcount[w] = n;
-      if (n > region) s_spill = 1;
+    int incl = count;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
     }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int u = 0; u < kCtaWarps; ++u) {
-      s_wbase[u] = t;
-      t += s_wcount[u];
-    }
-    s_wbase[kCtaWarps] = t;
-  }
-  __syncthreads();
-  if (s_spill) {
-    scan_columns(false);
-  } else {
-    const int nw = s_wcount[w];
-    int rJ[kStageRegs], run[kStageRegs];
-    double rd[kStageRegs][3];
+    if (lane == 31) s_wcount[w] = incl;
+    __syncthreads();
+    int start = incl - count;
+    for (int u = 0; u < w; ++u) start += s_wcount[u];
+    s_first[threadIdx.x] = j0;
+    s_start[threadIdx.x] = start;
+    if (threadIdx.x == kCtaThreads - 1) s_start[kCtaThreads] = start + count;
+    __syncthreads();
+    const int total = s_start[kCtaThreads];
+    for (int i0 = 0; i0 < total; i0 += kCtaThreads) {
+      const int i = i0 + threadIdx.x;
+      double d[3] = {0.0, 0.0, 0.0};
+      bool unsafe = false, cand = false;
+      int J = 0;
+      if (i < total) {
+        int c = 0;  // the last column that starts at or before i
 #pragma unroll
-    for (int u = 0; u < kStageRegs; ++u) {
-      const int i = lane + 32 * u, k = w * region + i;
-      if (i < nw) {
-        rJ[u] = c_J[k];
-        run[u] = c_un[k];
-        rd[u][0] = c_d[k];
-        rd[u][1] = c_d[cap + k];
-        rd[u][2] = c_d[2 * cap + k];
+        for (int step = kCtaThreads / 2; step > 0; step >>= 1)
+          if (s_start[c + step] <= i) c += step;
+        J = s_first[c] + i - s_start[c];
+        cand = test(J, d, &unsafe);
       }
+      const unsigned m = __ballot_sync(kFull, cand);
+      if (lane == 0) s_wcount[w] = __popc(m);
+      __syncthreads();
+      int k = n_cand + __popc(m & ((1u << lane) - 1u));
+      for (int u = 0; u < kCtaWarps; ++u) {
+        const int n = s_wcount[u];
+        k += u < w ? n : 0;
+        n_cand += n;
+      }
+      if (cand && k < cap) {
+        c_J[k] = J;
+        c_un[k] = unsafe ? 1 : 0;
+        c_d[k] = d[0];
+        c_d[cap + k] = d[1];
+        c_d[2 * cap + k] = d[2];
+      }
+      __syncthreads();
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < kStageRegs; ++u) {
-      const int i = lane + 32 * u, k = s_wbase[w] + i;
-      if (i < nw && k < cap) {
-        c_J[k] = rJ[u];
-        c_un[k] = run[u];
-        c_d[k] = rd[u][0];
-        c_d[cap + k] = rd[u][1];
-        c_d[2 * cap + k] = rd[u][2];
-      }
-    }
   }
-  __syncthreads();
-  int n_cand = s_wbase[kCtaWarps];
-  if (n_cand > cap) {  // cannot happen with the host-computed capacity
+  if (n_cand > cap) {  // more than the host expected: the list grows
     if (threadIdx.x == 0) report_status(a.status, kStatusTileOverflow);
     n_cand = cap;
   }
   // phase B: one warp per candidate; a particle is kept for a half of I when it lies within
   // reach of that half's box (the conservative sphere around it near a periodic image)
   int aj_n = -1;
-  double4 wp_n = make_double4(0.0, 0.0, 0.0, 0.0);
+  float4 lp_n = make_float4(0.f, 0.f, 0.f, 0.f);
+  double rj_n = 0.0;
   if (w < n_cand) {  // this warp's first candidate, fetched ahead
     const int slot = 32 * c_J[w] + lane;
+    rj_n = a.block_radius[c_J[w]];
     aj_n = a.sorted_atom[slot];
-    wp_n = a.slot_wpos[slot];
+    lp_n = a.slot_local[slot];
   }
   for (int c = w; c < n_cand; c += kCtaWarps) {
-    const int J = c_J[c];
     const bool un = c_un[c] != 0;
     const int aj = aj_n;
-    const double4 wp = wp_n;
+    const float4 lp = lp_n;
+    const float reach_c = reach_f + 1e-6f * (float)rj_n;
     if (c + kCtaWarps < n_cand) {  // the next candidate's particles, in flight meanwhile
       const int slot = 32 * c_J[c + kCtaWarps] + lane;
+      rj_n = a.block_radius[c_J[c + kCtaWarps]];
       aj_n = a.sorted_atom[slot];
-      wp_n = a.slot_wpos[slot];
+      lp_n = a.slot_local[slot];
     }
     bool in_a = false, in_b = false;
     if (aj >= 0) {
-      const double* cj = a.block_center + 3 * J;
-      const double rel[3] = {wp.x - cj[0] + c_d[c], wp.y - cj[1] + c_d[cap + c],
-                             wp.z - cj[2] + c_d[2 * cap + c]};
-      auto near_half = [&](const double* hcen, const double* hext) {
-        if (hext[0] < 0.0) return false;
-        double rh[3] = {rel[0] - hcen[0], rel[1] - hcen[1], rel[2] - hcen[2]};
+      const float rel[3] = {lp.x + (float)c_d[c], lp.y + (float)c_d[cap + c],
+                            lp.z + (float)c_d[2 * cap + c]};
+      auto near_half = [&](const float* hcen, const float* hext) {
+        if (hext[0] < 0.f) return false;
+        float rh[3] = {rel[0] - hcen[0], rel[1] - hcen[1], rel[2] - hcen[2]};
         if (un) {
-          min_image_fast(rh[0], rh[1], rh[2], bx);
-          const double rad = sqrt(hext[0] * hext[0] + hext[1] * hext[1] + hext[2] * hext[2]);
-          return sqrt(rh[0] * rh[0] + rh[1] * rh[1] + rh[2] * rh[2]) < reach + rad + 1e-6;
+          min_image_fast(rh[0], rh[1], rh[2], bxf);
+          const float rad =
+              reach_c + sqrtf(hext[0] * hext[0] + hext[1] * hext[1] + hext[2] * hext[2]);
+          return rh[0] * rh[0] + rh[1] * rh[1] + rh[2] * rh[2] < rad * rad;
         }
-        return box_gap2(rh, hext, nullptr) < reach2;
+        const float gx = fmaxf(fabsf(rh[0]) - hext[0], 0.f);
+        const float gy = fmaxf(fabsf(rh[1]) - hext[1], 0.f);
+        const float gz = fmaxf(fabsf(rh[2]) - hext[2], 0.f);
+        return gx * gx + gy * gy + gz * gz < reach_c * reach_c;
       };
       in_a = near_half(hcA, hhA);
       in_b = near_half(hcB, hhB);
@@ -843,15 +858,14 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
     int mslot = -1;
     int flags = flag;
     if (__any_sync(kFull, m != 0)) {
-      if (lane == 0) mslot = atomicAdd(a.n_masks, 1);
-      mslot = __shfl_sync(kFull, mslot, 0);
-      if (mslot < a.mask_capacity) {
-        a.masks[32 * mslot + lane] = m;
+      if (t < a.mask_capacity) {  // the host keeps it at least tile_capacity for this builder
+        mslot = t;
+        a.masks[32 * (size_t)mslot + lane] = m;
         flags |= kTileHasMask;
-      } else {
-        if (lane == 0) report_status(a.status, kStatusTileOverflow);
-        mslot = -1;
+      } else if (lane == 0) {
+        report_status(a.status, kStatusTileOverflow);
       }
+      if (lane == 0) atomicAdd(a.n_masks, 1);  // a statistic
     }
     if (lane == 0) a.tiles[t] = make_int4(I, flags, mslot, 0);
     if (k > 0) write_entry<kDouble>(a, t, lane, slot, sh);
@@ -859,13 +873,12 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
   }
 }
 
-__global__ void nl_finish(NlistArgs a) {
+template <bool kDouble>
+__global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
   if (*a.rebuild == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (int k = i; k < a.n_cols; k += gridDim.x * blockDim.x) {
-    a.col_count[k] = 0;
-    a.col_cursor[k] = 0;
-  }
+  if ((int)blockIdx.x < *a.n_blocks) build_block_list<kDouble>(a, blockIdx.x);
+  // every CTA counts itself after its last read of the flag
+  if (last_cta(a.done + 1) && threadIdx.x == 0) close_rebuild(a);
 }
 
 // Inside a captured step: the rebuild kernels sit in the body of a conditional graph node
@@ -874,11 +887,9 @@ __global__ void nl_set_condition(const int* rebuild, cudaGraphConditionalHandle 
   cudaGraphSetConditional(handle, *rebuild != 0 ? 1u : 0u);
 }
 
+// Triclinic boxes: closes the rebuild (the CTA builder of rectangular boxes does it itself).
 __global__ void nl_clear_flag(NlistArgs a) {
-  if (*a.rebuild == 0) return;
-  *a.rebuild = 0;
-  *a.rebuild_count += 1;
-  if (a.prune) *a.prune = 1;  // the pruned list derives from the tiles just built
+  if (*a.rebuild != 0) close_rebuild(a);
 }
 
 // ---- pruned list ---------------------------------------------------------------------------
@@ -1165,17 +1176,17 @@ void launch_nlist_prune(const NlistArgs& a, const PruneArgs& p, bool double_entr
 }
 
 void launch_nlist_rebuild(const NlistArgs& a, bool double_entries, cudaStream_t s,
-                          const std::function<void(cudaStream_t)>& with_list) {
-  const int tb = 256;
-  const int ga = ceil_div(a.n_atoms, tb);
+                          const std::function<void(cudaStream_t)>& with_columns) {
   const int block_cap = a.slot_capacity / 32;
-  nl_columns<<<ga, tb, 0, s>>>(a);
-  nl_col_scan<<<1, 1024, 0, s>>>(a);
-  nl_col_scatter<<<ga, tb, 0, s>>>(a);
+  nl_columns<<<ceil_div(a.n_atoms, 256), 256, 0, s>>>(a);
   int m = 1;
   while (m < a.col_max) m <<= 1;
-  nl_col_sort<<<a.n_cols, 256, sizeof(unsigned long long) * m, s>>>(a);
-  nl_bounds<<<ceil_div((long long)block_cap * 32, tb), tb, 0, s>>>(a);
+  const size_t keys = sizeof(unsigned long long) * m;
+  if (double_entries)
+    nl_col_sort<true><<<a.n_cols, 256, keys, s>>>(a);
+  else
+    nl_col_sort<false><<<a.n_cols, 256, keys, s>>>(a);
+  if (with_columns) with_columns(s);
   const bool rectangular = a.periodic && a.box.bx == 0.0 && a.box.cx == 0.0 && a.box.cy == 0.0;
   if (rectangular && a.max_cand > 0 && a.halves) {
     const size_t bytes = (size_t)a.max_cand * (3 * 8 + 4 + 4 + 2 * 4 + 2 * 4) + 8;
@@ -1192,10 +1203,8 @@ void launch_nlist_rebuild(const NlistArgs& a, bool double_entries, cudaStream_t 
       nl_lists<true><<<gl, 32 * kListWarps, 0, s>>>(a);
     else
       nl_lists<false><<<gl, 32 * kListWarps, 0, s>>>(a);
+    nl_clear_flag<<<1, 1, 0, s>>>(a);
   }
-  if (with_list) with_list(s);
-  nl_finish<<<std::max(1, std::min(ceil_div(a.n_cols, tb), 148 * 4)), tb, 0, s>>>(a);
-  nl_clear_flag<<<1, 1, 0, s>>>(a);
 }
 
 }  // namespace ommb200

@@ -832,15 +832,15 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
   }
 }
 
-// `only_after_rebuild` (may be null): pack only when that rebuild flag is set (the integrator
-// writes the packed coordinates of the other steps).
+// The packed particles of every slot (a rebuild packs its own, and between rebuilds the integrator
+// writes those it moves: this runs for non-periodic systems and after new parameters or a
+// checkpoint).
 template <class Real>
 __global__ void pack_kernel(int n_slots, const int* sorted_atom, const double* pos,
                             const int* image, const double* block_center, const double* qscaled,
                             const double* half_sigma, const double* two_sqrt_eps,
                             typename V4<Real>::T4* posq, typename V4<Real>::T2* ljp,
-                            Box<double> b, const int* only_after_rebuild) {
-  if (only_after_rebuild && *only_after_rebuild == 0) return;
+                            Box<double> b) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n_slots) return;
   const int a = sorted_atom[s];
@@ -913,20 +913,20 @@ template <class Real>
 void launch_pack(int n_slots, const int* sorted_atom, const double* pos, const int* image,
                  const double* block_center, const double* qscaled, const double* half_sigma,
                  const double* two_sqrt_eps, void* posq, void* ljp, const Box<double>& box,
-                 cudaStream_t s, const int* only_after_rebuild) {
+                 cudaStream_t s) {
   pack_kernel<Real><<<ceil_div(n_slots, 256), 256, 0, s>>>(
       n_slots, sorted_atom, pos, image, block_center, qscaled, half_sigma, two_sqrt_eps,
       reinterpret_cast<typename V4<Real>::T4*>(posq), reinterpret_cast<typename V4<Real>::T2*>(ljp),
-      box, only_after_rebuild);
+      box);
 }
 
 template void launch_pair<float>(const PairArgs<float>&, int, bool, bool, int, cudaStream_t);
 template void launch_pair<double>(const PairArgs<double>&, int, bool, bool, int, cudaStream_t);
 template void launch_pack<float>(int, const int*, const double*, const int*, const double*,
                                  const double*, const double*, const double*, void*, void*,
-                                 const Box<double>&, cudaStream_t, const int*);
+                                 const Box<double>&, cudaStream_t);
 template void launch_pack<double>(int, const int*, const double*, const int*, const double*,
                                   const double*, const double*, const double*, void*, void*,
-                                  const Box<double>&, cudaStream_t, const int*);
+                                  const Box<double>&, cudaStream_t);
 
 }  // namespace ommb200

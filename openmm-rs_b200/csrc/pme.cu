@@ -918,7 +918,7 @@ __global__ void brick_ranges_kernel(const NlistArgs a, const PmeBricks b) {
   if (i >= a.n_cols * b.nb[2]) return;
   const int c = i % a.n_cols, bz = i / a.n_cols;
   const int s0 = a.col_start[c];
-  const int n = min(a.col_scatter[c + 1] - a.col_scatter[c], a.col_max);
+  const int n = min(a.col_size[c], a.col_max);
   const double L = b.len[2];
   const double z0 = bz * kBrickEdge * b.cell[2] - b.below[2];
   const double z1 = min((bz + 1) * kBrickEdge, b.grid[2]) * b.cell[2] + b.above;

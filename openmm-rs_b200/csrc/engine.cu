@@ -468,6 +468,7 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
   a.posq = posq_;
   a.ljp = ljp_;
   if (!nb_periodic_) build_static_tiles();
+  if (nb.method == kCutoffNonPeriodic) static_box_ = mem_.alloc<float4>(2 * (size_t)n_blocks_);
   int dev_sms = 148;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, opt_.device);
   sm_count_ = dev_sms;
@@ -717,7 +718,7 @@ void Engine::build_static_tiles() {
         masks.insert(masks.end(), m, m + 32);
         flags |= kTileHasMask;
       }
-      tiles.push_back(make_int4(I, flags, slot, 0));
+      tiles.push_back(make_int4(I, flags, slot, J));
       // entries: the 32 slots of block J in its own (shared, unshifted) frame
       for (int k = 0; k < 32; ++k) {
         const int s = static_slot_atom_[32 * J + k] >= 0 ? 32 * J + k : -1;
@@ -1597,7 +1598,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     if (!packed_by_integrator()) {
       prof_begin("pack");
       launch_pack<Real>(n_slots_, nl_.sorted_atom, pos_, nl_.image, nl_.block_center, qscaled_,
-                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, direct_stream);
+                        half_sigma_, sqrt_eps_, posq_, ljp_, nl_.box, direct_stream, static_box_);
       prof_end();
     }
     const bool pruned = pruning();
@@ -1638,6 +1639,8 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     const double rc = nb.cutoff;
     p.cutoff2 = (Real)(rc * rc);
     p.cutoff2_exact = rc * rc;
+    p.block_box = static_box_;
+    p.skip2 = (float)(rc * rc * (1.0 + 1e-4));
     p.band = (Real)(rc * rc * (dp_ ? 1e-10 : 1e-4));
     p.alpha = (Real)alpha_;
     // the FP32 kernel evaluates exp(-alpha^2 r^2) as exp2(-alpha^2 log2(e) r^2)

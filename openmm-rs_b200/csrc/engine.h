@@ -294,6 +294,7 @@ class Engine {
   double* charge_ = nullptr;
   double* half_sigma_ = nullptr;
   double* sqrt_eps_ = nullptr;  // 2 sqrt(epsilon)
+  float4* static_box_ = nullptr;  // blocks' bounding boxes (CutoffNonPeriodic)
   int static_tile_count_ = 0;    // tiles of the non-periodic (segment-padded) pair list
   bool nb_gb_fusable_ = false;   // NoCutoff pair terms can run inside GB pass 2
   void* posq_ = nullptr;

@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Re
     const int4 tile = a.tiles[t];
     const int I = tile.x;
     const bool self = (tile.y & kTileSelf) != 0;
+    if (a.block_box && !self && boxes_apart(a.block_box, I, tile.w, a.skip2)) continue;
     const bool pair_image = (tile.y & kTilePairImage) != 0;
     const bool halves = (tile.y & kTileHalves) != 0;
     const int si = 32 * I + lane;
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
     const float4 e = entries[32 * t + lane];  // unused (unwritten) for self tiles
     const int I = tile.x;
     const bool self = (tile.y & kTileSelf) != 0;
+    if (a.block_box && !self && boxes_apart(a.block_box, I, tile.w, a.skip2)) continue;
     const bool pair_image = (tile.y & kTilePairImage) != 0;
     const bool halves = (tile.y & kTileHalves) != 0;
     const int si = 32 * I + lane;
@@ -840,7 +842,7 @@ __global__ void pack_kernel(int n_slots, const int* sorted_atom, const double* p
                             const int* image, const double* block_center, const double* qscaled,
                             const double* half_sigma, const double* two_sqrt_eps,
                             typename V4<Real>::T4* posq, typename V4<Real>::T2* ljp,
-                            Box<double> b) {
+                            Box<double> b, float4* block_box) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n_slots) return;
   const int a = sorted_atom[s];
@@ -863,6 +865,20 @@ __global__ void pack_kernel(int n_slots, const int* sorted_atom, const double* p
   }
   posq[s] = out;
   ljp[s] = lj;
+  if (block_box) {  // whole warps: n_slots is a multiple of 32
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    if (a >= 0) {
+      lo[0] = hi[0] = (float)out.x;
+      lo[1] = hi[1] = (float)out.y;
+      lo[2] = hi[2] = (float)out.z;
+    }
+    for (int o = 16; o > 0; o >>= 1)
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+      }
+    if ((s & 31) == 0) store_box(block_box, s >> 5, lo, hi);
+  }
 }
 
 }  // namespace
@@ -913,20 +929,20 @@ template <class Real>
 void launch_pack(int n_slots, const int* sorted_atom, const double* pos, const int* image,
                  const double* block_center, const double* qscaled, const double* half_sigma,
                  const double* two_sqrt_eps, void* posq, void* ljp, const Box<double>& box,
-                 cudaStream_t s) {
+                 cudaStream_t s, float4* block_box) {
   pack_kernel<Real><<<ceil_div(n_slots, 256), 256, 0, s>>>(
       n_slots, sorted_atom, pos, image, block_center, qscaled, half_sigma, two_sqrt_eps,
       reinterpret_cast<typename V4<Real>::T4*>(posq), reinterpret_cast<typename V4<Real>::T2*>(ljp),
-      box);
+      box, block_box);
 }
 
 template void launch_pair<float>(const PairArgs<float>&, int, bool, bool, int, cudaStream_t);
 template void launch_pair<double>(const PairArgs<double>&, int, bool, bool, int, cudaStream_t);
 template void launch_pack<float>(int, const int*, const double*, const int*, const double*,
                                  const double*, const double*, const double*, void*, void*,
-                                 const Box<double>&, cudaStream_t);
+                                 const Box<double>&, cudaStream_t, float4*);
 template void launch_pack<double>(int, const int*, const double*, const int*, const double*,
                                   const double*, const double*, const double*, void*, void*,
-                                  const Box<double>&, cudaStream_t);
+                                  const Box<double>&, cudaStream_t, float4*);
 
 }  // namespace ommb200

@@ -500,8 +500,10 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
       for (int r = 11; r * r <= prime; ++r) one = one && prime % r != 0;
       // where the direct sums beat cuFFT (three cubes of each size measured): cuFFT's own radices
       // end at 11, and its way round larger primes is slow except for some even sizes past 65
-      // (39^3: 58 us against 23; 65^3: 65, 38; 95^3: 94, 65; but 68^3: 31, 44 and 104^3: 42, 86)
-      if (one && prime >= kMinFftPrime && prime <= kMaxFftPrime && (m <= 65 || (m <= 96 && m % 2))) {
+      // (39^3: 58 us against 23; 65^3: 65, 38; 95^3: 94, 65; but 68^3: 31, 44 and 104^3: 42, 86).
+      // The one-launch form takes 11 too
+      const int least = n_ <= kClusterAtoms && opt_.pme_bricks < 0 ? 11 : kMinFftPrime;
+      if (one && prime >= least && prime <= kMaxFftPrime && (m <= 65 || (m <= 96 && m % 2))) {
         fft_.rad[d][k++] = prime;
         m /= prime;
       }
@@ -594,6 +596,20 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
   upload_nonbonded_parameters(nb);
 }
 
+// The cluster form of the reciprocal part, while its shared-memory sums cannot overflow; a
+// change of choice drops the captured graphs.
+void Engine::choose_cluster(const NonbondedDef& nb) {
+  int ctas = 0;
+  double total = 0.0;
+  for (double q : nb.charge) total += std::fabs(q);
+  // the pme_bricks option asks for one of the two gathers of the launch chain
+  if (nb_pme_ && own_fft_ && opt_.pme_bricks < 0 && total < kClusterCharge)
+    ctas = dp_ ? pme_cluster_ctas(pme_args<double>()) : pme_cluster_ctas(pme_args<float>());
+  if (ctas == cluster_ctas_) return;
+  cluster_ctas_ = ctas;
+  destroy_graph();
+}
+
 // Per-particle parameters, exception parameters and the parameter-dependent constants (self
 // energy, dispersion coefficient); the pair set and the tile masks do not depend on them.
 void Engine::upload_nonbonded_parameters(const NonbondedDef& nb) {
@@ -615,6 +631,7 @@ void Engine::upload_nonbonded_parameters(const NonbondedDef& nb) {
                            nb.charge[e.p1] * nb.charge[e.p2] * kOne4PiEps0);
   }
   OMMB200_CK(cudaMemcpy(exc_params_, epar.data(), sizeof(double4) * epar.size(), cudaMemcpyHostToDevice));
+  choose_cluster(nb);
   dispersion_coeff_ =
       (nb_periodic_ && nb.use_dispersion_correction) ? dispersion_coefficient(nb) : 0.0;
   double q2 = 0.0;
@@ -1495,9 +1512,49 @@ PruneArgs Engine::prune_args() const {
 }
 
 template <class Real>
+PmeArgs<Real> Engine::pme_args() const {
+  PmeArgs<Real> m{};
+  m.n_atoms = n_;
+  m.order = nl_.sorted_atom;
+  m.n_order = n_slots_;
+  m.pos = pos_;
+  m.charge = charge_;
+  m.nx = grid_[0];
+  m.ny = grid_[1];
+  m.nz = grid_[2];
+  for (int r = 0; r < 3; ++r)
+    for (int c = 0; c < 3; ++c) m.recip[r][c] = recip_[r][c];
+  m.grid_fixed = pme_fixed_;
+  m.grid_real = static_cast<Real*>(pme_real_);
+  m.grid_k = pme_k_;
+  m.influence = static_cast<const Real*>(influence_);
+  m.moduli = moduli_;
+  m.force = force_;
+  m.energy = energy_;
+  m.alpha = alpha_;
+  m.volume = volume_;
+  return m;
+}
+
+template <class Real>
 void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
                                int step_offset, cudaStream_t direct_stream) {
   const NonbondedDef& nb = *nb_;
+  // the reciprocal part of a small box needs nothing of the neighbour list: it starts before a
+  // rebuild and runs beside it
+  const bool cluster = reciprocal && nb_pme_ && cluster_ctas_ > 0;
+  auto fork_pme = [&] {
+    OMMB200_CK(cudaEventRecord(fork_ev_, stream_));
+    OMMB200_CK(cudaStreamWaitEvent(pme_stream_, fork_ev_, 0));
+  };
+  if (cluster) {
+    if (!profiling_) fork_pme();
+    cudaStream_t cs = profiling_ ? stream_ : pme_stream_;
+    const PmeArgs<Real> m = pme_args<Real>();
+    prof_begin("pme_cluster");
+    launch_pme_cluster<Real>(m, fft_, cluster_ctas_, energy, cs);
+    prof_end();
+  }
   if (nb_periodic_) {
     prof_begin("nlist_rebuild");
     if (capturing_)
@@ -1510,33 +1567,11 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
   // per-kernel events time one kernel at a time)
   const bool pme = reciprocal && nb_pme_;
   cudaStream_t ps = (pme && !profiling_) ? pme_stream_ : stream_;
-  if (ps != stream_) {
-    OMMB200_CK(cudaEventRecord(fork_ev_, stream_));
-    OMMB200_CK(cudaStreamWaitEvent(ps, fork_ev_, 0));
-  }
+  if (ps != stream_ && !cluster) fork_pme();
   // the reciprocal chain is enqueued first, so its kernels reach the GPU ahead of the direct
   // chain's (the two orders measured within run-to-run spread of each other)
-  if (reciprocal && nb_pme_) {
-    PmeArgs<Real> m{};
-    m.n_atoms = n_;
-    m.order = nl_.sorted_atom;
-    m.n_order = n_slots_;
-    m.pos = pos_;
-    m.charge = charge_;
-    m.nx = grid_[0];
-    m.ny = grid_[1];
-    m.nz = grid_[2];
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c) m.recip[r][c] = recip_[r][c];
-    m.grid_fixed = pme_fixed_;
-    m.grid_real = static_cast<Real*>(pme_real_);
-    m.grid_k = pme_k_;
-    m.influence = static_cast<const Real*>(influence_);
-    m.moduli = moduli_;
-    m.force = force_;
-    m.energy = energy_;
-    m.alpha = alpha_;
-    m.volume = volume_;
+  if (pme && !cluster) {
+    const PmeArgs<Real> m = pme_args<Real>();
     prof_begin("pme_spread");
     launch_pme_spread<Real>(m, ps);
     prof_end();

@@ -231,6 +231,9 @@ class Engine {
   void enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
                          int step_offset, cudaStream_t direct_stream);
   bool gb_packed_by_integrator() const;
+  template <class Real>
+  PmeArgs<Real> pme_args() const;
+  void choose_cluster(const NonbondedDef& nb);
   void prof_begin(const char* name);
   void prof_end();
   void harvest_profile();
@@ -314,6 +317,7 @@ class Engine {
   bool fft_ready_ = false;
   bool own_fft_ = false;  // the engine's pencil transform instead of cuFFT
   PmeFft fft_{};
+  int cluster_ctas_ = 0;  // CTAs of the one-launch reciprocal part (0: the launch chain)
   int n_exceptions_ = 0;
   int2* exc_pairs_ = nullptr;
   double4* exc_params_ = nullptr;

@@ -249,6 +249,16 @@ template <class Real>
 void prepare_pme_transform(const PmeArgs<Real>& a, const PmeFft& f);
 template <class Real>
 void launch_pme_transform(const PmeArgs<Real>& a, const PmeFft& f, bool energy, cudaStream_t s);
+// The whole reciprocal part in one launch of one thread-block cluster, for boxes of at most
+// kClusterAtoms particles whose grid fits the cluster's shared memory: the cluster size, 0 where
+// it does not apply.  Its shared-memory sums hold sum |q| up to kClusterCharge.
+constexpr int kClusterAtoms = 4095;
+constexpr double kClusterCharge = 8192.0;  // e: a grid point gets at most 0.22 of each charge
+template <class Real>
+int pme_cluster_ctas(const PmeArgs<Real>& a);
+template <class Real>
+void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, bool energy,
+                        cudaStream_t s);
 template <class Real>
 void launch_pme_convert(const PmeArgs<Real>& a, cudaStream_t s);
 template <class Real>

@@ -12,10 +12,14 @@
 //
 // Charges are spread into a 64-bit fixed-point grid (units of 2^-40 e) so the grid, and every
 // force derived from it, is independent of the order of the atomic additions.
+#include <cooperative_groups.h>
+
 #include "kernels.h"
 
 namespace ommb200 {
 namespace {
+
+namespace cg = cooperative_groups;
 
 // pme.rs:151-174
 template <class Real>
@@ -597,6 +601,7 @@ __host__ __device__ inline int fft_plane_elems(int ny, int nz) {
 }
 
 constexpr int kPlaneThreads = 512, kXPassThreads = 256;  // block size caps of the transform
+constexpr int kClusterThreads = 512;
 constexpr int kLoadBatch = 4;  // global loads each thread keeps in flight in the copy loops
 
 // for i in [0, total), strided over the block: v = load(i) for kLoadBatch items at a time,
@@ -766,6 +771,237 @@ __global__ void __launch_bounds__(kPlaneThreads) planes_inverse(const PmeArgs<Re
   }
 }
 
+// ---- the whole reciprocal part of a small box in one launch -----------------------------
+// Below a few thousand particles the five launches of the reciprocal chain (spread, three
+// transform passes, gather) are bound by their launches and by one round trip to L2 each; the
+// grid itself (23^3 to about 40^3) fits in the shared memory of one thread-block cluster.  CTA c
+// of the cluster owns the x planes [c P, (c + 1) P) of the grid from the charges to the
+// potential: it spreads every particle's stencil rows that fall in its planes into shared
+// memory (exact fixed point at 2^-40 e, split hi 2^20 + lo for native 32-bit atomics: at most
+// kClusterAtoms contributions keep lo inside 32 bits, and the host checks sum |q| for hi),
+// transforms its planes along z and y, transforms its share of the (y, kz) pencils along x with
+// the influence function, reading and writing the owners' planes through distributed shared
+// memory, transforms its planes back and gathers their part of every particle's force.  Two
+// cluster barriers (around the x pass) replace four kernel boundaries.  Each particle's force
+// is the fixed-point sum of its planes' parts.  1,524 particles on a 23^3 grid: the chain's step
+// took 55 us, with this form 46 us.
+template <class Real>
+struct ClusterLayout {  // element counts; every CTA of the cluster has the same
+  int planes, pencils;  // planes and x pencils per CTA
+  size_t plane_elems;   // of each of the two plane buffers
+  __host__ __device__ ClusterLayout(int nx, int ny, int nz, int ctas)
+      : planes((nx + ctas - 1) / ctas), pencils((ny * (nz / 2 + 1) + ctas - 1) / ctas),
+        plane_elems((size_t)planes * fft_plane_elems(ny, nz)) {}
+  __host__ __device__ size_t bytes(int nx, int ny, int nz) const {
+    return 2 * sizeof(Real) * ((size_t)nx + ny + nz + 2 * plane_elems + 2 * (size_t)pencils * nx) +
+           2 * sizeof(int) * (size_t)planes * ny * nz;
+  }
+};
+
+template <class Real, bool kEnergy>
+__global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Real> a, const PmeFft f) {
+  using C2 = typename Cplx<Real>::T;
+  extern __shared__ __align__(16) unsigned char fsm[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ctas = gridDim.x, rank = blockIdx.x;  // one cluster
+  const int nx = a.nx, ny = a.ny, nz = a.nz, nzh = nz / 2 + 1, nyp = (ny + 1) / 2;
+  const ClusterLayout<Real> L(nx, ny, nz, ctas);
+  C2* twx = reinterpret_cast<C2*>(fsm);
+  C2* twy = twx + nx;
+  C2* twz = twy + ny;
+  C2* A = twz + nz;
+  C2* B = A + L.plane_elems;
+  C2* XA = B + L.plane_elems;
+  C2* XB = XA + (size_t)L.pencils * nx;
+  int* c_hi = reinterpret_cast<int*>(XB + (size_t)L.pencils * nx);
+  unsigned* c_lo = reinterpret_cast<unsigned*>(c_hi + (size_t)L.planes * ny * nz);
+  const int x0 = rank * L.planes, np = max(0, min(L.planes, nx - x0));  // own planes
+  load_twiddles(twx, f.tw[0], nx);
+  load_twiddles(twy, f.tw[1], ny);
+  load_twiddles(twz, f.tw[2], nz);
+  for (int c = threadIdx.x; c < np * ny * nz; c += blockDim.x) {
+    c_hi[c] = 0;
+    c_lo[c] = 0u;
+  }
+  __syncthreads();
+  // spread (pme.rs:176-238)
+  const Real gscale = Real(kGridScale);
+  for (int i = threadIdx.x; i < a.n_atoms; i += blockDim.x) {
+    const double qd = a.charge[i];
+    int base[3];
+    Real frac[3], w[3][5], dw[3][5];
+    if (qd == 0.0 || !stencil(a, i, base, frac)) continue;
+    bool mine = false;
+#pragma unroll
+    for (int ix = 0; ix < 5; ++ix) {
+      int gx = base[0] + ix;
+      gx -= gx >= nx ? nx : 0;
+      mine = mine || (gx >= x0 && gx < x0 + np);
+    }
+    if (!mine) continue;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) spline5(frac[d], w[d], dw[d]);
+    const Real q = (Real)qd;
+#pragma unroll
+    for (int ix = 0; ix < 5; ++ix) {
+      int gx = base[0] + ix;
+      gx -= gx >= nx ? nx : 0;
+      if (gx < x0 || gx >= x0 + np) continue;
+      const Real qx = q * w[0][ix];
+      for (int iy = 0; iy < 5; ++iy) {
+        int gy = base[1] + iy;
+        gy -= gy >= ny ? ny : 0;
+        const Real qxy = qx * w[1][iy];
+        const int row = ((gx - x0) * ny + gy) * nz;
+#pragma unroll
+        for (int iz = 0; iz < 5; ++iz) {
+          int gz = base[2] + iz;
+          gz -= gz >= nz ? nz : 0;
+          const long long v = to_fixed(qxy * w[2][iz], gscale);
+          atomicAdd(&c_hi[row + gz], (int)(v >> 20));
+          atomicAdd(&c_lo[row + gz], (unsigned)(v & 0xFFFFF));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // rows y = 2 yp (real part) and 2 yp + 1 (imaginary part) as one complex row, z transform
+  for (int i = threadIdx.x; i < np * nyp * nz; i += blockDim.x) {
+    const int z = i % nz, r = i / nz, lp = r / nyp, yp = r - lp * nyp;
+    const int c0 = (lp * ny + 2 * yp) * nz + z;
+    C2 v;
+    v.x = (Real)((double)((long long)c_hi[c0] * (1ll << 20) + (long long)c_lo[c0]) * kGridScaleInv);
+    v.y = 0;
+    if (2 * yp + 1 < ny) {
+      const int c1 = c0 + nz;
+      v.y = (Real)((double)((long long)c_hi[c1] * (1ll << 20) + (long long)c_lo[c1]) * kGridScaleInv);
+    }
+    A[i] = v;
+  }
+  __syncthreads();
+  C2* r = stockham(A, B, twz, f, 2, nz, np * nyp);
+  C2* o = r == A ? B : A;
+  // split the two real rows' spectra into pencils along y: o[plane][kz][y] (planes_forward)
+  for (int i = threadIdx.x; i < np * nzh * ny; i += blockDim.x) {
+    const int y = i % ny, t = i / ny, lp = t / nzh, kz = t - lp * nzh, yp = y >> 1;
+    const C2* row = r + (lp * nyp + yp) * nz;
+    const C2 zk = row[kz], zm = row[kz == 0 ? 0 : nz - kz];
+    C2 v;
+    if ((y & 1) == 0) {
+      v.x = (Real)0.5 * (zk.x + zm.x);
+      v.y = (Real)0.5 * (zk.y - zm.y);
+    } else {
+      v.x = (Real)0.5 * (zk.y + zm.y);
+      v.y = (Real)0.5 * (zm.x - zk.x);
+    }
+    o[i] = v;
+  }
+  __syncthreads();
+  // the same buffer in every CTA: the swaps depend on the axes' stage counts alone
+  C2* s = stockham(o, r, twy, f, 1, ny, np * nzh);
+  cluster.sync();
+  // x pass over this CTA's pencils q = kz ny + y
+  const int q0 = rank * L.pencils, nq = max(0, min(L.pencils, nzh * ny - q0));
+  for (int i = threadIdx.x; i < nq * nx; i += blockDim.x) {
+    const int x = i / nq, q = i - x * nq, owner = x / L.planes, lp = x - owner * L.planes;
+    XA[q * nx + x] = cluster.map_shared_rank(s, owner)[lp * nzh * ny + q0 + q];
+  }
+  __syncthreads();
+  C2* xr = stockham(XA, XB, twx, f, 0, nx, nq);
+  C2* xo = xr == XA ? XB : XA;
+  double e = 0.0, vir[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = threadIdx.x; i < nq * nx; i += blockDim.x) {
+    const int q = i / nx, x = i - q * nx, kz = (q0 + q) / ny, y = q0 + q - kz * ny;
+    const long long at = ((long long)x * ny + y) * nzh + kz;
+    const Real infl = __ldg(a.influence + at);
+    C2 v = xr[i];
+    if (kEnergy && at != 0)
+      mode_energy(a, x, y, kz, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, vir);
+    v.x *= infl;
+    v.y *= -infl;  // conjugated for the inverse transform
+    xr[i] = v;
+  }
+  if (kEnergy) commit_energy(a, e, vir);
+  __syncthreads();
+  C2* xs = stockham(xr, xo, twx, f, 0, nx, nq);
+  // back to the owners, still conjugated: the inverse y transform starts from conj H.  Each
+  // element was read, and is written, by this CTA alone
+  for (int i = threadIdx.x; i < nq * nx; i += blockDim.x) {
+    const int x = i / nq, q = i - x * nq, owner = x / L.planes, lp = x - owner * L.planes;
+    cluster.map_shared_rank(s, owner)[lp * nzh * ny + q0 + q] = xs[q * nx + x];
+  }
+  cluster.sync();
+  C2* h = stockham(s, s == A ? B : A, twy, f, 1, ny, np * nzh);
+  C2* g = h == A ? B : A;
+  // rows 2 yp and 2 yp + 1, Hermitian-completed along z, as one conjugated row (planes_inverse)
+  for (int i = threadIdx.x; i < np * nyp * nz; i += blockDim.x) {
+    const int k = i % nz, t = i / nz, lp = t / nyp, y0 = 2 * (t - lp * nyp);
+    const bool low = k < nzh;
+    const C2* col = h + ((size_t)lp * nzh + (low ? k : nz - k)) * ny + y0;
+    C2 ca = col[0];
+    if (!low) ca = conjg(ca);
+    C2 cb;
+    cb.x = cb.y = 0;
+    if (y0 + 1 < ny) {
+      cb = col[1];
+      if (!low) cb = conjg(cb);
+    }
+    C2 v;
+    v.x = ca.x + cb.y;
+    v.y = ca.y - cb.x;
+    g[i] = v;
+  }
+  __syncthreads();
+  const C2* pot = stockham(g, h, twz, f, 2, nz, np * nyp);  // row 2 yp = Re, row 2 yp + 1 = -Im
+  // gather (pme.rs:377-425): this CTA's planes' part of every particle's force
+  for (int i = threadIdx.x; i < a.n_atoms; i += blockDim.x) {
+    const double qd = a.charge[i];
+    int base[3];
+    Real frac[3], w[3][5], dw[3][5];
+    if (qd == 0.0 || !stencil(a, i, base, frac)) continue;
+    bool mine = false;
+#pragma unroll
+    for (int ix = 0; ix < 5; ++ix) {
+      int gx = base[0] + ix;
+      gx -= gx >= nx ? nx : 0;
+      mine = mine || (gx >= x0 && gx < x0 + np);
+    }
+    if (!mine) continue;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) spline5(frac[d], w[d], dw[d]);
+    Real g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll
+    for (int ix = 0; ix < 5; ++ix) {
+      int gx = base[0] + ix;
+      gx -= gx >= nx ? nx : 0;
+      if (gx < x0 || gx >= x0 + np) continue;
+      for (int iy = 0; iy < 5; ++iy) {
+        int gy = base[1] + iy;
+        gy -= gy >= ny ? ny : 0;
+        const C2* row = pot + ((gx - x0) * nyp + (gy >> 1)) * nz;
+        Real sum = 0, dsum = 0;
+#pragma unroll
+        for (int iz = 0; iz < 5; ++iz) {
+          int gz = base[2] + iz;
+          gz -= gz >= nz ? nz : 0;
+          const C2 v = row[gz];
+          const Real phi = (gy & 1) ? -v.y : v.x;
+          sum += phi * w[2][iz];
+          dsum += phi * dw[2][iz];
+        }
+        g0 += dw[0][ix] * w[1][iy] * sum;
+        g1 += w[0][ix] * dw[1][iy] * sum;
+        g2 += w[0][ix] * w[1][iy] * dsum;
+      }
+    }
+    const double gd[3] = {(double)g0 * nx, (double)g1 * ny, (double)g2 * nz};
+    for (int c = 0; c < 3; ++c) {
+      const double fc = -qd * (gd[0] * a.recip[0][c] + gd[1] * a.recip[1][c] + gd[2] * a.recip[2][c]);
+      add_fixed(a.force + (long long)c * a.n_atoms + i, to_fixed(fc, kForceScale));
+    }
+  }
+}
+
 }  // namespace
 
 template <class Real>
@@ -796,6 +1032,66 @@ void prepare_pme_transform(const PmeArgs<Real>& a, const PmeFft& f) {
   cudaFuncSetAttribute((const void*)x_convolve<Real, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
 }
 
+// The cluster form's launch: `ctas` CTAs of one cluster.
+template <class Real, bool kEnergy>
+cudaLaunchConfig_t cluster_config(const PmeArgs<Real>& a, int ctas, cudaLaunchAttribute* attr,
+                                  cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = ClusterLayout<Real>(a.nx, a.ny, a.nz, ctas).bytes(a.nx, a.ny, a.nz);
+  cfg.stream = s;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+template <class Real, bool kEnergy>
+bool prepare_cluster(const PmeArgs<Real>& a, int ctas) {
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config<Real, kEnergy>(a, ctas, &attr, nullptr);
+  if (cfg.dynamicSmemBytes > 200 * 1024) return false;
+  auto* fn = pme_cluster<Real, kEnergy>;
+  if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+      (ctas > 8 && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                        1) != cudaSuccess)) {
+    cudaGetLastError();
+    return false;
+  }
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) cudaGetLastError();
+  return clusters > 0;
+}
+
+template <class Real>
+int pme_cluster_ctas(const PmeArgs<Real>& a) {
+  if (a.n_atoms > kClusterAtoms) return 0;
+  for (int ctas : {16, 8})
+    if (prepare_cluster<Real, false>(a, ctas) && prepare_cluster<Real, true>(a, ctas)) return ctas;
+  return 0;
+}
+
+template <class Real>
+void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, bool energy,
+                        cudaStream_t s) {
+  cudaLaunchAttribute attr;
+  if (energy) {
+    const cudaLaunchConfig_t cfg = cluster_config<Real, true>(a, ctas, &attr, s);
+    cudaLaunchKernelEx(&cfg, pme_cluster<Real, true>, a, f);
+  } else {
+    const cudaLaunchConfig_t cfg = cluster_config<Real, false>(a, ctas, &attr, s);
+    cudaLaunchKernelEx(&cfg, pme_cluster<Real, false>, a, f);
+  }
+}
+
+template int pme_cluster_ctas<float>(const PmeArgs<float>&);
+template int pme_cluster_ctas<double>(const PmeArgs<double>&);
+template void launch_pme_cluster<float>(const PmeArgs<float>&, const PmeFft&, int, bool, cudaStream_t);
+template void launch_pme_cluster<double>(const PmeArgs<double>&, const PmeFft&, int, bool, cudaStream_t);
 template size_t pme_transform_smem<float>(const PmeArgs<float>&, const PmeFft&, int);
 template size_t pme_transform_smem<double>(const PmeArgs<double>&, const PmeFft&, int);
 template void launch_pme_transform<float>(const PmeArgs<float>&, const PmeFft&, bool, cudaStream_t);

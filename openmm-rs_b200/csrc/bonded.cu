@@ -15,32 +15,35 @@ __device__ __forceinline__ void commit_pair(long long* force, int n, int i, int 
   }
 }
 
-// `seg`: the term's system in a batch (energy at energy[8 * seg]), or -1 for a single
-// system, whose warp sums are committed once.
+// `seg`: the term's system in a batch (energy at energy[8 * seg]), or -1 for a single system,
+// whose CTA sums are committed once.  A batch's terms come in system order, so the lanes of a warp
+// mostly share theirs and commit one sum.  Every thread of the CTA calls it.
+template <int kTerms>
 __device__ __forceinline__ void reduce_commit(long long* energy, double e, const double w[6],
                                               int seg) {
-  if (seg >= 0) {
-    long long* dst = energy + 8 * seg;
-    const long long ef = to_fixed(e, kEnergyScale);
-    if (ef) add_fixed(dst, ef);
-    for (int c = 0; c < 6; ++c) {
-      const long long wf = to_fixed(w[c], kEnergyScale);
-      if (wf) add_fixed(dst + 1 + c, wf);
+  constexpr unsigned FULL = 0xffffffffu;
+  long long ef = to_fixed(e, kEnergyScale);
+  long long wf[6] = {0, 0, 0, 0, 0, 0};
+  if (kTerms > kTermsEnergy)
+    for (int c = 0; c < 6; ++c) wf[c] = to_fixed(w[c], kEnergyScale);
+  const bool shared = __all_sync(FULL, seg == __shfl_sync(FULL, seg, 0));
+  if (shared) {
+    for (int off = 16; off > 0; off >>= 1) {
+      ef += __shfl_xor_sync(FULL, ef, off);
+      if (kTerms > kTermsEnergy)
+        for (int c = 0; c < 6; ++c) wf[c] += __shfl_xor_sync(FULL, wf[c], off);
     }
+  }
+  if (seg >= 0) {
+    if (shared && (threadIdx.x & 31) != 0) return;
+    long long* dst = energy + 8 * seg;
+    if (ef) add_fixed(dst, ef);
+    if (kTerms > kTermsEnergy)
+      for (int c = 0; c < 6; ++c)
+        if (wf[c]) add_fixed(dst + 1 + c, wf[c]);
     return;
   }
-  long long ef = to_fixed(e, kEnergyScale);
-  long long wf[6];
-  for (int c = 0; c < 6; ++c) wf[c] = to_fixed(w[c], kEnergyScale);
-  for (int off = 16; off > 0; off >>= 1) {
-    ef += __shfl_xor_sync(0xffffffffu, ef, off);
-    for (int c = 0; c < 6; ++c) wf[c] += __shfl_xor_sync(0xffffffffu, wf[c], off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (ef) add_fixed(energy, ef);
-    for (int c = 0; c < 6; ++c)
-      if (wf[c]) add_fixed(energy + 1 + c, wf[c]);
-  }
+  commit_cta<kTerms>(energy, ef, wf);
 }
 
 __device__ __forceinline__ void pair_virial(double w[6], double fo, const double d[3]) {
@@ -52,7 +55,7 @@ __device__ __forceinline__ void pair_virial(double w[6], double fo, const double
   w[5] -= fo * d[1] * d[2];
 }
 
-template <bool kEnergy>
+template <int kTerms>
 __global__ void exceptions_kernel(const ExceptionArgs a, int n_atoms) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   double en = 0.0, w[6] = {0, 0, 0, 0, 0, 0};
@@ -92,15 +95,15 @@ __global__ void exceptions_kernel(const ExceptionArgs a, int n_atoms) {
       fo -= cf;
     }
     commit_pair(a.force, n_atoms, p.x, p.y, fo, d);
-    if (kEnergy) {
+    if (kTerms) {
       en = ee;
-      pair_virial(w, fo, d);
+      if (kTerms > kTermsEnergy) pair_virial(w, fo, d);
     }
   }
-  if (kEnergy) reduce_commit(a.energy, en, w, seg);
+  if (kTerms) reduce_commit<kTerms>(a.energy, en, w, seg);
 }
 
-template <bool kEnergy>
+template <int kTerms>
 __global__ void bonded_kernel(const BondedArgs a, int n_atoms) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   double en = 0.0, w[6] = {0, 0, 0, 0, 0, 0};
@@ -116,9 +119,9 @@ __global__ void bonded_kernel(const BondedArgs a, int n_atoms) {
     const double dr = r - prm.x;
     const double fm = prm.y * dr / r;
     commit_pair(a.force, n_atoms, b.x, b.y, fm, d);
-    if (kEnergy) {
+    if (kTerms) {
       en = 0.5 * prm.y * dr * dr;
-      pair_virial(w, fm, d);
+      if (kTerms > kTermsEnergy) pair_virial(w, fm, d);
     }
   } else if (t < a.n_bonds + a.n_angles) {
     const int4 an = a.angles[t - a.n_bonds];
@@ -148,7 +151,7 @@ __global__ void bonded_kernel(const BondedArgs a, int n_atoms) {
       add_fixed(a.force + (long long)d * n_atoms + i, -vi);
       add_fixed(a.force + (long long)d * n_atoms + k, -vk);
       add_fixed(a.force + (long long)d * n_atoms + j, vi + vk);
-      if (kEnergy) {
+      if (kTerms > kTermsEnergy) {
         // W_ab = sum_atoms F_a r_b, positions relative to the vertex
         if (d == 0) {
           w[0] += -fi * rji[0] - fk * rjk[0];
@@ -162,29 +165,34 @@ __global__ void bonded_kernel(const BondedArgs a, int n_atoms) {
         }
       }
     }
-    if (kEnergy) en = 0.5 * prm.y * dtheta * dtheta;
+    if (kTerms) en = 0.5 * prm.y * dtheta * dtheta;
   }
-  if (kEnergy) reduce_commit(a.energy, en, w, seg);
+  if (kTerms) reduce_commit<kTerms>(a.energy, en, w, seg);
 }
 
 }  // namespace
 
-void launch_exceptions(const ExceptionArgs& a, bool energy, cudaStream_t s) {
+void launch_exceptions(const ExceptionArgs& a, int terms, cudaStream_t s) {
   if (a.n == 0) return;
-  const int n_atoms = a.n_atoms_for_force;
-  if (energy)
-    exceptions_kernel<true><<<ceil_div(a.n, 128), 128, 0, s>>>(a, n_atoms);
+  const int n_atoms = a.n_atoms_for_force, grid = ceil_div(a.n, 128);
+  if (terms == kTermsVirial)
+    exceptions_kernel<kTermsVirial><<<grid, 128, 0, s>>>(a, n_atoms);
+  else if (terms == kTermsEnergy)
+    exceptions_kernel<kTermsEnergy><<<grid, 128, 0, s>>>(a, n_atoms);
   else
-    exceptions_kernel<false><<<ceil_div(a.n, 128), 128, 0, s>>>(a, n_atoms);
+    exceptions_kernel<kTermsNone><<<grid, 128, 0, s>>>(a, n_atoms);
 }
 
-void launch_bonded(const BondedArgs& a, bool energy, cudaStream_t s) {
+void launch_bonded(const BondedArgs& a, int terms, cudaStream_t s) {
   const int total = a.n_bonds + a.n_angles;
   if (total == 0) return;
-  if (energy)
-    bonded_kernel<true><<<ceil_div(total, 128), 128, 0, s>>>(a, a.n_atoms_for_force);
+  const int grid = ceil_div(total, 128);
+  if (terms == kTermsVirial)
+    bonded_kernel<kTermsVirial><<<grid, 128, 0, s>>>(a, a.n_atoms_for_force);
+  else if (terms == kTermsEnergy)
+    bonded_kernel<kTermsEnergy><<<grid, 128, 0, s>>>(a, a.n_atoms_for_force);
   else
-    bonded_kernel<false><<<ceil_div(total, 128), 128, 0, s>>>(a, a.n_atoms_for_force);
+    bonded_kernel<kTermsNone><<<grid, 128, 0, s>>>(a, a.n_atoms_for_force);
 }
 
 }  // namespace ommb200

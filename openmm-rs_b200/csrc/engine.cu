@@ -1537,7 +1537,7 @@ PmeArgs<Real> Engine::pme_args() const {
 }
 
 template <class Real>
-void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
+void Engine::enqueue_nonbonded(int terms, bool direct, bool reciprocal, bool dump, bool pairs,
                                int step_offset, cudaStream_t direct_stream) {
   const NonbondedDef& nb = *nb_;
   // the reciprocal part of a small box needs nothing of the neighbour list: it starts before a
@@ -1552,7 +1552,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     cudaStream_t cs = profiling_ ? stream_ : pme_stream_;
     const PmeArgs<Real> m = pme_args<Real>();
     prof_begin("pme_cluster");
-    launch_pme_cluster<Real>(m, fft_, cluster_ctas_, energy, cs);
+    launch_pme_cluster<Real>(m, fft_, cluster_ctas_, terms, cs);
     prof_end();
   }
   if (nb_periodic_) {
@@ -1577,7 +1577,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     prof_end();
     if (own_fft_) {
       prof_begin("pme_transform");
-      launch_pme_transform<Real>(m, fft_, energy, ps);
+      launch_pme_transform<Real>(m, fft_, terms, ps);
       prof_end();
     } else {
     prof_begin("pme_convert");
@@ -1592,7 +1592,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
       OMMB200_CKFFT(cufftExecR2C(fft_fwd_, (cufftReal*)pme_real_, (cufftComplex*)pme_k_));
     prof_end();
     prof_begin("pme_convolve");
-    launch_pme_convolve<Real>(m, energy, ps);
+    launch_pme_convolve<Real>(m, terms, ps);
     prof_end();
     prof_begin("pme_fft_inverse");
     if (dp_)
@@ -1626,7 +1626,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
     e.alpha = alpha_;
     e.n_atoms_for_force = n_;
     prof_begin("exceptions");
-    launch_exceptions(e, energy, direct_stream);
+    launch_exceptions(e, terms, direct_stream);
     prof_end();
   }
   if (direct && pairs) {
@@ -1714,7 +1714,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
       p.cull_rounds = cull_rounds_;
     }
     prof_begin("pair");
-    launch_pair<Real>(p, elec_, energy, dump, pair_grid_, direct_stream);
+    launch_pair<Real>(p, elec_, terms, dump, pair_grid_, direct_stream);
     prof_end();
   }
   if (ps != stream_) {  // join
@@ -1723,7 +1723,7 @@ void Engine::enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool d
   }
 }
 
-void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step_offset) {
+void Engine::compute_forces(int terms, uint32_t groups, bool in_step, int step_offset) {
   // inside a captured group of steps the previous step's integrator left the forces zeroed
   if (!(in_step && capturing_ && step_offset > 0)) {
     prof_begin("zero_forces");
@@ -1750,17 +1750,17 @@ void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step
     const bool fuse = nb_gb_fusable_ && direct && !dump_mode_ && gb_on;
     gb_.fuse_nonbonded = fuse ? 1 : 0;
     if (dp_)
-      enqueue_nonbonded<double>(energy, direct, recip, dump_mode_, !fuse, step_offset, side);
+      enqueue_nonbonded<double>(terms, direct, recip, dump_mode_, !fuse, step_offset, side);
     else
-      enqueue_nonbonded<float>(energy, direct, recip, dump_mode_, !fuse, step_offset, side);
+      enqueue_nonbonded<float>(terms, direct, recip, dump_mode_, !fuse, step_offset, side);
   }
   if (gb_on) {
     auto gb = [&](int phase, const char* name) {
       prof_begin(name);
       if (dp_)
-        launch_gbsa_phase<double>(gb_, phase, energy, sm_count_, stream_);
+        launch_gbsa_phase<double>(gb_, phase, terms, sm_count_, stream_);
       else
-        launch_gbsa_phase<float>(gb_, phase, energy, sm_count_, stream_);
+        launch_gbsa_phase<float>(gb_, phase, terms, sm_count_, stream_);
       prof_end();
     };
     auto lr = [&](int phase, const char* name) {
@@ -1796,7 +1796,7 @@ void Engine::compute_forces(bool energy, uint32_t groups, bool in_step, int step
   for (auto& L : bonded_) {
     if (!((groups >> L.group) & 1u)) continue;
     prof_begin("bonded");
-    launch_bonded(L.args, energy, side);
+    launch_bonded(L.args, terms, side);
     prof_end();
   }
   if (side != stream_) {
@@ -1848,7 +1848,7 @@ IntegrateArgs Engine::integrate_args(int step_offset) const {
 }
 
 void Engine::enqueue_step(int step_offset, int group) {
-  compute_forces(false, integ_->integration_force_groups, true, step_offset);
+  compute_forces(kTermsNone, integ_->integration_force_groups, true, step_offset);
   IntegrateArgs a = integrate_args(step_offset);
   a.zero_force = 1;
   if (packed_by_integrator()) {
@@ -2029,7 +2029,7 @@ void Engine::set_velocities_to_temperature(double temperature, int seed) {
   }
   // LFMiddle velocity_time_offset = dt/2 (langevin.rs:204-206): v -= F/m * dt/2
   const double offset = 0.5 * integ_->step_size;
-  compute_forces_checked(false, 0xffffffffu);
+  compute_forces_checked(kTermsNone, 0xffffffffu);
   std::vector<long long> f(3 * (size_t)n_);
   OMMB200_CK(cudaMemcpyAsync(f.data(), force_, 8 * f.size(), cudaMemcpyDeviceToHost, stream_));
   sync();
@@ -2079,11 +2079,11 @@ void Engine::apply_velocity_constraints(double tolerance) {
 // compute_forces with the energy sums zeroed first and `outputs` enqueued behind it,
 // synchronised, and run again after the neighbour list grew when it overflowed; any other device
 // error is raised.
-void Engine::compute_forces_checked(bool energy, uint32_t groups,
+void Engine::compute_forces_checked(int terms, uint32_t groups,
                                     const std::function<void()>& outputs) {
   for (;;) {
     OMMB200_CK(cudaMemsetAsync(energy_, 0, 8 * segments_.size() * sizeof(long long), stream_));
-    compute_forces(energy, groups);
+    compute_forces(terms, groups);
     if (outputs) outputs();
     const int st = take_status();
     if (st == kStatusTileOverflow && grow_neighbor_capacity()) continue;
@@ -2092,22 +2092,22 @@ void Engine::compute_forces_checked(bool energy, uint32_t groups,
   }
 }
 
-// Forces (into `forces`, may be null) and, with `energy`, the fixed-point energy/virial
-// terms of every segment: [8 * segment + (energy, virial xx yy zz xy xz yz)].  `outputs`:
+// Forces (into `forces`, may be null) and the fixed-point energy/virial sums that `terms` asks for
+// of every segment: [8 * segment + (energy, virial xx yy zz xy xz yz)].  `outputs`:
 // further device-to-host copies of the same call.
-std::vector<long long> Engine::evaluate(bool energy, uint32_t groups, double* forces,
+std::vector<long long> Engine::evaluate(int terms, uint32_t groups, double* forces,
                                         const std::function<void()>& outputs) {
-  std::vector<long long> terms(8 * segments_.size());
-  compute_forces_checked(energy, groups, [&] {
+  std::vector<long long> sums(8 * segments_.size());
+  compute_forces_checked(terms, groups, [&] {
     if (forces) {
       launch_state_forces(n_, force_, scratch3_, stream_);
       OMMB200_CK(cudaMemcpyAsync(forces, scratch3_, 24 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
     }
-    OMMB200_CK(cudaMemcpyAsync(terms.data(), energy_, 8 * terms.size(), cudaMemcpyDeviceToHost, stream_));
+    OMMB200_CK(cudaMemcpyAsync(sums.data(), energy_, 8 * sums.size(), cudaMemcpyDeviceToHost, stream_));
     if (outputs) outputs();
   });
   harvest_profile();
-  return terms;
+  return sums;
 }
 
 void Engine::segment_energies(uint32_t groups, double* potential, double* kinetic) {
@@ -2120,7 +2120,7 @@ void Engine::segment_energies(uint32_t groups, double* potential, double* kineti
     return;
   }
   if (potential) {
-    std::vector<long long> terms = evaluate(true, groups, nullptr);
+    std::vector<long long> terms = evaluate(kTermsEnergy, groups, nullptr);
     for (int s = 0; s < ns; ++s) potential[s] = (double)terms[8 * s] * kEnergyScaleInv;
   }
   if (kinetic) {
@@ -2151,7 +2151,8 @@ void Engine::get_state(int flags, uint32_t groups, double* pos, double* vel, dou
   };
   long long e[8] = {0};
   if (need_forces) {
-    std::vector<long long> terms = evaluate(need_energy, groups, forces, outputs);
+    const int sums = (flags & OMMB200_STATE_VIRIAL) ? kTermsVirial : need_energy ? kTermsEnergy : kTermsNone;
+    std::vector<long long> terms = evaluate(sums, groups, forces, outputs);
     for (size_t k = 0; k < terms.size(); ++k) e[k % 8] += terms[k];
   } else {
     outputs();
@@ -2168,7 +2169,10 @@ void Engine::get_state(int flags, uint32_t groups, double* pos, double* vel, dou
   const double pe = assemble_energy(e, need_energy ? groups : 0u, w);
   info->potential_energy = need_energy ? pe : 0.0;
   const double vir[9] = {w[0], w[3], w[4], w[3], w[1], w[5], w[4], w[5], w[2]};
-  std::copy(vir, vir + 9, info->virial);
+  if (flags & OMMB200_STATE_VIRIAL)
+    std::copy(vir, vir + 9, info->virial);
+  else
+    std::fill(info->virial, info->virial + 9, 0.0);
 }
 
 double Engine::assemble_energy(const long long e[8], uint32_t groups, double w[6]) const {
@@ -2194,7 +2198,7 @@ double Engine::assemble_energy(const long long e[8], uint32_t groups, double w[6
 
 double Engine::potential_energy(uint32_t groups) {
   long long e[8] = {0};
-  const std::vector<long long> terms = evaluate(true, groups, nullptr);
+  const std::vector<long long> terms = evaluate(kTermsEnergy, groups, nullptr);
   for (size_t k = 0; k < terms.size(); ++k) e[k % 8] += terms[k];
   double w[6];
   return assemble_energy(e, groups, w);
@@ -2654,7 +2658,7 @@ int64_t Engine::debug_pair_list(int64_t max_pairs, int32_t* pairs) {
   try {
     for (;;) {  // an overflowing list grows and the dump starts again
       OMMB200_CK(cudaMemsetAsync(dump_count_, 0, 8, stream_));
-      compute_forces(false, 0xffffffffu);
+      compute_forces(kTermsNone, 0xffffffffu);
       sync();
       const int st = take_status();
       if (st == kStatusTileOverflow && grow_neighbor_capacity()) continue;

@@ -188,13 +188,13 @@ class Engine {
   PruneArgs prune_args() const;
   // `in_step`: an MD step's evaluation (the learned radii may judge and train there);
   // `step_offset`: its position inside the captured group of steps.
-  void compute_forces(bool energy, uint32_t groups, bool in_step = false, int step_offset = 0);
-  void compute_forces_checked(bool energy, uint32_t groups,
+  void compute_forces(int terms, uint32_t groups, bool in_step = false, int step_offset = 0);
+  void compute_forces_checked(int terms, uint32_t groups,
                               const std::function<void()>& outputs = {});
   void request_rebuild();
   void setup_learned(const LearnedRadiiDef& def);
   void upload_nonbonded_parameters(const NonbondedDef& nb);
-  std::vector<long long> evaluate(bool energy, uint32_t groups, double* forces,
+  std::vector<long long> evaluate(int terms, uint32_t groups, double* forces,
                                   const std::function<void()>& outputs = {});
   // One step of a group of `group` (1 outside a captured group).
   void enqueue_step(int step_offset, int group);
@@ -228,7 +228,7 @@ class Engine {
   void sync();
   void destroy_graph();
   template <class Real>
-  void enqueue_nonbonded(bool energy, bool direct, bool reciprocal, bool dump, bool pairs,
+  void enqueue_nonbonded(int terms, bool direct, bool reciprocal, bool dump, bool pairs,
                          int step_offset, cudaStream_t direct_stream);
   bool gb_packed_by_integrator() const;
   template <class Real>

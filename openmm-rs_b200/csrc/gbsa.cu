@@ -51,7 +51,7 @@ __device__ __forceinline__ bool within_cutoff(const GbArgs& a, float r2) {
 // GB pair term, sharing the distance, 1/r and the force rotation.  Pass 2 reads each slot's
 // Born radius with its reciprocal, so r^2 / (4 R_i R_j) needs no division, and needs r itself
 // only for the cutoff (kCutoff) and 1/r only for the nonbonded terms.
-template <int kPass, bool kEnergy, bool kCutoff, bool kNb = false>
+template <int kPass, int kTerms, bool kCutoff, bool kNb = false>
 __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
   using Real = double;
   if (kPass != 2 && a.use_learned && *a.use_learned) return;  // the network replaces them
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
           const Real bd = Real(-0.5) * pe * ex * (Real(1) + d) * inv2;
           acc_i += bd * bj.x;
           if (!self) acc_j += bd * bi.x;
-          if (kEnergy) {
+          if (kTerms) {
             const double e = kCutoff ? (double)pe - (double)coefficient / a.cutoff : (double)pe;
             e_tile += (self ? 0.5 : 1.0) * e;
           }
@@ -155,19 +155,21 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
             const T4 nbj = s_nb[w][jl];
             PairArgs<Real> none{};
             Real f_nb, en_nb;
-            pair_terms_r<Real, kElecCoulomb, kEnergy, false>(none, r2, inv_r, nbi.x * nbj.x,
+            pair_terms_r<Real, kElecCoulomb, kTerms, false>(none, r2, inv_r, nbi.x * nbj.x,
                                                              nbi.y + nbj.y, nbi.z * nbj.z, f_nb,
                                                              en_nb);
             fo += f_nb;
-            if (kEnergy) {
+            if (kTerms) {
               const double scale = self ? 0.5 : 1.0;
               e_nb += scale * (double)en_nb;
-              w_nb[0] -= scale * (double)(f_nb * dx * dx);
-              w_nb[1] -= scale * (double)(f_nb * dy * dy);
-              w_nb[2] -= scale * (double)(f_nb * dz * dz);
-              w_nb[3] -= scale * (double)(f_nb * dx * dy);
-              w_nb[4] -= scale * (double)(f_nb * dx * dz);
-              w_nb[5] -= scale * (double)(f_nb * dy * dz);
+              if (kTerms > kTermsEnergy) {
+                w_nb[0] -= scale * (double)(f_nb * dx * dx);
+                w_nb[1] -= scale * (double)(f_nb * dy * dy);
+                w_nb[2] -= scale * (double)(f_nb * dz * dz);
+                w_nb[3] -= scale * (double)(f_nb * dx * dy);
+                w_nb[4] -= scale * (double)(f_nb * dx * dz);
+                w_nb[5] -= scale * (double)(f_nb * dy * dz);
+              }
             }
           }
         }
@@ -218,21 +220,21 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
         if (!self && aj >= 0) add_fixed(a.dedr_sum + aj, to_fixed((double)acc_j, kForceScale));
       }
     }
-    if (kEnergy && kPass == 2) {
+    if (kTerms && kPass == 2) {
       for (int off = 16; off > 0; off >>= 1) e_tile += __shfl_xor_sync(FULL, e_tile, off);
-      const long long ef = to_fixed(e_tile, kEnergyScale);
-      if (lane == 0 && ef) add_fixed(a.energy + 8 * a.block_segment[I], ef);
+      long long ef = to_fixed(e_tile, kEnergyScale);
+      long long* dst = a.energy + 8 * a.block_segment[I];
       if constexpr (kNb) {  // rounded per tile on its own, as the nonbonded pair kernel does
         for (int off = 16; off > 0; off >>= 1) {
           e_nb += __shfl_xor_sync(FULL, e_nb, off);
-          for (int c = 0; c < 6; ++c) w_nb[c] += __shfl_xor_sync(FULL, w_nb[c], off);
+          if (kTerms > kTermsEnergy)
+            for (int c = 0; c < 6; ++c) w_nb[c] += __shfl_xor_sync(FULL, w_nb[c], off);
         }
-        if (lane == 0) {
-          long long* dst = a.energy + 8 * a.block_segment[I];
-          add_fixed(dst, to_fixed(e_nb, kEnergyScale));
+        ef += to_fixed(e_nb, kEnergyScale);
+        if (kTerms > kTermsEnergy && lane == 0)
           for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_nb[c], kEnergyScale));
-        }
       }
+      if (lane == 0 && ef) add_fixed(dst, ef);
     }
     __syncwarp();
   }
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(128) gb_pass(const GbArgs a) {
 // without exclusion take a loop without masks; self tiles (each pair seen from both sides, i
 // sums only, half energy), padded and excluded tiles apply bit masks kept in step order, and so
 // do all tiles when there is a cutoff (r <= cutoff, gbsa_obc.rs:169).
-template <bool kEnergy, bool kNb, bool kCutoff>
+template <int kTerms, bool kNb, bool kCutoff>
 __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ float4 s_pos[4][32];                // x, y, z, q sqrt|prefactor|
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
         const float2 pi2 = x2::mul(pen, x2::mul(inv, inv));          // -pe / den^2
         float2 fo = x2::mul(pi2, x2::fma(x2::bc(-0.25f), ex, x2::bc(1.f)));
         float2 bd = x2::mul(x2::mul(pi2, ex), x2::fma(d, x2::bc(0.5f), x2::bc(0.5f)));
-        if (kEnergy) {
+        if (kTerms) {
           const double sc = self ? 0.5 : 1.0;
           // with a cutoff the pair energy is shifted by -prefactor q_i q_j / cutoff
           const double inv_rc = kCutoff ? 1.0 / a.cutoff : 0.0;
@@ -372,7 +374,7 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
           const float2 qq = x2::mul(nq, x2::bc(nj.x));
           float2 f_nb = x2::sub(f_lj, x2::mul(x2::mul(qq, inv_r), inv_r2));
           if (kMasked) f_nb = x2::select(u1 && x1, u2 && x2v, f_nb, 0.f);
-          if (kEnergy) {
+          if (kTerms) {
             const double sc = self ? 0.5 : 1.0;
             const float2 e_lj = x2::mul(e6, x2::add(s6, x2::bc(-1.f)));
             const float2 e_el = x2::mul(qq, inv_r);
@@ -384,6 +386,7 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
               if (!(h ? (u2 && x2v) : (u1 && x1))) continue;
               const float elj = h ? (eps4.y == 0.f ? 0.f : e_lj.y) : (eps4.x == 0.f ? 0.f : e_lj.x);
               e_nb += sc * ((double)elj + (double)(h ? e_el.y : e_el.x));
+              if (kTerms == kTermsEnergy) continue;
               w_nb[0] -= sc * (double)(h ? wxx.y : wxx.x);
               w_nb[1] -= sc * (double)(h ? wyy.y : wyy.x);
               w_nb[2] -= sc * (double)(h ? wzz.y : wzz.x);
@@ -445,21 +448,21 @@ __global__ void __launch_bounds__(128) gb_pairs_x2(const GbArgs a) {
       add_fixed(a.force + 2 * a.n_atoms + aj, to_fixed(fjz, fs));
       add_fixed(a.dedr_sum + aj, to_fixed((double)acc_j, kForceScale));
     }
-    if (kEnergy) {
+    if (kTerms) {
       for (int off = 16; off > 0; off >>= 1) e_gb += __shfl_xor_sync(FULL, e_gb, off);
-      const long long ef = to_fixed(e_gb, kEnergyScale);
-      if (lane == 0 && ef) add_fixed(a.energy + 8 * a.block_segment[I], ef);
-      if constexpr (kNb) {
+      long long ef = to_fixed(e_gb, kEnergyScale);
+      long long* dst = a.energy + 8 * a.block_segment[I];
+      if constexpr (kNb) {  // rounded per tile on its own, as the nonbonded pair kernel does
         for (int off = 16; off > 0; off >>= 1) {
           e_nb += __shfl_xor_sync(FULL, e_nb, off);
-          for (int c = 0; c < 6; ++c) w_nb[c] += __shfl_xor_sync(FULL, w_nb[c], off);
+          if (kTerms > kTermsEnergy)
+            for (int c = 0; c < 6; ++c) w_nb[c] += __shfl_xor_sync(FULL, w_nb[c], off);
         }
-        if (lane == 0) {
-          long long* dst = a.energy + 8 * a.block_segment[I];
-          add_fixed(dst, to_fixed(e_nb, kEnergyScale));
+        ef += to_fixed(e_nb, kEnergyScale);
+        if (kTerms > kTermsEnergy && lane == 0)
           for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_nb[c], kEnergyScale));
-        }
       }
+      if (lane == 0 && ef) add_fixed(dst, ef);
     }
     __syncwarp();
   }
@@ -658,17 +661,11 @@ __global__ void __launch_bounds__(128) gb_descreen_x2(const GbArgs a) {
   }
 }
 
-// gbsa_obc.rs:214-237: radii, chain factor, self + ACE energies, dE/dR from them.
-template <class Real, bool kEnergy>
-__global__ void gb_radii(const GbArgs a) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n_slots) return;
-  const int atom = a.slot_atom[s];
-  typename V4<Real>::T2* born = reinterpret_cast<typename V4<Real>::T2*>(a.born_slot);
-  if (atom < 0) {
-    born[s].x = born[s].y = Real(1);
-    return;
-  }
+// gbsa_obc.rs:214-237 of one particle: radius, chain factor, dE/dR from the self and ACE energies,
+// which it returns.
+template <class Real>
+__device__ __forceinline__ double radius_terms(const GbArgs& a, int s, int atom,
+                                               typename V4<Real>::T2* born) {
   const double rho = a.radius[atom];
   const double offset = rho - kDielectricOffset;
   const double integral = (a.use_learned && *a.use_learned)
@@ -695,7 +692,25 @@ __global__ void gb_radii(const GbArgs a) {
     dedr -= 6.0 * area / R;
   }
   a.dedr_self[atom] = dedr;
-  if (kEnergy) add_fixed(a.energy + 8 * a.atom_segment[atom], to_fixed(e, kEnergyScale));
+  return e;
+}
+
+template <class Real, int kTerms>
+__global__ void gb_radii(const GbArgs a) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n_slots) return;  // whole warps: n_slots is a multiple of 32
+  const int atom = a.slot_atom[s];
+  typename V4<Real>::T2* born = reinterpret_cast<typename V4<Real>::T2*>(a.born_slot);
+  if (kTerms) {  // a block's particles are of one system: one sum per warp
+    long long ef = atom >= 0 ? to_fixed(radius_terms<Real>(a, s, atom, born), kEnergyScale) : 0;
+    if (atom < 0) born[s].x = born[s].y = Real(1);
+    for (int off = 16; off > 0; off >>= 1) ef += __shfl_xor_sync(0xffffffffu, ef, off);
+    if ((s & 31) == 0) add_fixed(a.energy + 8 * a.block_segment[s >> 5], ef);
+  } else if (atom >= 0) {
+    radius_terms<Real>(a, s, atom, born);
+  } else {
+    born[s].x = born[s].y = Real(1);
+  }
 }
 
 // gbsa_obc.rs:261-263
@@ -767,29 +782,29 @@ __global__ void gb_pack(const GbArgs a) {
 }  // namespace
 
 // Pass `kPass` in the form for Real: FP32 packed, FP64 one pair per lane.
-template <class Real, int kPass, bool kEnergy, bool kNb, bool kCutoff>
+template <class Real, int kPass, int kTerms, bool kNb, bool kCutoff>
 void launch_gb_pass(const GbArgs& a, int grid, cudaStream_t s) {
   if constexpr (sizeof(Real) == 8)
-    gb_pass<kPass, kEnergy, kCutoff, kNb><<<grid, 128, 0, s>>>(a);
+    gb_pass<kPass, kTerms, kCutoff, kNb><<<grid, 128, 0, s>>>(a);
   else if constexpr (kPass == 2)
-    gb_pairs_x2<kEnergy, kNb, kCutoff><<<grid, 128, 0, s>>>(a);
+    gb_pairs_x2<kTerms, kNb, kCutoff><<<grid, 128, 0, s>>>(a);
   else
     gb_descreen_x2<kPass, kCutoff><<<grid, 128, 0, s>>>(a);
 }
 
 // `fuse`: the NoCutoff nonbonded terms join pass 2 (never with a cutoff).
-template <class Real, int kPass, bool kEnergy>
+template <class Real, int kPass, int kTerms>
 void launch_gb_pass(const GbArgs& a, bool fuse, int grid, cudaStream_t s) {
   if (a.use_cutoff)
-    launch_gb_pass<Real, kPass, kEnergy, false, true>(a, grid, s);
+    launch_gb_pass<Real, kPass, kTerms, false, true>(a, grid, s);
   else if (kPass == 2 && fuse)
-    launch_gb_pass<Real, kPass, kEnergy, kPass == 2, false>(a, grid, s);
+    launch_gb_pass<Real, kPass, kTerms, kPass == 2, false>(a, grid, s);
   else
-    launch_gb_pass<Real, kPass, kEnergy, false, false>(a, grid, s);
+    launch_gb_pass<Real, kPass, kTerms, false, false>(a, grid, s);
 }
 
 template <class Real>
-void launch_gbsa_phase(const GbArgs& a, int phase, bool energy, int sm_count, cudaStream_t s) {
+void launch_gbsa_phase(const GbArgs& a, int phase, int terms, int sm_count, cudaStream_t s) {
   const int tb = 256;
   const int gs = ceil_div(a.n_slots, tb);
   const int gt = (int)std::min<long long>((a.n_tiles + 3) / 4, (long long)sm_count * 16);
@@ -798,30 +813,33 @@ void launch_gbsa_phase(const GbArgs& a, int phase, bool energy, int sm_count, cu
       gb_pack<Real><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass1:
-      launch_gb_pass<Real, 1, false>(a, false, gt, s);
+      launch_gb_pass<Real, 1, kTermsNone>(a, false, gt, s);
       break;
     case kGbRadii:
-      if (energy)
-        gb_radii<Real, true><<<gs, tb, 0, s>>>(a);
+      if (terms)
+        gb_radii<Real, kTermsEnergy><<<gs, tb, 0, s>>>(a);
       else
-        gb_radii<Real, false><<<gs, tb, 0, s>>>(a);
+        gb_radii<Real, kTermsNone><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass2:
-      if (energy)
-        launch_gb_pass<Real, 2, true>(a, a.fuse_nonbonded != 0, gt, s);
+      // GBSAOBCForce adds no virial: only the fused nonbonded terms have one
+      if (terms == kTermsVirial && a.fuse_nonbonded)
+        launch_gb_pass<Real, 2, kTermsVirial>(a, true, gt, s);
+      else if (terms)
+        launch_gb_pass<Real, 2, kTermsEnergy>(a, a.fuse_nonbonded != 0, gt, s);
       else
-        launch_gb_pass<Real, 2, false>(a, a.fuse_nonbonded != 0, gt, s);
+        launch_gb_pass<Real, 2, kTermsNone>(a, a.fuse_nonbonded != 0, gt, s);
       break;
     case kGbChain:
       gb_chain<Real><<<gs, tb, 0, s>>>(a);
       break;
     case kGbPass3:
-      launch_gb_pass<Real, 3, false>(a, false, gt, s);
+      launch_gb_pass<Real, 3, kTermsNone>(a, false, gt, s);
       break;
   }
 }
 
-template void launch_gbsa_phase<float>(const GbArgs&, int, bool, int, cudaStream_t);
-template void launch_gbsa_phase<double>(const GbArgs&, int, bool, int, cudaStream_t);
+template void launch_gbsa_phase<float>(const GbArgs&, int, int, int, cudaStream_t);
+template void launch_gbsa_phase<double>(const GbArgs&, int, int, int, cudaStream_t);
 
 }  // namespace ommb200

@@ -159,7 +159,7 @@ struct PairArgs {
 };
 
 template <class Real>
-void launch_pair(const PairArgs<Real>& a, int elec, bool energy, bool dump, int grid,
+void launch_pair(const PairArgs<Real>& a, int elec, int terms, bool dump, int grid,
                  cudaStream_t s);
 
 // Packing of block-local coordinates and LJ parameters into the sorted slots; `block_box` (may be
@@ -248,7 +248,7 @@ size_t pme_transform_smem(const PmeArgs<Real>& a, const PmeFft& f, int kernel);
 template <class Real>
 void prepare_pme_transform(const PmeArgs<Real>& a, const PmeFft& f);
 template <class Real>
-void launch_pme_transform(const PmeArgs<Real>& a, const PmeFft& f, bool energy, cudaStream_t s);
+void launch_pme_transform(const PmeArgs<Real>& a, const PmeFft& f, int terms, cudaStream_t s);
 // The whole reciprocal part in one launch of one thread-block cluster, for boxes of at most
 // kClusterAtoms particles whose grid fits the cluster's shared memory: the cluster size, 0 where
 // it does not apply.  Its shared-memory sums hold sum |q| up to kClusterCharge.
@@ -257,12 +257,12 @@ constexpr double kClusterCharge = 8192.0;  // e: a grid point gets at most 0.22 
 template <class Real>
 int pme_cluster_ctas(const PmeArgs<Real>& a);
 template <class Real>
-void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, bool energy,
+void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, int terms,
                         cudaStream_t s);
 template <class Real>
 void launch_pme_convert(const PmeArgs<Real>& a, cudaStream_t s);
 template <class Real>
-void launch_pme_convolve(const PmeArgs<Real>& a, bool energy, cudaStream_t s);
+void launch_pme_convolve(const PmeArgs<Real>& a, int terms, cudaStream_t s);
 template <class Real>
 void launch_pme_gather(const PmeArgs<Real>& a, cudaStream_t s);
 
@@ -386,7 +386,7 @@ void launch_learned_phase(const LearnedGbArgs& a, const GbArgs& g, int phase, in
 // GBSAOBCForce launches, in step order.
 enum GbPhase : int { kGbPack, kGbPass1, kGbRadii, kGbPass2, kGbChain, kGbPass3 };
 template <class Real>
-void launch_gbsa_phase(const GbArgs& a, int phase, bool energy, int sm_count, cudaStream_t s);
+void launch_gbsa_phase(const GbArgs& a, int phase, int terms, int sm_count, cudaStream_t s);
 
 // ---- exceptions and bonded terms (exceptions always in f64) ------------------------------
 struct ExceptionArgs {
@@ -403,7 +403,7 @@ struct ExceptionArgs {
   int n_atoms_for_force;  // row stride of the [3][N] force array
   const int* atom_segment;  // batch: system of each particle, energy at energy[8 * system]
 };
-void launch_exceptions(const ExceptionArgs& a, bool energy, cudaStream_t s);
+void launch_exceptions(const ExceptionArgs& a, int terms, cudaStream_t s);
 
 struct BondedArgs {
   int n_bonds;
@@ -421,7 +421,7 @@ struct BondedArgs {
   int n_atoms_for_force;
   const int* atom_segment;  // batch: system of each particle, energy at energy[8 * system]
 };
-void launch_bonded(const BondedArgs& a, bool energy, cudaStream_t s);
+void launch_bonded(const BondedArgs& a, int terms, cudaStream_t s);
 
 // ---- integration -----------------------------------------------------------------------
 struct WaterGeometry {

@@ -25,7 +25,7 @@ namespace {
 
 constexpr int kPairWarps = 4;
 
-template <class Real, int kElec, bool kEnergy, bool kDump, bool kSwitch>
+template <class Real, int kElec, int kTerms, bool kDump, bool kSwitch>
 __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Real> a) {
   using T4 = typename V4<Real>::T4;
   using T2 = typename V4<Real>::T2;
@@ -121,21 +121,23 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Re
         }
       }
       Real fo, en;
-      pair_terms<Real, kElec, kEnergy, kSwitch>(a, use ? r2 : Real(1), pi.w * pj.w, li.x + lj.x,
+      pair_terms<Real, kElec, kTerms, kSwitch>(a, use ? r2 : Real(1), pi.w * pj.w, li.x + lj.x,
                                                 li.y * lj.y, fo, en);
       fo = use ? fo : Real(0);
       fix = fma(fo, dx, fix);
       fiy = fma(fo, dy, fiy);
       fiz = fma(fo, dz, fiz);
-      if (kEnergy && use) {
+      if (kTerms && use) {
         const double scale = self ? 0.5 : 1.0;
         e_tile += scale * (double)en;
-        w_tile[0] -= scale * (double)(fo * dx * dx);
-        w_tile[1] -= scale * (double)(fo * dy * dy);
-        w_tile[2] -= scale * (double)(fo * dz * dz);
-        w_tile[3] -= scale * (double)(fo * dx * dy);
-        w_tile[4] -= scale * (double)(fo * dx * dz);
-        w_tile[5] -= scale * (double)(fo * dy * dz);
+        if (kTerms > kTermsEnergy) {
+          w_tile[0] -= scale * (double)(fo * dx * dx);
+          w_tile[1] -= scale * (double)(fo * dy * dy);
+          w_tile[2] -= scale * (double)(fo * dz * dz);
+          w_tile[3] -= scale * (double)(fo * dx * dy);
+          w_tile[4] -= scale * (double)(fo * dx * dz);
+          w_tile[5] -= scale * (double)(fo * dy * dz);
+        }
       }
       if (!self) {
         fjx = fma(-fo, dx, fjx);
@@ -157,32 +159,30 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Re
       add_fixed(a.force + a.n_atoms + aj, to_fixed(fjy, fscale));
       add_fixed(a.force + 2 * a.n_atoms + aj, to_fixed(fjz, fscale));
     }
-    if (kEnergy) {
+    if (kTerms) {
       // one fixed-point rounding per tile: reduce the tile's partial sums across the warp in
       // f64 first (a fixed order, so the result stays deterministic)
       for (int off = 16; off > 0; off >>= 1) {
         e_tile += __shfl_xor_sync(FULL, e_tile, off);
-        for (int c = 0; c < 6; ++c) w_tile[c] += __shfl_xor_sync(FULL, w_tile[c], off);
+        if (kTerms > kTermsEnergy)
+          for (int c = 0; c < 6; ++c) w_tile[c] += __shfl_xor_sync(FULL, w_tile[c], off);
       }
       if (a.block_segment) {  // a batch: each tile's energy goes to its own system
         if (lane == 0) {
           long long* dst = a.energy + 8 * a.block_segment[I];
           add_fixed(dst, to_fixed(e_tile, kEnergyScale));
-          for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_tile[c], kEnergyScale));
+          if (kTerms > kTermsEnergy)
+            for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_tile[c], kEnergyScale));
         }
       } else {
         e_fixed += to_fixed(e_tile, kEnergyScale);
-        for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_tile[c], kEnergyScale);
+        if (kTerms > kTermsEnergy)
+          for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_tile[c], kEnergyScale);
       }
     }
     __syncwarp();
   }
-  if (kEnergy && !a.block_segment) {
-    if (lane == 0) {
-      add_fixed(a.energy, e_fixed);
-      for (int c = 0; c < 6; ++c) add_fixed(a.energy + 1 + c, w_fixed[c]);
-    }
-  }
+  if (kTerms && !a.block_segment) commit_cta<kTerms>(a.energy, e_fixed, w_fixed);
 }
 
 // The FP32 form with two i-particles per lane and packed (f32x2) arithmetic.  The warp splits
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Re
 // Entry data sit in shared memory already duplicated into both lanes of each packed value, so
 // a step moves no register.  The cutoff (and with it the exact decision band) applies to the
 // Ewald and reaction-field forms; the bare-Coulomb form is the no-cutoff method.
-template <int kElec, bool kEnergy, bool kDump, bool kSwitch>
+template <int kElec, int kTerms, bool kDump, bool kSwitch>
 __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairArgs<float> a) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr bool kCutoff = kElec != kElecCoulomb;
@@ -333,35 +333,37 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
           }
         }
         float2 fo, en;
-        pair_terms_x2<kElec, kEnergy, kSwitch>(
+        pair_terms_x2<kElec, kTerms, kSwitch>(
             a, x2::select(u1, u2, r2, 1.f), x2::mul(make_float2(jzq.z, jzq.w), qi),
             x2::add(make_float2(jse.x, jse.y), sgi), x2::mul(make_float2(jse.z, jse.w), epi), fo, en);
         fo = x2::select(u1, u2, fo, 0.f);
         fx = x2::fma(fo, dx, fx);
         fy = x2::fma(fo, dy, fy);
         fz = x2::fma(fo, dz, fz);
-        if (kEnergy) {
+        if (kTerms) {
           const double scale = self ? 0.5 : 1.0;
-          const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
-          const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
-                       wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
-          if (u1) {
-            e_tile += scale * (double)en.x;
-            w_tile[0] -= scale * (double)wxx.x;
-            w_tile[1] -= scale * (double)wyy.x;
-            w_tile[2] -= scale * (double)wzz.x;
-            w_tile[3] -= scale * (double)wxy.x;
-            w_tile[4] -= scale * (double)wxz.x;
-            w_tile[5] -= scale * (double)wyz.x;
-          }
-          if (u2) {
-            e_tile += scale * (double)en.y;
-            w_tile[0] -= scale * (double)wxx.y;
-            w_tile[1] -= scale * (double)wyy.y;
-            w_tile[2] -= scale * (double)wzz.y;
-            w_tile[3] -= scale * (double)wxy.y;
-            w_tile[4] -= scale * (double)wxz.y;
-            w_tile[5] -= scale * (double)wyz.y;
+          if (u1) e_tile += scale * (double)en.x;
+          if (u2) e_tile += scale * (double)en.y;
+          if (kTerms > kTermsEnergy) {
+            const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
+            const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
+                         wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
+            if (u1) {
+              w_tile[0] -= scale * (double)wxx.x;
+              w_tile[1] -= scale * (double)wyy.x;
+              w_tile[2] -= scale * (double)wzz.x;
+              w_tile[3] -= scale * (double)wxy.x;
+              w_tile[4] -= scale * (double)wxz.x;
+              w_tile[5] -= scale * (double)wyz.x;
+            }
+            if (u2) {
+              w_tile[0] -= scale * (double)wxx.y;
+              w_tile[1] -= scale * (double)wyy.y;
+              w_tile[2] -= scale * (double)wzz.y;
+              w_tile[3] -= scale * (double)wxy.y;
+              w_tile[4] -= scale * (double)wxz.y;
+              w_tile[5] -= scale * (double)wyz.y;
+            }
           }
         }
         if (!self) {
@@ -400,30 +402,28 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
       add_fixed(a.force + a.n_atoms + aj, to_fixed(fjy, fs));
       add_fixed(a.force + 2 * a.n_atoms + aj, to_fixed(fjz, fs));
     }
-    if (kEnergy) {
+    if (kTerms) {
       for (int off = 16; off > 0; off >>= 1) {
         e_tile += __shfl_xor_sync(FULL, e_tile, off);
-        for (int c = 0; c < 6; ++c) w_tile[c] += __shfl_xor_sync(FULL, w_tile[c], off);
+        if (kTerms > kTermsEnergy)
+          for (int c = 0; c < 6; ++c) w_tile[c] += __shfl_xor_sync(FULL, w_tile[c], off);
       }
       if (a.block_segment) {
         if (lane == 0) {
           long long* dst = a.energy + 8 * a.block_segment[I];
           add_fixed(dst, to_fixed(e_tile, kEnergyScale));
-          for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_tile[c], kEnergyScale));
+          if (kTerms > kTermsEnergy)
+            for (int c = 0; c < 6; ++c) add_fixed(dst + 1 + c, to_fixed(w_tile[c], kEnergyScale));
         }
       } else {
         e_fixed += to_fixed(e_tile, kEnergyScale);
-        for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_tile[c], kEnergyScale);
+        if (kTerms > kTermsEnergy)
+          for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_tile[c], kEnergyScale);
       }
     }
     __syncwarp();
   }
-  if (kEnergy && !a.block_segment) {
-    if (lane == 0) {
-      add_fixed(a.energy, e_fixed);
-      for (int c = 0; c < 6; ++c) add_fixed(a.energy + 1 + c, w_fixed[c]);
-    }
-  }
+  if (kTerms && !a.block_segment) commit_cta<kTerms>(a.energy, e_fixed, w_fixed);
 }
 
 // ---- culling form -----------------------------------------------------------------------
@@ -496,7 +496,7 @@ enum CullRound : int {
 // base + ((m + k) mod 8), with its i-slots i1 and i2, in 8 steps.  The entry's force rotates
 // one lane per step and ends in the lane whose m is the entry's position (self rounds keep no
 // entry forces: every pair is met from both sides, at half energy).
-template <int kElec, bool kEnergy, bool kDump, bool kSwitch>
+template <int kElec, int kTerms, bool kDump, bool kSwitch>
 __device__ __forceinline__ void cull_steps(const PairArgs<float>& a, const CullRing& r, int base,
                                            int m, int src, int i1, int i2, bool image, bool self,
                                            float2 npx, float2 npy, float2 npz, float2 qi,
@@ -552,35 +552,37 @@ __device__ __forceinline__ void cull_steps(const PairArgs<float>& a, const CullR
       }
     }
     float2 fo, en;
-    pair_terms_x2<kElec, kEnergy, kSwitch>(
+    pair_terms_x2<kElec, kTerms, kSwitch>(
         a, x2::select(u1, u2, r2, 1.f), x2::mul(make_float2(jzq.z, jzq.w), qi),
         x2::add(make_float2(jse.x, jse.y), sgi), x2::mul(make_float2(jse.z, jse.w), epi), fo, en);
     fo = x2::select(u1, u2, fo, 0.f);
     fx = x2::fma(fo, dx, fx);
     fy = x2::fma(fo, dy, fy);
     fz = x2::fma(fo, dz, fz);
-    if (kEnergy) {
+    if (kTerms) {
       const double scale = self ? 0.5 : 1.0;
-      const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
-      const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
-                   wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
-      if (u1) {
-        e_acc += scale * (double)en.x;
-        w_acc[0] -= scale * (double)wxx.x;
-        w_acc[1] -= scale * (double)wyy.x;
-        w_acc[2] -= scale * (double)wzz.x;
-        w_acc[3] -= scale * (double)wxy.x;
-        w_acc[4] -= scale * (double)wxz.x;
-        w_acc[5] -= scale * (double)wyz.x;
-      }
-      if (u2) {
-        e_acc += scale * (double)en.y;
-        w_acc[0] -= scale * (double)wxx.y;
-        w_acc[1] -= scale * (double)wyy.y;
-        w_acc[2] -= scale * (double)wzz.y;
-        w_acc[3] -= scale * (double)wxy.y;
-        w_acc[4] -= scale * (double)wxz.y;
-        w_acc[5] -= scale * (double)wyz.y;
+      if (u1) e_acc += scale * (double)en.x;
+      if (u2) e_acc += scale * (double)en.y;
+      if (kTerms > kTermsEnergy) {
+        const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
+        const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
+                     wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
+        if (u1) {
+          w_acc[0] -= scale * (double)wxx.x;
+          w_acc[1] -= scale * (double)wyy.x;
+          w_acc[2] -= scale * (double)wzz.x;
+          w_acc[3] -= scale * (double)wxy.x;
+          w_acc[4] -= scale * (double)wxz.x;
+          w_acc[5] -= scale * (double)wyz.x;
+        }
+        if (u2) {
+          w_acc[0] -= scale * (double)wxx.y;
+          w_acc[1] -= scale * (double)wyy.y;
+          w_acc[2] -= scale * (double)wzz.y;
+          w_acc[3] -= scale * (double)wxy.y;
+          w_acc[4] -= scale * (double)wxz.y;
+          w_acc[5] -= scale * (double)wyz.y;
+        }
       }
     }
     if (!self) {
@@ -597,7 +599,7 @@ __device__ __forceinline__ void cull_steps(const PairArgs<float>& a, const CullR
   }
 }
 
-template <int kElec, bool kEnergy, bool kDump, bool kSwitch>
+template <int kElec, int kTerms, bool kDump, bool kSwitch>
 __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const PairArgs<float> a) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ CullRing s_ring[kPairWarps];
@@ -707,7 +709,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
         const int base = mode == kRoundQueue ? kRing * h + ((h ? hd1 : hd0) & (kRing - 1)) + gsub
                                              : kRing * (h ^ (mode == kRoundSelf1)) + gsub;
         float fjx = 0.f, fjy = 0.f, fjz = 0.f;
-        cull_steps<kElec, kEnergy, kDump, kSwitch>(
+        cull_steps<kElec, kTerms, kDump, kSwitch>(
             a, rg, base, m, src8, i1, i2, mode == kRoundImage || (self && staged_image), self,
             npx, npy, npz, qi, sgi, epi, fx, fy, fz, fjx, fjy, fjz, e_acc, w_acc);
         ++n_rounds;
@@ -809,20 +811,19 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
       add_fixed(a.force + a.n_atoms + ai, to_fixed(second ? fy.y : fy.x, fs));
       add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(second ? fz.y : fz.x, fs));
     }
-    if (kEnergy) {
+    if (kTerms) {
       for (int off = 16; off > 0; off >>= 1) {
         e_acc += __shfl_xor_sync(FULL, e_acc, off);
-        for (int c = 0; c < 6; ++c) w_acc[c] += __shfl_xor_sync(FULL, w_acc[c], off);
+        if (kTerms > kTermsEnergy)
+          for (int c = 0; c < 6; ++c) w_acc[c] += __shfl_xor_sync(FULL, w_acc[c], off);
       }
       e_fixed += to_fixed(e_acc, kEnergyScale);
-      for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_acc[c], kEnergyScale);
+      if (kTerms > kTermsEnergy)
+        for (int c = 0; c < 6; ++c) w_fixed[c] += to_fixed(w_acc[c], kEnergyScale);
     }
     __syncwarp();
   }
-  if (kEnergy && lane == 0) {
-    add_fixed(a.energy, e_fixed);
-    for (int c = 0; c < 6; ++c) add_fixed(a.energy + 1 + c, w_fixed[c]);
-  }
+  if (kTerms) commit_cta<kTerms>(a.energy, e_fixed, w_fixed);
   // a warp counts itself only after its last fetch returned (the fetch's value decided the
   // loop's exit), so when the last warp counts itself no fetch is left and it may reset both
   // counters for the next launch
@@ -884,7 +885,7 @@ __global__ void pack_kernel(int n_slots, const int* sorted_atom, const double* p
 }  // namespace
 
 template <class Real>
-void launch_pair(const PairArgs<Real>& a, int elec, bool energy, bool dump, int grid,
+void launch_pair(const PairArgs<Real>& a, int elec, int terms, bool dump, int grid,
                  cudaStream_t s) {
 #define OMMB200_PAIR(E, EN, D, SW)                                                  \
   if constexpr (sizeof(Real) == 4) {                                                \
@@ -914,11 +915,13 @@ void launch_pair(const PairArgs<Real>& a, int elec, bool energy, bool dump, int 
     OMMB200_PAIR_SW(kElecCoulomb, EN, D);                          \
   }
   if (dump) {
-    OMMB200_PAIR_E(false, true)
-  } else if (energy) {
-    OMMB200_PAIR_E(true, false)
+    OMMB200_PAIR_E(kTermsNone, true)
+  } else if (terms == kTermsVirial) {
+    OMMB200_PAIR_E(kTermsVirial, false)
+  } else if (terms == kTermsEnergy) {
+    OMMB200_PAIR_E(kTermsEnergy, false)
   } else {
-    OMMB200_PAIR_E(false, false)
+    OMMB200_PAIR_E(kTermsNone, false)
   }
 #undef OMMB200_PAIR_E
 #undef OMMB200_PAIR_SW
@@ -936,8 +939,8 @@ void launch_pack(int n_slots, const int* sorted_atom, const double* pos, const i
       box, block_box);
 }
 
-template void launch_pair<float>(const PairArgs<float>&, int, bool, bool, int, cudaStream_t);
-template void launch_pair<double>(const PairArgs<double>&, int, bool, bool, int, cudaStream_t);
+template void launch_pair<float>(const PairArgs<float>&, int, int, bool, int, cudaStream_t);
+template void launch_pair<double>(const PairArgs<double>&, int, int, bool, int, cudaStream_t);
 template void launch_pack<float>(int, const int*, const double*, const int*, const double*,
                                  const double*, const double*, const double*, void*, void*,
                                  const Box<double>&, cudaStream_t, float4*);

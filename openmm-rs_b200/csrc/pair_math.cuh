@@ -98,7 +98,7 @@ __device__ __forceinline__ bool exact_inside(const double* pos, int a, int b, in
 
 // dE/dr / r and E of one pair at squared distance r2 with inv_r = 1 / sqrt(r2);
 // `eps4` = 4 sqrt(eps_i eps_j), `sig` = (sigma_i + sigma_j) / 2.
-template <class Real, int kElec, bool kEnergy, bool kSwitch>
+template <class Real, int kElec, int kTerms, bool kSwitch>
 __device__ __forceinline__ void pair_terms_r(const PairArgs<Real>& a, Real r2, Real inv_r, Real qq,
                                              Real sig, Real eps4, Real& f_over_r, Real& energy) {
   const Real inv_r2 = inv_r * inv_r;
@@ -106,7 +106,7 @@ __device__ __forceinline__ void pair_terms_r(const PairArgs<Real>& a, Real r2, R
   const Real s2 = sig * sig * inv_r2;
   const Real s6 = s2 * s2 * s2;
   Real f_lj = eps4 * s6 * fma(Real(-12), s6, Real(6)) * inv_r2;
-  Real e_lj = kEnergy ? eps4 * s6 * (s6 - Real(1)) : Real(0);
+  Real e_lj = kTerms ? eps4 * s6 * (s6 - Real(1)) : Real(0);
   if (eps4 == Real(0)) {
     f_lj = Real(0);
     e_lj = Real(0);
@@ -120,7 +120,7 @@ __device__ __forceinline__ void pair_terms_r(const PairArgs<Real>& a, Real r2, R
       const Real sw = Real(1) + t * t * t * (Real(-10) + t * (Real(15) - Real(6) * t));
       const Real dsw = Real(-30) * t * t * (Real(1) - t) * (Real(1) - t) * a.switch_inv_width;
       f_lj = sw * f_lj + (eps4 == Real(0) ? Real(0) : e_full) * dsw * inv_r;
-      e_lj = kEnergy ? e_lj * sw : Real(0);
+      e_lj = kTerms ? e_lj * sw : Real(0);
     }
   }
   Real f_el, e_el = Real(0);
@@ -136,29 +136,29 @@ __device__ __forceinline__ void pair_terms_r(const PairArgs<Real>& a, Real r2, R
       ec = erfc(a.alpha * r);
     }
     f_el = -qq * fma(ec, inv_r, a.two_alpha_sqrtpi * ex) * inv_r2;
-    if (kEnergy) e_el = qq * ec * inv_r;
+    if (kTerms) e_el = qq * ec * inv_r;
   } else if (kElec == kElecReactionField) {
     // reaction_field (nonbonded.rs:1222-1243)
     f_el = qq * (Real(2) * a.krf - inv_r * inv_r2);
-    if (kEnergy) e_el = qq * (inv_r + a.krf * r2 - a.crf);
+    if (kTerms) e_el = qq * (inv_r + a.krf * r2 - a.crf);
   } else {
     // coulomb_pair (nonbonded.rs:1186-1192)
     f_el = -qq * inv_r * inv_r2;
-    if (kEnergy) e_el = qq * inv_r;
+    if (kTerms) e_el = qq * inv_r;
   }
   f_over_r = f_lj + f_el;
   energy = e_lj + e_el;
 }
 
-template <class Real, int kElec, bool kEnergy, bool kSwitch>
+template <class Real, int kElec, int kTerms, bool kSwitch>
 __device__ __forceinline__ void pair_terms(const PairArgs<Real>& a, Real r2, Real qq, Real sig,
                                            Real eps4, Real& f_over_r, Real& energy) {
-  pair_terms_r<Real, kElec, kEnergy, kSwitch>(a, r2, rsqrt_r(r2), qq, sig, eps4, f_over_r, energy);
+  pair_terms_r<Real, kElec, kTerms, kSwitch>(a, r2, rsqrt_r(r2), qq, sig, eps4, f_over_r, energy);
 }
 
 // pair_terms for two pairs at once in the lanes of packed FP32 values (same operations and
 // rounding as the scalar FP32 form, erfc by the same fit).
-template <int kElec, bool kEnergy, bool kSwitch>
+template <int kElec, int kTerms, bool kSwitch>
 __device__ __forceinline__ void pair_terms_x2(const PairArgs<float>& a, float2 r2, float2 qq,
                                               float2 sig, float2 eps4, float2& f_over_r,
                                               float2& energy) {
@@ -169,7 +169,7 @@ __device__ __forceinline__ void pair_terms_x2(const PairArgs<float>& a, float2 r
   const float2 s6 = x2::mul(x2::mul(s2, s2), s2);
   const float2 e6 = x2::mul(eps4, s6);
   float2 f_lj = x2::mul(x2::mul(e6, x2::fma(x2::bc(-12.f), s6, x2::bc(6.f))), inv_r2);
-  float2 e_lj = kEnergy ? x2::mul(e6, x2::add(s6, x2::bc(-1.f))) : x2::bc(0.f);
+  float2 e_lj = kTerms ? x2::mul(e6, x2::add(s6, x2::bc(-1.f))) : x2::bc(0.f);
   if (eps4.x == 0.f) f_lj.x = e_lj.x = 0.f;
   if (eps4.y == 0.f) f_lj.y = e_lj.y = 0.f;
   if (kSwitch) {  // nonbonded.rs:888-900, per lane (switching is the uncommon path)
@@ -181,7 +181,7 @@ __device__ __forceinline__ void pair_terms_x2(const PairArgs<float>& a, float2 r
         const float s = 1.f + t * t * t * (-10.f + t * (15.f - 6.f * t));
         const float ds = -30.f * t * t * (1.f - t) * (1.f - t) * a.switch_inv_width;
         f = s * f + (e4 == 0.f ? 0.f : e_full) * ds * ir;
-        e = kEnergy ? e * s : 0.f;
+        e = kTerms ? e * s : 0.f;
       }
     };
     sw(r.x, eps4.x, s6.x, inv_r.x, f_lj.x, e_lj.x);
@@ -206,18 +206,18 @@ __device__ __forceinline__ void pair_terms_x2(const PairArgs<float>& a, float2 r
     const float2 ec = x2::mul(ex, p);
     const float2 v = x2::fma(ec, inv_r, x2::mul(x2::bc(a.two_alpha_sqrtpi), ex));
     f_over_r = x2::sub(f_lj, x2::mul(x2::mul(qq, v), inv_r2));
-    if (kEnergy) energy = x2::fma(x2::mul(qq, ec), inv_r, e_lj);
+    if (kTerms) energy = x2::fma(x2::mul(qq, ec), inv_r, e_lj);
   } else if (kElec == kElecReactionField) {
     // reaction_field (nonbonded.rs:1222-1243)
     f_over_r = x2::add(f_lj, x2::mul(qq, x2::sub(x2::bc(2.f * a.krf), x2::mul(inv_r, inv_r2))));
-    if (kEnergy)
+    if (kTerms)
       energy = x2::fma(qq, x2::sub(x2::fma(x2::bc(a.krf), r2, inv_r), x2::bc(a.crf)), e_lj);
   } else {
     // coulomb_pair (nonbonded.rs:1186-1192)
     f_over_r = x2::sub(f_lj, x2::mul(x2::mul(qq, inv_r), inv_r2));
-    if (kEnergy) energy = x2::fma(qq, inv_r, e_lj);
+    if (kTerms) energy = x2::fma(qq, inv_r, e_lj);
   }
-  if (!kEnergy) energy = x2::bc(0.f);
+  if (!kTerms) energy = x2::bc(0.f);
 }
 
 

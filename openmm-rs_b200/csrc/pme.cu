@@ -241,8 +241,52 @@ struct Cplx<double> {
 
 __device__ __forceinline__ double freq(int k, int n) { return k < (n + 1) / 2 ? (double)k : (double)(k - n); }
 
-template <class Real, bool kEnergy>
-__global__ void convolve_kernel(const PmeArgs<Real> a, const double* moduli) {
+// Reciprocal-space energy and virial of half-spectrum element (x, y, z) with |S|^2 = s2 and
+// influence value infl (pme.rs:307-372): the element and its conjugate partner each carry
+// half of the virial, elements with 0 < z < nz/2 count twice.
+template <int kTerms, class Real>
+__device__ __forceinline__ void mode_energy(const PmeArgs<Real>& a, int x, int y, int z, double s2,
+                                            double infl, double& e, double (&w)[6]) {
+  const double wz = (z == 0 || (a.nz % 2 == 0 && z == a.nz / 2)) ? 1.0 : 2.0;
+  e += wz * 0.5 * infl * s2;
+  if (kTerms == kTermsEnergy) return;
+  const int idx[2][3] = {{x, y, z}, {(a.nx - x) % a.nx, (a.ny - y) % a.ny, (a.nz - z) % a.nz}};
+  for (int p = 0; p < 2; ++p) {
+    const double m[3] = {freq(idx[p][0], a.nx), freq(idx[p][1], a.ny), freq(idx[p][2], a.nz)};
+    double k[3];
+    for (int c = 0; c < 3; ++c) k[c] = m[0] * a.recip[0][c] + m[1] * a.recip[1][c] + m[2] * a.recip[2][c];
+    const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
+    const double bm = a.moduli[idx[p][0]] * a.moduli[a.nx + idx[p][1]] * a.moduli[a.nx + a.ny + idx[p][2]];
+    const double pa = kPiD * kPiD / (a.alpha * a.alpha);
+    const double g_m = kOne4PiEps0 * exp(-pa * k2) / (kPiD * a.volume * k2 * bm);
+    const double em = wz * 0.5 * 0.5 * g_m * s2;
+    const double c = 2.0 * (1.0 + pa * k2) / k2;
+    w[0] += em * (1.0 - c * k[0] * k[0]);
+    w[1] += em * (1.0 - c * k[1] * k[1]);
+    w[2] += em * (1.0 - c * k[2] * k[2]);
+    w[3] -= em * c * k[0] * k[1];
+    w[4] -= em * c * k[0] * k[2];
+    w[5] -= em * c * k[1] * k[2];
+  }
+}
+
+// The CTA's sums in fixed point (every thread of the block calls it).
+template <int kTerms, class Real>
+__device__ __forceinline__ void commit_energy(const PmeArgs<Real>& a, double e, const double (&w)[6]) {
+  long long ef = to_fixed(e, kEnergyScale);
+  long long wf[6] = {0, 0, 0, 0, 0, 0};
+  if (kTerms > kTermsEnergy)
+    for (int c = 0; c < 6; ++c) wf[c] = to_fixed(w[c], kEnergyScale);
+  for (int off = 16; off > 0; off >>= 1) {
+    ef += __shfl_xor_sync(0xffffffffu, ef, off);
+    if (kTerms > kTermsEnergy)
+      for (int c = 0; c < 6; ++c) wf[c] += __shfl_xor_sync(0xffffffffu, wf[c], off);
+  }
+  commit_cta<kTerms>(a.energy, ef, wf);
+}
+
+template <class Real, int kTerms>
+__global__ void convolve_kernel(const PmeArgs<Real> a) {
   using C2 = typename Cplx<Real>::T;
   C2* g = reinterpret_cast<C2*>(a.grid_k);
   const int nzh = a.nz / 2 + 1;
@@ -252,50 +296,17 @@ __global__ void convolve_kernel(const PmeArgs<Real> a, const double* moduli) {
        i += (long long)gridDim.x * blockDim.x) {
     C2 v = g[i];
     const Real infl = a.influence[i];
-    if (kEnergy && i != 0) {
+    if (kTerms && i != 0) {
       const int z = (int)(i % nzh);
       const int y = (int)((i / nzh) % a.ny);
       const int x = (int)(i / ((long long)nzh * a.ny));
-      const double wz = (z == 0 || (a.nz % 2 == 0 && z == a.nz / 2)) ? 1.0 : 2.0;
-      const double s2 = (double)v.x * v.x + (double)v.y * v.y;
-      e += wz * 0.5 * (double)infl * s2;
-      // virial: average over the element's mode and its conjugate partner's mode
-      const int idx[2][3] = {{x, y, z}, {(a.nx - x) % a.nx, (a.ny - y) % a.ny, (a.nz - z) % a.nz}};
-      for (int p = 0; p < 2; ++p) {
-        const double m[3] = {freq(idx[p][0], a.nx), freq(idx[p][1], a.ny), freq(idx[p][2], a.nz)};
-        double k[3];
-        for (int c = 0; c < 3; ++c) k[c] = m[0] * a.recip[0][c] + m[1] * a.recip[1][c] + m[2] * a.recip[2][c];
-        const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
-        const double bm = moduli[idx[p][0]] * moduli[a.nx + idx[p][1]] * moduli[a.nx + a.ny + idx[p][2]];
-        const double pa = kPiD * kPiD / (a.alpha * a.alpha);
-        const double g_m = kOne4PiEps0 * exp(-pa * k2) / (kPiD * a.volume * k2 * bm);
-        const double em = wz * 0.5 * 0.5 * g_m * s2;
-        const double c = 2.0 * (1.0 + pa * k2) / k2;
-        w[0] += em * (1.0 - c * k[0] * k[0]);
-        w[1] += em * (1.0 - c * k[1] * k[1]);
-        w[2] += em * (1.0 - c * k[2] * k[2]);
-        w[3] -= em * c * k[0] * k[1];
-        w[4] -= em * c * k[0] * k[2];
-        w[5] -= em * c * k[1] * k[2];
-      }
+      mode_energy<kTerms>(a, x, y, z, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, w);
     }
     v.x *= infl;
     v.y *= infl;
     g[i] = v;
   }
-  if (kEnergy) {
-    long long ef = to_fixed(e, kEnergyScale);
-    long long wf[6];
-    for (int c = 0; c < 6; ++c) wf[c] = to_fixed(w[c], kEnergyScale);
-    for (int off = 16; off > 0; off >>= 1) {
-      ef += __shfl_xor_sync(0xffffffffu, ef, off);
-      for (int c = 0; c < 6; ++c) wf[c] += __shfl_xor_sync(0xffffffffu, wf[c], off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      add_fixed(a.energy, ef);
-      for (int c = 0; c < 6; ++c) add_fixed(a.energy + 1 + c, wf[c]);
-    }
-  }
+  if (kTerms) commit_energy<kTerms>(a, e, w);
 }
 
 // pme.rs:377-425.  Eight lanes per atom: lane k < 5 sums the 25 grid points of stencil plane
@@ -549,51 +560,6 @@ __device__ __forceinline__ void load_twiddles(C2* dst, const void* src, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = t[i];
 }
 
-// Reciprocal-space energy and virial of half-spectrum element (x, y, z) with |S|^2 = s2 and
-// influence value infl (pme.rs:307-372): the element and its conjugate partner each carry
-// half of the virial, elements with 0 < z < nz/2 count twice.
-template <class Real>
-__device__ __forceinline__ void mode_energy(const PmeArgs<Real>& a, int x, int y, int z, double s2,
-                                            double infl, double& e, double (&w)[6]) {
-  const double wz = (z == 0 || (a.nz % 2 == 0 && z == a.nz / 2)) ? 1.0 : 2.0;
-  e += wz * 0.5 * infl * s2;
-  const int idx[2][3] = {{x, y, z}, {(a.nx - x) % a.nx, (a.ny - y) % a.ny, (a.nz - z) % a.nz}};
-  for (int p = 0; p < 2; ++p) {
-    const double m[3] = {freq(idx[p][0], a.nx), freq(idx[p][1], a.ny), freq(idx[p][2], a.nz)};
-    double k[3];
-    for (int c = 0; c < 3; ++c) k[c] = m[0] * a.recip[0][c] + m[1] * a.recip[1][c] + m[2] * a.recip[2][c];
-    const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
-    const double bm = a.moduli[idx[p][0]] * a.moduli[a.nx + idx[p][1]] * a.moduli[a.nx + a.ny + idx[p][2]];
-    const double pa = kPiD * kPiD / (a.alpha * a.alpha);
-    const double g_m = kOne4PiEps0 * exp(-pa * k2) / (kPiD * a.volume * k2 * bm);
-    const double em = wz * 0.5 * 0.5 * g_m * s2;
-    const double c = 2.0 * (1.0 + pa * k2) / k2;
-    w[0] += em * (1.0 - c * k[0] * k[0]);
-    w[1] += em * (1.0 - c * k[1] * k[1]);
-    w[2] += em * (1.0 - c * k[2] * k[2]);
-    w[3] -= em * c * k[0] * k[1];
-    w[4] -= em * c * k[0] * k[2];
-    w[5] -= em * c * k[1] * k[2];
-  }
-}
-
-// Warp sums of the energy and virial in fixed point, one atomic per warp and term (every
-// thread of the block calls it).
-template <class Real>
-__device__ __forceinline__ void commit_energy(const PmeArgs<Real>& a, double e, const double (&w)[6]) {
-  long long ef = to_fixed(e, kEnergyScale);
-  long long wf[6];
-  for (int c = 0; c < 6; ++c) wf[c] = to_fixed(w[c], kEnergyScale);
-  for (int off = 16; off > 0; off >>= 1) {
-    ef += __shfl_xor_sync(0xffffffffu, ef, off);
-    for (int c = 0; c < 6; ++c) wf[c] += __shfl_xor_sync(0xffffffffu, wf[c], off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    add_fixed(a.energy, ef);
-    for (int c = 0; c < 6; ++c) add_fixed(a.energy + 1 + c, wf[c]);
-  }
-}
-
 // Shared memory of a plane kernel: z and y twiddles, two buffers of `plane` elements.
 __host__ __device__ inline int fft_plane_elems(int ny, int nz) {
   const int a = (ny + 1) / 2 * nz, b = (nz / 2 + 1) * ny;
@@ -681,7 +647,7 @@ __global__ void __launch_bounds__(kPlaneThreads) planes_forward(const PmeArgs<Re
   }
 }
 
-template <class Real, bool kEnergy>
+template <class Real, int kTerms>
 __global__ void __launch_bounds__(kXPassThreads) x_convolve(const PmeArgs<Real> a, const PmeFft f) {
   using C2 = typename Cplx<Real>::T;
   extern __shared__ __align__(16) unsigned char fsm[];
@@ -706,13 +672,13 @@ __global__ void __launch_bounds__(kXPassThreads) x_convolve(const PmeArgs<Real> 
       [&](int i, Real infl) {
         const int p = i / nx, x = i - p * nx;
         C2 v = r[i];
-        if (kEnergy && base + x * sx + p != 0)
-          mode_energy(a, x, y, kz0 + p, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, w);
+        if (kTerms && base + x * sx + p != 0)
+          mode_energy<kTerms>(a, x, y, kz0 + p, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, w);
         v.x *= infl;
         v.y *= -infl;  // conjugated for the inverse transform
         r[i] = v;
       });
-  if (kEnergy) commit_energy(a, e, w);
+  if (kTerms) commit_energy<kTerms>(a, e, w);
   __syncthreads();
   C2* s = stockham(r, o, tw, f, 0, nx, P);
   for (int i = threadIdx.x; i < nx * P; i += blockDim.x) {
@@ -798,7 +764,7 @@ struct ClusterLayout {  // element counts; every CTA of the cluster has the same
   }
 };
 
-template <class Real, bool kEnergy>
+template <class Real, int kTerms>
 __global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Real> a, const PmeFft f) {
   using C2 = typename Cplx<Real>::T;
   extern __shared__ __align__(16) unsigned char fsm[];
@@ -915,13 +881,13 @@ __global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Rea
     const long long at = ((long long)x * ny + y) * nzh + kz;
     const Real infl = __ldg(a.influence + at);
     C2 v = xr[i];
-    if (kEnergy && at != 0)
-      mode_energy(a, x, y, kz, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, vir);
+    if (kTerms && at != 0)
+      mode_energy<kTerms>(a, x, y, kz, (double)v.x * v.x + (double)v.y * v.y, (double)infl, e, vir);
     v.x *= infl;
     v.y *= -infl;  // conjugated for the inverse transform
     xr[i] = v;
   }
-  if (kEnergy) commit_energy(a, e, vir);
+  if (kTerms) commit_energy<kTerms>(a, e, vir);
   __syncthreads();
   C2* xs = stockham(xr, xo, twx, f, 0, nx, nq);
   // back to the owners, still conjugated: the inverse y transform starts from conj H.  Each
@@ -1012,14 +978,16 @@ size_t pme_transform_smem(const PmeArgs<Real>& a, const PmeFft& f, int kernel) {
 }
 
 template <class Real>
-void launch_pme_transform(const PmeArgs<Real>& a, const PmeFft& f, bool energy, cudaStream_t s) {
+void launch_pme_transform(const PmeArgs<Real>& a, const PmeFft& f, int terms, cudaStream_t s) {
   const size_t sp = pme_transform_smem(a, f, 0), sx = pme_transform_smem(a, f, 1);
   const int nzh = a.nz / 2 + 1, nkb = ceil_div(nzh, f.pencils_x);
   planes_forward<Real><<<a.nx, f.threads[0], sp, s>>>(a, f);
-  if (energy)
-    x_convolve<Real, true><<<a.ny * nkb, f.threads[1], sx, s>>>(a, f);
+  if (terms == kTermsVirial)
+    x_convolve<Real, kTermsVirial><<<a.ny * nkb, f.threads[1], sx, s>>>(a, f);
+  else if (terms == kTermsEnergy)
+    x_convolve<Real, kTermsEnergy><<<a.ny * nkb, f.threads[1], sx, s>>>(a, f);
   else
-    x_convolve<Real, false><<<a.ny * nkb, f.threads[1], sx, s>>>(a, f);
+    x_convolve<Real, kTermsNone><<<a.ny * nkb, f.threads[1], sx, s>>>(a, f);
   planes_inverse<Real><<<a.nx, f.threads[2], sp, s>>>(a, f);
 }
 
@@ -1028,12 +996,13 @@ void prepare_pme_transform(const PmeArgs<Real>& a, const PmeFft& f) {
   const int sp = (int)pme_transform_smem(a, f, 0), sx = (int)pme_transform_smem(a, f, 1);
   cudaFuncSetAttribute((const void*)planes_forward<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp);
   cudaFuncSetAttribute((const void*)planes_inverse<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp);
-  cudaFuncSetAttribute((const void*)x_convolve<Real, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
-  cudaFuncSetAttribute((const void*)x_convolve<Real, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
+  cudaFuncSetAttribute((const void*)x_convolve<Real, kTermsVirial>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
+  cudaFuncSetAttribute((const void*)x_convolve<Real, kTermsEnergy>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
+  cudaFuncSetAttribute((const void*)x_convolve<Real, kTermsNone>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
 }
 
 // The cluster form's launch: `ctas` CTAs of one cluster.
-template <class Real, bool kEnergy>
+template <class Real, int kTerms>
 cudaLaunchConfig_t cluster_config(const PmeArgs<Real>& a, int ctas, cudaLaunchAttribute* attr,
                                   cudaStream_t s) {
   cudaLaunchConfig_t cfg{};
@@ -1049,12 +1018,12 @@ cudaLaunchConfig_t cluster_config(const PmeArgs<Real>& a, int ctas, cudaLaunchAt
   return cfg;
 }
 
-template <class Real, bool kEnergy>
+template <class Real, int kTerms>
 bool prepare_cluster(const PmeArgs<Real>& a, int ctas) {
   cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = cluster_config<Real, kEnergy>(a, ctas, &attr, nullptr);
+  const cudaLaunchConfig_t cfg = cluster_config<Real, kTerms>(a, ctas, &attr, nullptr);
   if (cfg.dynamicSmemBytes > 200 * 1024) return false;
-  auto* fn = pme_cluster<Real, kEnergy>;
+  auto* fn = pme_cluster<Real, kTerms>;
   if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)cfg.dynamicSmemBytes) != cudaSuccess ||
       (ctas > 8 && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed,
@@ -1071,31 +1040,38 @@ template <class Real>
 int pme_cluster_ctas(const PmeArgs<Real>& a) {
   if (a.n_atoms > kClusterAtoms) return 0;
   for (int ctas : {16, 8})
-    if (prepare_cluster<Real, false>(a, ctas) && prepare_cluster<Real, true>(a, ctas)) return ctas;
+    if (prepare_cluster<Real, kTermsNone>(a, ctas) && prepare_cluster<Real, kTermsEnergy>(a, ctas) &&
+        prepare_cluster<Real, kTermsVirial>(a, ctas))
+      return ctas;
   return 0;
 }
 
-template <class Real>
-void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, bool energy,
-                        cudaStream_t s) {
+template <class Real, int kTerms>
+void launch_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, cudaStream_t s) {
   cudaLaunchAttribute attr;
-  if (energy) {
-    const cudaLaunchConfig_t cfg = cluster_config<Real, true>(a, ctas, &attr, s);
-    cudaLaunchKernelEx(&cfg, pme_cluster<Real, true>, a, f);
-  } else {
-    const cudaLaunchConfig_t cfg = cluster_config<Real, false>(a, ctas, &attr, s);
-    cudaLaunchKernelEx(&cfg, pme_cluster<Real, false>, a, f);
-  }
+  const cudaLaunchConfig_t cfg = cluster_config<Real, kTerms>(a, ctas, &attr, s);
+  cudaLaunchKernelEx(&cfg, pme_cluster<Real, kTerms>, a, f);
+}
+
+template <class Real>
+void launch_pme_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, int terms,
+                        cudaStream_t s) {
+  if (terms == kTermsVirial)
+    launch_cluster<Real, kTermsVirial>(a, f, ctas, s);
+  else if (terms == kTermsEnergy)
+    launch_cluster<Real, kTermsEnergy>(a, f, ctas, s);
+  else
+    launch_cluster<Real, kTermsNone>(a, f, ctas, s);
 }
 
 template int pme_cluster_ctas<float>(const PmeArgs<float>&);
 template int pme_cluster_ctas<double>(const PmeArgs<double>&);
-template void launch_pme_cluster<float>(const PmeArgs<float>&, const PmeFft&, int, bool, cudaStream_t);
-template void launch_pme_cluster<double>(const PmeArgs<double>&, const PmeFft&, int, bool, cudaStream_t);
+template void launch_pme_cluster<float>(const PmeArgs<float>&, const PmeFft&, int, int, cudaStream_t);
+template void launch_pme_cluster<double>(const PmeArgs<double>&, const PmeFft&, int, int, cudaStream_t);
 template size_t pme_transform_smem<float>(const PmeArgs<float>&, const PmeFft&, int);
 template size_t pme_transform_smem<double>(const PmeArgs<double>&, const PmeFft&, int);
-template void launch_pme_transform<float>(const PmeArgs<float>&, const PmeFft&, bool, cudaStream_t);
-template void launch_pme_transform<double>(const PmeArgs<double>&, const PmeFft&, bool, cudaStream_t);
+template void launch_pme_transform<float>(const PmeArgs<float>&, const PmeFft&, int, cudaStream_t);
+template void launch_pme_transform<double>(const PmeArgs<double>&, const PmeFft&, int, cudaStream_t);
 template void prepare_pme_transform<float>(const PmeArgs<float>&, const PmeFft&);
 template void prepare_pme_transform<double>(const PmeArgs<double>&, const PmeFft&);
 
@@ -1154,13 +1130,15 @@ void launch_pme_convert(const PmeArgs<Real>& a, cudaStream_t s) {
   convert_kernel<Real><<<(int)std::min<long long>((total + 255) / 256, 148LL * 16), 256, 0, s>>>(a);
 }
 template <class Real>
-void launch_pme_convolve(const PmeArgs<Real>& a, bool energy, cudaStream_t s) {
+void launch_pme_convolve(const PmeArgs<Real>& a, int terms, cudaStream_t s) {
   const long long total = (long long)a.nx * a.ny * (a.nz / 2 + 1);
   const int grid = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
-  if (energy)
-    convolve_kernel<Real, true><<<grid, 256, 0, s>>>(a, a.moduli);
+  if (terms == kTermsVirial)
+    convolve_kernel<Real, kTermsVirial><<<grid, 256, 0, s>>>(a);
+  else if (terms == kTermsEnergy)
+    convolve_kernel<Real, kTermsEnergy><<<grid, 256, 0, s>>>(a);
   else
-    convolve_kernel<Real, false><<<grid, 256, 0, s>>>(a, a.moduli);
+    convolve_kernel<Real, kTermsNone><<<grid, 256, 0, s>>>(a);
 }
 template <class Real>
 void launch_pme_gather(const PmeArgs<Real>& a, cudaStream_t s) {
@@ -1171,8 +1149,8 @@ template void launch_pme_spread<float>(const PmeArgs<float>&, cudaStream_t);
 template void launch_pme_spread<double>(const PmeArgs<double>&, cudaStream_t);
 template void launch_pme_convert<float>(const PmeArgs<float>&, cudaStream_t);
 template void launch_pme_convert<double>(const PmeArgs<double>&, cudaStream_t);
-template void launch_pme_convolve<float>(const PmeArgs<float>&, bool, cudaStream_t);
-template void launch_pme_convolve<double>(const PmeArgs<double>&, bool, cudaStream_t);
+template void launch_pme_convolve<float>(const PmeArgs<float>&, int, cudaStream_t);
+template void launch_pme_convolve<double>(const PmeArgs<double>&, int, cudaStream_t);
 template void launch_pme_gather<float>(const PmeArgs<float>&, cudaStream_t);
 template void launch_pme_gather<double>(const PmeArgs<double>&, cudaStream_t);
 

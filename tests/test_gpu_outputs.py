@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import ommb200
-from ommb200 import systems
+from ommb200 import synth, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,32 @@ def test_kinetic_energy_and_forces(n):
         f[i + 1] -= g
     # one fixed-point rounding per bond end (2^-33 kJ/mol/nm) and the f64 arithmetic's
     assert np.abs(st.forces - f).max() < 1e-9
+
+
+def _water(precision):
+    w = synth.water_box(216, 1.9, (6, 6, 6), seed=3)
+    ctx = ommb200.Context(systems.water_system(w), systems.langevin(seed=5), precision=precision)
+    ctx.set_positions(w.positions)
+    return ctx
+
+
+def _chains(precision):
+    chs = [synth.chain(n, seed=n) for n in (40, 97, 33)]
+    ctx = ommb200.BatchContext([systems.chain_system(c) for c in chs],
+                               systems.langevin(step_size=0.001), precision=precision)
+    ctx.set_positions(np.concatenate([c.positions for c in chs]))
+    return ctx
+
+
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+@pytest.mark.parametrize("make", [_water, _chains])
+def test_energy_with_and_without_the_virial(make, precision):
+    ctx = make(precision)
+    plain = ctx.get_state(forces=True, energy=True)
+    both = ctx.get_state(forces=True, energy=True, virial=True)
+    only = ctx.get_state(virial=True)
+    assert plain.virial is None
+    assert np.array_equal(plain.forces, both.forces)
+    # the same pair energies; f64 expressions may contract differently in the two forms
+    assert abs(plain.potential_energy - both.potential_energy) <= 1e-12 * abs(both.potential_energy)
+    assert np.array_equal(only.virial, both.virial) and np.abs(both.virial).max() > 0.0

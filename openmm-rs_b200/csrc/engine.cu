@@ -425,6 +425,10 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
   n_slots_ = a.slot_capacity;
   n_blocks_ = n_slots_ / 32;
   a.sorted_atom = mem_.alloc<int>(n_slots_);
+  if (nb_periodic_) {
+    a.order = mem_.alloc<int>(2 * (size_t)n_slots_);
+    a.order_parity = mem_.alloc<int>(1);
+  }
   a.atom_slot = mem_.alloc<int>(n_);
   a.image = mem_.alloc<int>(3 * (size_t)n_);
   a.slot_wpos = mem_.alloc<double4>(n_slots_);
@@ -436,6 +440,7 @@ void Engine::setup_nonbonded(const NonbondedDef& nb) {
     std::vector<int> sorted(n_slots_, -1);
     for (int i = 0; i < n_; ++i) sorted[i] = i;
     OMMB200_CK(cudaMemcpy(a.sorted_atom, sorted.data(), 4 * n_slots_, cudaMemcpyHostToDevice));
+    OMMB200_CK(cudaMemcpy(a.order, sorted.data(), 4 * n_slots_, cudaMemcpyHostToDevice));
     OMMB200_CK(cudaMemcpy(a.atom_slot, sorted.data(), 4 * n_, cudaMemcpyHostToDevice));
   } else {
     OMMB200_CK(cudaMemcpy(a.sorted_atom, static_slot_atom_.data(), 4 * n_slots_, cudaMemcpyHostToDevice));
@@ -1540,9 +1545,13 @@ template <class Real>
 void Engine::enqueue_nonbonded(int terms, bool direct, bool reciprocal, bool dump, bool pairs,
                                int step_offset, cudaStream_t direct_stream) {
   const NonbondedDef& nb = *nb_;
-  // the reciprocal part of a small box needs nothing of the neighbour list: it starts before a
-  // rebuild and runs beside it
+  // The reciprocal part needs nothing of a new neighbour list: it starts before a rebuild and runs
+  // beside it.  The one-launch form reads the particles as they come; the launch chain visits them
+  // in the sorted order of the rebuild before (its second copy, inside captured groups, where the
+  // copy's parity is set between the steps; 23,958 particles: 106 -> 102 us per step).  The brick
+  // gather does need the new slot ranges.
   const bool cluster = reciprocal && nb_pme_ && cluster_ctas_ > 0;
+  const bool early = reciprocal && nb_pme_ && !cluster && !use_bricks_ && capturing_;
   auto fork_pme = [&] {
     OMMB200_CK(cudaEventRecord(fork_ev_, stream_));
     OMMB200_CK(cudaStreamWaitEvent(pme_stream_, fork_ev_, 0));
@@ -1555,23 +1564,17 @@ void Engine::enqueue_nonbonded(int terms, bool direct, bool reciprocal, bool dum
     launch_pme_cluster<Real>(m, fft_, cluster_ctas_, terms, cs);
     prof_end();
   }
-  if (nb_periodic_) {
-    prof_begin("nlist_rebuild");
-    if (capturing_)
-      enqueue_conditional_rebuild(step_offset == 0);
-    else
-      launch_nlist_rebuild(nl_, dp_, stream_, with_new_list(nl_));
-    prof_end();
-  }
-  // fork: PME on its own stream (serialised on the main stream while profiling, so that
-  // per-kernel events time one kernel at a time)
   const bool pme = reciprocal && nb_pme_;
+  // the chain's own stream (serialised on the main stream while profiling, so that per-kernel
+  // events time one kernel at a time)
   cudaStream_t ps = (pme && !profiling_) ? pme_stream_ : stream_;
-  if (ps != stream_ && !cluster) fork_pme();
-  // the reciprocal chain is enqueued first, so its kernels reach the GPU ahead of the direct
-  // chain's (the two orders measured within run-to-run spread of each other)
-  if (pme && !cluster) {
-    const PmeArgs<Real> m = pme_args<Real>();
+  auto reciprocal_chain = [&] {
+    if (ps != stream_) fork_pme();
+    PmeArgs<Real> m = pme_args<Real>();
+    if (early) {
+      m.order = nl_.order;
+      m.order_parity = nl_.order_parity;
+    }
     prof_begin("pme_spread");
     launch_pme_spread<Real>(m, ps);
     prof_end();
@@ -1608,7 +1611,19 @@ void Engine::enqueue_nonbonded(int terms, bool direct, bool reciprocal, bool dum
     } else
       launch_pme_gather<Real>(m, ps);
     prof_end();
+  };
+  if (early) reciprocal_chain();
+  if (nb_periodic_) {
+    prof_begin("nlist_rebuild");
+    if (capturing_)
+      enqueue_conditional_rebuild(step_offset == 0);
+    else
+      launch_nlist_rebuild(nl_, dp_, stream_, with_new_list(nl_));
+    prof_end();
   }
+  // the reciprocal chain is enqueued ahead of the direct chain, so its kernels reach the GPU first
+  // (the two orders measured within run-to-run spread of each other)
+  if (pme && !cluster && !early) reciprocal_chain();
   // the exclusion corrections first: a small kernel that leaves SMs free while the reciprocal
   // chain starts beside it, before the pair kernel fills every SM
   if (direct && n_exceptions_) {
@@ -1869,6 +1884,8 @@ void Engine::enqueue_step(int step_offset, int group) {
     rebuild_condition_ = new_condition();
     a.has_condition = 1;
     a.condition = rebuild_condition_;
+    a.rebuild_count = nl_.rebuild_count;
+    a.order_parity = nl_.order_parity;
   }
   prof_begin("integrate");
   launch_integrate(a, stream_);

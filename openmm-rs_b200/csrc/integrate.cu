@@ -409,6 +409,7 @@ __device__ void cluster_step(const IntegrateArgs& a, int c, uint64_t step, int n
 __global__ void integrate_kernel(const IntegrateArgs a, int n) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t step = *a.rng_step + (uint64_t)a.step_offset;
+  if (t == 0 && a.order_parity) *a.order_parity = (int)(*a.rebuild_count & 1ull);
   if (t < 4 * a.n_water) {
     const int lane = threadIdx.x & 31;
     water_step_lanes(a, t >> 2, t & 3, step, n, 0xFu << (lane & ~3));

@@ -38,6 +38,9 @@ struct NlistArgs {
   unsigned* done;     // [2] CTAs done of the column and list kernels (zero between launches)
   int* n_blocks;      // device: blocks in use after the last rebuild
   int* sorted_atom;   // [slot_capacity] particle in each slot, -1 for padding
+  int* order;         // [2][slot_capacity] its copies, written in turn: rebuild r writes the copy
+                      //   r & 1, so a launch beside it can read the last one
+  int* order_parity;  // the copy that is complete, set between evaluations
   int* atom_slot;     // [N] inverse of sorted_atom
   double4* slot_wpos;    // [slot_capacity] wrapped rebuild position of each slot (w = 0)
   double* block_center;  // [3 * slot_capacity / 32]
@@ -176,6 +179,7 @@ struct PmeArgs {
   int n_atoms;
   const int* order;     // particle visiting order (sorted slots) or nullptr
   int n_order;
+  const int* order_parity;  // null, or which of the two orders at `order` to read
   const double* pos;
   const double* charge;
   int nx, ny, nz;
@@ -477,6 +481,8 @@ struct IntegrateArgs {
   // together with `rebuild`
   int has_condition;
   cudaGraphConditionalHandle condition;
+  const unsigned long long* rebuild_count;  // order_parity = rebuild_count & 1 (may be null)
+  int* order_parity;
 };
 void launch_integrate(const IntegrateArgs& a, cudaStream_t s);
 // Barostat volume move: positions scaled, per particle or per molecule (CSR lists of atoms)

@@ -141,9 +141,10 @@ __global__ void __launch_bounds__(256) nl_col_sort(NlistArgs a) {
   extern __shared__ unsigned long long keys[];
   const int c = blockIdx.x;
   // the slots past the last column's, shared out over the CTAs
+  int* order = a.order + (size_t)((*a.rebuild_count + 1) & 1) * a.slot_capacity;
   for (int s = a.col_start[a.n_cols] + c * 256 + threadIdx.x; s < a.slot_capacity;
        s += gridDim.x * 256)
-    a.sorted_atom[s] = -1;
+    a.sorted_atom[s] = order[s] = -1;
   const int n = a.col_size[c];
   if (n > a.col_max || n == 0) return;
   int m = 1;
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(256) nl_col_sort(NlistArgs a) {
     if (base + k0 + 32 > a.slot_capacity) break;
     const int slot = base + k0 + lane, blk = (base + k0) >> 5;
     const int atom = k0 + lane < n ? (int)(keys[k0 + lane] & 0xffffffffu) : -1;
-    a.sorted_atom[slot] = atom;
+    a.sorted_atom[slot] = order[slot] = atom;
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     double x[3] = {0.0, 0.0, 0.0}, im[3] = {0.0, 0.0, 0.0}, wp[3] = {0.0, 0.0, 0.0};
     if (atom >= 0) {
@@ -883,8 +884,10 @@ __global__ void __launch_bounds__(32 * kCtaWarps, 4) nl_lists_cta(NlistArgs a) {
 
 // Inside a captured step: the rebuild kernels sit in the body of a conditional graph node
 // that runs only when the integrator raised the flag.
-__global__ void nl_set_condition(const int* rebuild, cudaGraphConditionalHandle handle) {
+__global__ void nl_set_condition(const int* rebuild, cudaGraphConditionalHandle handle,
+                                 const unsigned long long* rebuild_count, int* order_parity) {
   cudaGraphSetConditional(handle, *rebuild != 0 ? 1u : 0u);
+  *order_parity = (int)(*rebuild_count & 1ull);
 }
 
 // Triclinic boxes: closes the rebuild (the CTA builder of rectangular boxes does it itself).
@@ -1144,7 +1147,7 @@ __global__ void nl_prune_condition(const int* prune, cudaGraphConditionalHandle 
 
 void launch_nlist_condition(const NlistArgs& a, cudaGraphConditionalHandle handle,
                             cudaStream_t s) {
-  nl_set_condition<<<1, 1, 0, s>>>(a.rebuild, handle);
+  nl_set_condition<<<1, 1, 0, s>>>(a.rebuild, handle, a.rebuild_count, a.order_parity);
 }
 
 void launch_prune_condition(const PruneArgs& p, cudaGraphConditionalHandle handle, cudaStream_t s) {

@@ -65,11 +65,19 @@ __device__ __forceinline__ bool stencil(const PmeArgs<Real>& a, int atom, int ba
   return ok;
 }
 
+// The particle in place s of the visiting order (which of its two copies is the same for every
+// thread of the launch: nothing beside it writes the parity), -1 for padding.
+template <class Real>
+__device__ __forceinline__ int ordered_atom(const PmeArgs<Real>& a, int s) {
+  if (s >= a.n_order) return -1;
+  if (!a.order) return s;
+  return a.order[a.order_parity ? (size_t)*a.order_parity * a.n_order + s : s];
+}
+
 template <class Real>
 __global__ void spread_kernel(const PmeArgs<Real> a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n_order) return;
-  const int atom = a.order ? a.order[s] : s;
+  const int atom = ordered_atom(a, s);
   if (atom < 0) return;
   const double qd = a.charge[atom];
   if (qd == 0.0) return;
@@ -111,8 +119,9 @@ __global__ void spread_kernel(const PmeArgs<Real> a) {
 // inside 32 bits for |q| < 2 e (the order-5 B-spline peaks at 115/192 per axis, so a point gets
 // at most 0.22 |q| from an atom); the box is added to the 2^-40 global grid scaled by 2^14,
 // exactly.  Either way the sums are exact integers, so the grid does not depend on the order
-// of the additions.  A CTA whose box exceeds kSpreadCells (it straddles a periodic edge of the
-// column order) or that holds a larger charge spreads directly.
+// of the additions; nor on how the particles are grouped into CTAs: a CTA whose box exceeds
+// kSpreadCells (it straddles a periodic edge of the column order) spreads directly with the same
+// rounding, and a particle of larger charge spreads directly at 2^-40 e wherever it is.
 constexpr int kSpreadAtoms = 64;
 constexpr int kSpreadCells = 4096;
 constexpr float kSpreadScale32 = 67108864.f;           // 2^26 (FP32 form, staged)
@@ -122,34 +131,32 @@ template <class Real>
 __global__ void __launch_bounds__(2 * kSpreadAtoms) spread_staged_kernel(const PmeArgs<Real> a) {
   __shared__ int c_hi[kSpreadCells];
   __shared__ unsigned int c_lo[kSpreadCells];
-  __shared__ int s_lo[3], s_hi[3], s_big;
+  __shared__ int s_lo[3], s_hi[3];
   const int tid = threadIdx.x, half = tid / kSpreadAtoms;  // half 0: ix 0..2, half 1: ix 3..4
   const int s = blockIdx.x * kSpreadAtoms + (tid % kSpreadAtoms);
-  int atom = -1;
-  if (s < a.n_order) atom = a.order ? a.order[s] : s;
+  const int atom = ordered_atom(a, s);
   const double qd = atom >= 0 ? a.charge[atom] : 0.0;
   int base[3] = {0, 0, 0};
   Real frac[3] = {Real(0), Real(0), Real(0)};
   const bool ok = atom >= 0 && qd != 0.0 && stencil(a, atom, base, frac);
+  // the 32-bit partial sums need |q| < 2 e (FP32 form) or |q| < 16 e (FP64 form)
+  const bool big = ok && fabs(qd) >= (sizeof(Real) == 4 ? 2.0 : 16.0), staged = ok && !big;
   if (tid < 3) {
     s_lo[tid] = 0x7fffffff;
     s_hi[tid] = -1;
   }
-  if (tid == 0) s_big = 0;
   __syncthreads();
-  if (ok && half == 0) {
+  if (staged && half == 0) {
     for (int d = 0; d < 3; ++d) {
       atomicMin(&s_lo[d], base[d]);
       atomicMax(&s_hi[d], base[d]);
     }
-    // the 32-bit partial sums need |q| < 2 e (FP32 form) or |q| < 16 e (FP64 form)
-    if (fabs(qd) >= (sizeof(Real) == 4 ? 2.0 : 16.0)) s_big = 1;
   }
   __syncthreads();
-  if (s_hi[0] < 0) return;  // no charged atom in this CTA (uniform)
   const int lo0 = s_lo[0], lo1 = s_lo[1], lo2 = s_lo[2];
   const int ex = s_hi[0] - lo0 + 5, ey = s_hi[1] - lo1 + 5, ez = s_hi[2] - lo2 + 5;
-  const long long n_cells = s_big ? (long long)kSpreadCells + 1 : (long long)ex * ey * ez;
+  const bool any = s_hi[0] >= 0;
+  const long long n_cells = any ? (long long)ex * ey * ez : 0;
   Real w[3][5], dw[3][5];
   if (ok) {
 #pragma unroll
@@ -158,8 +165,7 @@ __global__ void __launch_bounds__(2 * kSpreadAtoms) spread_staged_kernel(const P
   const Real q = (Real)qd;
   const Real gscale = Real(kGridScale);
   const int ix0 = half == 0 ? 0 : 3, ix1 = half == 0 ? 3 : 5;
-  if (n_cells > kSpreadCells) {  // direct spreading (uniform branch)
-    if (!ok) return;
+  if (big || (staged && n_cells > kSpreadCells)) {  // direct spreading
     for (int ix = ix0; ix < ix1; ++ix) {
       int gx = base[0] + ix;
       gx -= gx >= a.nx ? a.nx : 0;
@@ -173,19 +179,26 @@ __global__ void __launch_bounds__(2 * kSpreadAtoms) spread_staged_kernel(const P
         for (int iz = 0; iz < 5; ++iz) {
           int gz = base[2] + iz;
           gz -= gz >= a.nz ? a.nz : 0;
-          add_fixed(row + gz, to_fixed(qxy * w[2][iz], gscale));
+          // rounded as the particle's staged contributions are, whatever CTA it is in, so the
+          // grid does not depend on the visiting order
+          long long v;
+          if (sizeof(Real) == 4 && !big)
+            v = (long long)__float2int_rn((float)(qxy * w[2][iz]) * kSpreadScale32) * kSpreadWiden32;
+          else
+            v = to_fixed(qxy * w[2][iz], gscale);
+          add_fixed(row + gz, v);
         }
       }
     }
-    return;
   }
+  if (!any || n_cells > kSpreadCells) return;  // uniform
   const int nc = (int)n_cells;
   for (int c = tid; c < nc; c += 2 * kSpreadAtoms) {
     c_hi[c] = 0;
     if constexpr (sizeof(Real) == 8) c_lo[c] = 0u;
   }
   __syncthreads();
-  if (ok) {
+  if (staged) {
     for (int ix = ix0; ix < ix1; ++ix) {
       const Real qx = q * w[0][ix];
       for (int iy = 0; iy < 5; ++iy) {
@@ -315,8 +328,7 @@ template <class Real>
 __global__ void gather_kernel(const PmeArgs<Real> a) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int s = t >> 3, k = t & 7;
-  int atom = -1;
-  if (s < a.n_order) atom = a.order ? a.order[s] : s;
+  const int atom = ordered_atom(a, s);
   const double qd = atom >= 0 ? a.charge[atom] : 0.0;
   int base[3] = {0, 0, 0};
   Real frac[3] = {Real(0), Real(0), Real(0)};

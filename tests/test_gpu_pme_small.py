@@ -40,9 +40,10 @@ def system(n, q, box, grid, exceptions=()):
     return s
 
 
-def check(n, box, grid, precision, **options):
+def check(n, box, grid, precision, scale=1.0, **options):
     box = np.asarray(box)
     pos, q = ions(n, box, seed=n + grid[0])
+    q = scale * q
     ctx = ommb200.Context(system(n, q, box, grid), systems.langevin(seed=3), precision=precision,
                           **options)
     ctx.set_positions(pos)
@@ -77,6 +78,15 @@ def test_cluster_sizes(n, grid, precision):
     # the last two particle counts are past the cluster form's; 17 planes over 16 CTAs leave some
     # CTAs without planes
     check(n, (2.6, 2.4, 2.5), grid, precision)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+@pytest.mark.parametrize("scale", [2.5, 30.0])
+@pytest.mark.parametrize("bricks", [-1, 0])
+def test_charges_on_both_sides_of_the_staged_limits(precision, scale, bricks):
+    # |q| from 0.5 to 2.5 e and from 6 to 30 e: the staged spread takes those below 2 e (FP32) or
+    # 16 e (FP64), the others go to the grid one by one
+    check(300, (1.9, 1.9, 1.9), (20, 21, 22), precision, scale=scale, pme_bricks=bricks)
 
 
 def test_charges_beyond_the_shared_sums_take_the_launch_chain():

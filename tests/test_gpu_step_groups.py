@@ -17,6 +17,10 @@ def _water(**kw):
     return ctx
 
 
+def _water_chain(**kw):  # the reciprocal part as a launch chain, beside the rebuilds
+    return _water(pme_bricks=0, **kw)
+
+
 def _chain(**kw):
     ch = synth.chain(150, seed=2)
     ctx = ommb200.Context(systems.chain_system(ch), systems.langevin(seed=5, step_size=0.001), **kw)
@@ -24,7 +28,7 @@ def _chain(**kw):
     return ctx
 
 
-@pytest.mark.parametrize("make", [_water, _chain])
+@pytest.mark.parametrize("make", [_water, _water_chain, _chain])
 @pytest.mark.parametrize("calls", [[47], [20, 20, 7], [1] * 47, [19, 21, 7], [46, 1], [3, 40, 4]])
 def test_step_groups_give_one_trajectory(make, calls):
     res = []

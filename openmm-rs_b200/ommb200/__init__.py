@@ -664,9 +664,9 @@ class Context:
         flags = ((STATE_POSITIONS if positions else 0) | (STATE_VELOCITIES if velocities else 0) |
                  (STATE_FORCES if forces else 0) | (STATE_ENERGY if energy else 0) |
                  (STATE_VIRIAL if virial else 0))
-        p = np.zeros((self._n, 3)) if positions else None
-        v = np.zeros((self._n, 3)) if velocities else None
-        f = np.zeros((self._n, 3)) if forces else None
+        p = np.empty((self._n, 3)) if positions else None  # filled by the call
+        v = np.empty((self._n, 3)) if velocities else None
+        f = np.empty((self._n, 3)) if forces else None
         info = StateInfo()
         null = C.POINTER(C.c_double)()
         _check(library().ommb200_context_get_state(

@@ -57,14 +57,12 @@ __device__ __forceinline__ bool stencil(const PmeArgs<Real>& a, int atom, int ba
     const double coord = (f - floor(f)) * (double)dims[d];
     ok = ok && coord >= 0.0 && coord <= (double)dims[d];
     const double fl = ok ? floor(coord) : 0.0;
-    int b = (int)fl;
-    b %= dims[d];
-    base[d] = b;
+    const int b = (int)fl;
+    base[d] = (unsigned)b < (unsigned)dims[d] ? b : 0;  // fl may round up to dims
     frac[d] = (Real)(ok ? coord - fl : 0.0);
   }
   return ok;
 }
-
 // The particle in place s of the visiting order (which of its two copies is the same for every
 // thread of the launch: nothing beside it writes the parity), -1 for padding.
 template <class Real>
@@ -73,7 +71,6 @@ __device__ __forceinline__ int ordered_atom(const PmeArgs<Real>& a, int s) {
   if (!a.order) return s;
   return a.order[a.order_parity ? (size_t)*a.order_parity * a.n_order + s : s];
 }
-
 template <class Real>
 __global__ void spread_kernel(const PmeArgs<Real> a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -761,29 +758,33 @@ __global__ void __launch_bounds__(kPlaneThreads) planes_inverse(const PmeArgs<Re
 // the influence function, reading and writing the owners' planes through distributed shared
 // memory, transforms its planes back and gathers their part of every particle's force.  Two
 // cluster barriers (around the x pass) replace four kernel boundaries.  Each particle's force
-// is the fixed-point sum of its planes' parts.  1,524 particles on a 23^3 grid: the chain's step
-// took 55 us, with this form 46 us.
+// is the fixed-point sum of its planes' parts.  1,524 particles on a 23^3 grid: a step with the
+// chain's launches takes 55 us, with this form 42 (46 when each thread walked its particles'
+// whole stencils, spread and gather, instead of a list).
 template <class Real>
 struct ClusterLayout {  // element counts; every CTA of the cluster has the same
   int planes, pencils;  // planes and x pencils per CTA
   size_t plane_elems;   // of each of the two plane buffers
-  __host__ __device__ ClusterLayout(int nx, int ny, int nz, int ctas)
+  int list;             // capacity of the particle list
+  __host__ __device__ ClusterLayout(int nx, int ny, int nz, int ctas, int list_capacity)
       : planes((nx + ctas - 1) / ctas), pencils((ny * (nz / 2 + 1) + ctas - 1) / ctas),
-        plane_elems((size_t)planes * fft_plane_elems(ny, nz)) {}
+        plane_elems((size_t)planes * fft_plane_elems(ny, nz)), list(list_capacity) {}
   __host__ __device__ size_t bytes(int nx, int ny, int nz) const {
     return 2 * sizeof(Real) * ((size_t)nx + ny + nz + 2 * plane_elems + 2 * (size_t)pencils * nx) +
+           (sizeof(double) + 30 * sizeof(Real) + 4 * sizeof(int)) * (size_t)list +
            2 * sizeof(int) * (size_t)planes * ny * nz;
   }
 };
 
 template <class Real, int kTerms>
-__global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Real> a, const PmeFft f) {
+__global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Real> a, const PmeFft f,
+                                                               int list_capacity) {
   using C2 = typename Cplx<Real>::T;
   extern __shared__ __align__(16) unsigned char fsm[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ctas = gridDim.x, rank = blockIdx.x;  // one cluster
   const int nx = a.nx, ny = a.ny, nz = a.nz, nzh = nz / 2 + 1, nyp = (ny + 1) / 2;
-  const ClusterLayout<Real> L(nx, ny, nz, ctas);
+  const ClusterLayout<Real> L(nx, ny, nz, ctas, list_capacity);
   C2* twx = reinterpret_cast<C2*>(fsm);
   C2* twy = twx + nx;
   C2* twz = twy + ny;
@@ -791,7 +792,11 @@ __global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Rea
   C2* B = A + L.plane_elems;
   C2* XA = B + L.plane_elems;
   C2* XB = XA + (size_t)L.pencils * nx;
-  int* c_hi = reinterpret_cast<int*>(XB + (size_t)L.pencils * nx);
+  double* l_q = reinterpret_cast<double*>(XB + (size_t)L.pencils * nx);  // the particle list:
+  Real* l_w = reinterpret_cast<Real*>(l_q + L.list);          // [30][list] weights, then slopes
+  int* l_base = reinterpret_cast<int*>(l_w + 30 * (size_t)L.list);  // [3][list]
+  int* l_at = l_base + 3 * (size_t)L.list;
+  int* c_hi = l_at + L.list;
   unsigned* c_lo = reinterpret_cast<unsigned*>(c_hi + (size_t)L.planes * ny * nz);
   const int x0 = rank * L.planes, np = max(0, min(L.planes, nx - x0));  // own planes
   load_twiddles(twx, f.tw[0], nx);
@@ -802,47 +807,102 @@ __global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Rea
     c_lo[c] = 0u;
   }
   __syncthreads();
-  // spread (pme.rs:176-238)
-  const Real gscale = Real(kGridScale);
-  for (int i = threadIdx.x; i < a.n_atoms; i += blockDim.x) {
-    const double qd = a.charge[i];
-    int base[3];
-    Real frac[3], w[3][5], dw[3][5];
-    if (qd == 0.0 || !stencil(a, i, base, frac)) continue;
-    bool mine = false;
+  // The particles whose stencils touch this CTA's planes (a quarter of them at 23 planes over 16
+  // CTAs) are listed with their spline weights, kClusterThreads particles at a time: each thread
+  // forms one stencil, and the work on those that count spreads evenly over every thread.  The
+  // order of the list does not matter: the grid's and the forces' sums are fixed point.  A list
+  // that holds every particle of this CTA is kept for the gather.
+  __shared__ int s_n;
+  auto weight = [&](int d, int k, int e) -> Real& { return l_w[(5 * d + k) * L.list + e]; };
+  auto slope = [&](int d, int k, int e) -> Real& { return l_w[(15 + 5 * d + k) * L.list + e]; };
+  bool whole = false;  // the list holds all of this CTA's particles
+  auto for_each_list = [&](auto use) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    int lists = 0;
+    for (int i0 = 0; i0 < a.n_atoms; i0 += kClusterThreads) {
+      const int i = i0 + threadIdx.x;
+      const double q = i < a.n_atoms ? a.charge[i] : 0.0;
+      int base[3] = {0, 0, 0};
+      Real frac[3] = {Real(0), Real(0), Real(0)};
+      bool mine = q != 0.0 && stencil(a, i, base, frac);
+      if (mine) {  // planes base .. base + 4, cyclic, against x0 .. x0 + np - 1
+        int first = x0 - base[0];
+        first += first < 0 ? nx : 0;  // distance from the base to the first own plane
+        mine = np > 0 && (first < 5 || first + np > nx);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, mine);
+      int at = 0;
+      if (lane == 0 && m) at = atomicAdd(&s_n, __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+      if (mine) {
+        l_at[at] = i;
+        l_q[at] = q;
+        for (int d = 0; d < 3; ++d) l_base[d * L.list + at] = base[d];
 #pragma unroll
-    for (int ix = 0; ix < 5; ++ix) {
-      int gx = base[0] + ix;
-      gx -= gx >= nx ? nx : 0;
-      mine = mine || (gx >= x0 && gx < x0 + np);
-    }
-    if (!mine) continue;
+        for (int d = 0; d < 3; ++d) {
+          Real w[5], dw[5];
+          spline5(frac[d], w, dw);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) spline5(frac[d], w[d], dw[d]);
-    const Real q = (Real)qd;
-#pragma unroll
-    for (int ix = 0; ix < 5; ++ix) {
-      int gx = base[0] + ix;
-      gx -= gx >= nx ? nx : 0;
-      if (gx < x0 || gx >= x0 + np) continue;
-      const Real qx = q * w[0][ix];
-      for (int iy = 0; iy < 5; ++iy) {
-        int gy = base[1] + iy;
-        gy -= gy >= ny ? ny : 0;
-        const Real qxy = qx * w[1][iy];
-        const int row = ((gx - x0) * ny + gy) * nz;
-#pragma unroll
-        for (int iz = 0; iz < 5; ++iz) {
-          int gz = base[2] + iz;
-          gz -= gz >= nz ? nz : 0;
-          const long long v = to_fixed(qxy * w[2][iz], gscale);
-          atomicAdd(&c_hi[row + gz], (int)(v >> 20));
-          atomicAdd(&c_lo[row + gz], (unsigned)(v & 0xFFFFF));
+          for (int k = 0; k < 5; ++k) {
+            weight(d, k, at) = w[k];
+            slope(d, k, at) = dw[k];
+          }
+        }
+      }
+      __syncthreads();
+      const int n = s_n;
+      __syncthreads();  // every thread has read the count before the next particles add to it
+      const bool last = i0 + kClusterThreads >= a.n_atoms;
+      if (last || n > L.list - kClusterThreads) {
+        use(n);
+        ++lists;
+        __syncthreads();
+        if (!last) {
+          if (threadIdx.x == 0) s_n = 0;
+          __syncthreads();
         }
       }
     }
-  }
-  __syncthreads();
+    whole = lists == 1;
+  };
+  // own plane p of a particle with base plane b: the stencil plane it is, or >= 5
+  auto stencil_plane = [&](int b, int p) {
+    const int ix = x0 + p - b;
+    return ix < 0 ? ix + nx : ix;
+  };
+  // spread (pme.rs:176-238): a thread takes one row in y of one own plane of a particle
+  for_each_list([&](int n) {
+    for (int t = threadIdx.x; t < 5 * np * n; t += blockDim.x) {
+      const int e = t / (5 * np), r = t - e * 5 * np, p = r / 5, iy = r - 5 * p;
+      const int ix = stencil_plane(l_base[e], p);
+      if (ix >= 5) continue;
+      int gy = l_base[L.list + e] + iy;
+      gy -= gy >= ny ? ny : 0;
+      const int bz = l_base[2 * L.list + e], row = (p * ny + gy) * nz;
+      const Real qxy = (Real)l_q[e] * weight(0, ix, e) * weight(1, iy, e);
+#pragma unroll
+      for (int iz = 0; iz < 5; ++iz) {
+        int gz = bz + iz;
+        gz -= gz >= nz ? nz : 0;
+        const Real v = qxy * weight(2, iz, e);
+        int hi;
+        unsigned lo;
+        if constexpr (sizeof(Real) == 4) {  // v 2^40 to an integer, in 32-bit steps
+          const float scaled = v * 1048576.f, whole_part = floorf(scaled);
+          hi = (int)whole_part;
+          lo = (unsigned)__float2int_rn((scaled - whole_part) * 1048576.f);
+        } else {
+          const long long f = to_fixed(v, Real(kGridScale));
+          hi = (int)(f >> 20);
+          lo = (unsigned)(f & 0xFFFFF);
+        }
+        atomicAdd(&c_hi[row + gz], hi);
+        atomicAdd(&c_lo[row + gz], lo);
+      }
+    }
+  });
   // rows y = 2 yp (real part) and 2 yp + 1 (imaginary part) as one complex row, z transform
   for (int i = threadIdx.x; i < np * nyp * nz; i += blockDim.x) {
     const int z = i % nz, r = i / nz, lp = r / nyp, yp = r - lp * nyp;
@@ -931,53 +991,57 @@ __global__ void __launch_bounds__(kClusterThreads) pme_cluster(const PmeArgs<Rea
   }
   __syncthreads();
   const C2* pot = stockham(g, h, twz, f, 2, nz, np * nyp);  // row 2 yp = Re, row 2 yp + 1 = -Im
-  // gather (pme.rs:377-425): this CTA's planes' part of every particle's force
-  for (int i = threadIdx.x; i < a.n_atoms; i += blockDim.x) {
-    const double qd = a.charge[i];
-    int base[3];
-    Real frac[3], w[3][5], dw[3][5];
-    if (qd == 0.0 || !stencil(a, i, base, frac)) continue;
-    bool mine = false;
-#pragma unroll
-    for (int ix = 0; ix < 5; ++ix) {
-      int gx = base[0] + ix;
-      gx -= gx >= nx ? nx : 0;
-      mine = mine || (gx >= x0 && gx < x0 + np);
-    }
-    if (!mine) continue;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) spline5(frac[d], w[d], dw[d]);
-    Real g0 = 0, g1 = 0, g2 = 0;
-#pragma unroll
-    for (int ix = 0; ix < 5; ++ix) {
-      int gx = base[0] + ix;
-      gx -= gx >= nx ? nx : 0;
-      if (gx < x0 || gx >= x0 + np) continue;
-      for (int iy = 0; iy < 5; ++iy) {
-        int gy = base[1] + iy;
+  // gather (pme.rs:377-425): this CTA's planes' part of each listed particle's force, eight lanes
+  // to a particle, five of them with a row in y each
+  auto gather = [&](int n) {
+    const int k = threadIdx.x & 7;
+    for (int e0 = 0; e0 < n; e0 += kClusterThreads / 8) {
+      const int e = e0 + (threadIdx.x >> 3);
+      Real g0 = 0, g1 = 0, g2 = 0;
+      if (e < n && k < 5) {
+        int gy = l_base[L.list + e] + k;
         gy -= gy >= ny ? ny : 0;
-        const C2* row = pot + ((gx - x0) * nyp + (gy >> 1)) * nz;
-        Real sum = 0, dsum = 0;
+        const int bx = l_base[e], bz = l_base[2 * L.list + e];
+        for (int p = 0; p < np; ++p) {
+          const int ix = stencil_plane(bx, p);
+          if (ix >= 5) continue;
+          const C2* row = pot + (p * nyp + (gy >> 1)) * nz;
+          Real sum = 0, dsum = 0;
 #pragma unroll
-        for (int iz = 0; iz < 5; ++iz) {
-          int gz = base[2] + iz;
-          gz -= gz >= nz ? nz : 0;
-          const C2 v = row[gz];
-          const Real phi = (gy & 1) ? -v.y : v.x;
-          sum += phi * w[2][iz];
-          dsum += phi * dw[2][iz];
+          for (int iz = 0; iz < 5; ++iz) {
+            int gz = bz + iz;
+            gz -= gz >= nz ? nz : 0;
+            const C2 v = row[gz];
+            const Real phi = (gy & 1) ? -v.y : v.x;
+            sum += phi * weight(2, iz, e);
+            dsum += phi * slope(2, iz, e);
+          }
+          g0 += slope(0, ix, e) * sum;
+          g1 += weight(0, ix, e) * sum;
+          g2 += weight(0, ix, e) * dsum;
         }
-        g0 += dw[0][ix] * w[1][iy] * sum;
-        g1 += w[0][ix] * dw[1][iy] * sum;
-        g2 += w[0][ix] * w[1][iy] * dsum;
+        g0 *= weight(1, k, e);
+        g1 *= slope(1, k, e);
+        g2 *= weight(1, k, e);
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        g0 += __shfl_xor_sync(0xffffffffu, g0, o, 8);
+        g1 += __shfl_xor_sync(0xffffffffu, g1, o, 8);
+        g2 += __shfl_xor_sync(0xffffffffu, g2, o, 8);
+      }
+      if (e < n && k < 3) {  // one component per lane
+        const double gd[3] = {(double)g0 * nx, (double)g1 * ny, (double)g2 * nz};
+        const double fc =
+            -l_q[e] * (gd[0] * a.recip[0][k] + gd[1] * a.recip[1][k] + gd[2] * a.recip[2][k]);
+        add_fixed(a.force + (long long)k * a.n_atoms + l_at[e], to_fixed(fc, kForceScale));
       }
     }
-    const double gd[3] = {(double)g0 * nx, (double)g1 * ny, (double)g2 * nz};
-    for (int c = 0; c < 3; ++c) {
-      const double fc = -qd * (gd[0] * a.recip[0][c] + gd[1] * a.recip[1][c] + gd[2] * a.recip[2][c]);
-      add_fixed(a.force + (long long)c * a.n_atoms + i, to_fixed(fc, kForceScale));
-    }
-  }
+  };
+  if (whole)
+    gather(s_n);
+  else
+    for_each_list(gather);
 }
 
 }  // namespace
@@ -1013,6 +1077,14 @@ void prepare_pme_transform(const PmeArgs<Real>& a, const PmeFft& f) {
   cudaFuncSetAttribute((const void*)x_convolve<Real, kTermsNone>, cudaFuncAttributeMaxDynamicSharedMemorySize, sx);
 }
 
+// Capacity of the cluster form's particle lists: two batches, or one where shared memory is short.
+constexpr size_t kClusterSmem = 200 * 1024;
+template <class Real>
+int cluster_list(const PmeArgs<Real>& a, int ctas) {
+  const ClusterLayout<Real> two(a.nx, a.ny, a.nz, ctas, 2 * kClusterThreads);
+  return two.bytes(a.nx, a.ny, a.nz) <= kClusterSmem ? 2 * kClusterThreads : kClusterThreads;
+}
+
 // The cluster form's launch: `ctas` CTAs of one cluster.
 template <class Real, int kTerms>
 cudaLaunchConfig_t cluster_config(const PmeArgs<Real>& a, int ctas, cudaLaunchAttribute* attr,
@@ -1020,7 +1092,8 @@ cudaLaunchConfig_t cluster_config(const PmeArgs<Real>& a, int ctas, cudaLaunchAt
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kClusterThreads);
-  cfg.dynamicSmemBytes = ClusterLayout<Real>(a.nx, a.ny, a.nz, ctas).bytes(a.nx, a.ny, a.nz);
+  cfg.dynamicSmemBytes =
+      ClusterLayout<Real>(a.nx, a.ny, a.nz, ctas, cluster_list(a, ctas)).bytes(a.nx, a.ny, a.nz);
   cfg.stream = s;
   attr->id = cudaLaunchAttributeClusterDimension;
   attr->val.clusterDim.x = ctas;
@@ -1034,7 +1107,7 @@ template <class Real, int kTerms>
 bool prepare_cluster(const PmeArgs<Real>& a, int ctas) {
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = cluster_config<Real, kTerms>(a, ctas, &attr, nullptr);
-  if (cfg.dynamicSmemBytes > 200 * 1024) return false;
+  if (cfg.dynamicSmemBytes > kClusterSmem) return false;
   auto* fn = pme_cluster<Real, kTerms>;
   if (cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)cfg.dynamicSmemBytes) != cudaSuccess ||
@@ -1062,7 +1135,7 @@ template <class Real, int kTerms>
 void launch_cluster(const PmeArgs<Real>& a, const PmeFft& f, int ctas, cudaStream_t s) {
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = cluster_config<Real, kTerms>(a, ctas, &attr, s);
-  cudaLaunchKernelEx(&cfg, pme_cluster<Real, kTerms>, a, f);
+  cudaLaunchKernelEx(&cfg, pme_cluster<Real, kTerms>, a, f, cluster_list(a, ctas));
 }
 
 template <class Real>

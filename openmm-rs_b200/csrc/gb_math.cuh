@@ -54,14 +54,10 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 
 // FP32 forms with SFU reciprocals and logarithm; inv_r = 1 / r.  The integral and its gradient
-// together, and each alone (the compiler drops what a caller does not use).
+// together, and each alone (the compiler drops what a caller does not use).  The case without
+// overlap is selected, not branched to, so that several calls run side by side.
 __device__ __forceinline__ void descreening_fast(float radius, float scaled, float r, float inv_r,
                                                  float* h, float* grad) {
-  if (radius >= r + scaled) {
-    *h = 0.f;
-    *grad = 0.f;
-    return;
-  }
   const float lo_den = fmaxf(radius, fabsf(r - scaled));
   const float lower = rcp_approx(lo_den), upper = rcp_approx(r + scaled);
   const float l2u2 = lower * lower - upper * upper;
@@ -69,9 +65,11 @@ __device__ __forceinline__ void descreening_fast(float radius, float scaled, flo
   float v = lower - upper - 0.25f * r * l2u2 + 0.5f * inv_r * lg +
             0.25f * scaled * scaled * inv_r * l2u2;
   if (radius < scaled - r) v += 2.f * (rcp_approx(radius) - lower);
-  *h = v;
-  *grad = (0.125f * (1.f + scaled * scaled * inv_r * inv_r) * l2u2 + 0.25f * lg * inv_r * inv_r) *
-          inv_r;
+  const float g =
+      (0.125f * (1.f + scaled * scaled * inv_r * inv_r) * l2u2 + 0.25f * lg * inv_r * inv_r) * inv_r;
+  const bool inside = radius >= r + scaled;
+  *h = inside ? 0.f : v;
+  *grad = inside ? 0.f : g;
 }
 __device__ __forceinline__ float descreening_fast(float radius, float scaled, float r,
                                                   float inv_r) {

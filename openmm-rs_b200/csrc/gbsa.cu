@@ -504,8 +504,11 @@ __device__ __forceinline__ float2 far_gradient(float2 t) {
 // that is a few per cent of the pairs, in few tiles.  Bound by the FP32 pipe.  The general
 // expressions for every pair, one pair per lane (7 SFU operations and about 100 FP32 instructions
 // for both directions), took 114 us (pass 1) and 118 us (pass 3) on 48 chains of 200 to 2,000
-// particles (35.6 M pairs); this form takes 68 and 81 us, and the forces' error against 64 bits
-// falls too (4,999-particle chain, 2 nm cutoff: 1.8e-6 to 1.4e-6).
+// particles (35.6 M pairs); this form takes 62 and 75 us, and the forces' error against 64 bits
+// falls too (4,999-particle chain, 2 nm cutoff: 1.8e-6 to 1.4e-6).  A step with a near pair runs
+// the general expressions of both pairs and directions side by side and selects: one dependent
+// chain of SFU calls instead of up to four in turn (603-particle chain, where they are the whole
+// latency: 31 us per step against 28).
 template <int kPass, bool kCutoff>
 __global__ void __launch_bounds__(128) gb_descreen_x2(const GbArgs a) {
   if (a.use_learned && *a.use_learned) return;  // the network replaces them
@@ -585,15 +588,14 @@ __global__ void __launch_bounds__(128) gb_descreen_x2(const GbArgs a) {
       if (kPass == 1) {
         float2 hi = x2::mul(x2::mul(uu, x2::bc(qj.w)), far_integral(ti));  // adds to I_i
         float2 hj = x2::mul(x2::mul(uu, s3i), far_integral(tj));           // adds to I_j
-        if (near1) {
-          const float inv = rsqrt_r(r2.x), r = r2.x * inv;
-          hi.x = descreening_fast(q1.x, qj.y, r, inv);
-          hj.x = descreening_fast(qj.x, q1.y, r, inv);
-        }
-        if (near_2) {
-          const float inv = rsqrt_r(r2.y), r = r2.y * inv;
-          hi.y = descreening_fast(q2.x, qj.y, r, inv);
-          hj.y = descreening_fast(qj.x, q2.y, r, inv);
+        if (near1 || near_2) {
+          const float2 inv = x2::rsqrt_approx(r2), r = x2::mul(r2, inv);
+          const float i1h = descreening_fast(q1.x, qj.y, r.x, inv.x);
+          const float i2h = descreening_fast(q2.x, qj.y, r.y, inv.y);
+          const float j1h = descreening_fast(qj.x, q1.y, r.x, inv.x);
+          const float j2h = descreening_fast(qj.x, q2.y, r.y, inv.y);
+          hi = make_float2(near1 ? i1h : hi.x, near_2 ? i2h : hi.y);
+          hj = make_float2(near1 ? j1h : hj.x, near_2 ? j2h : hj.y);
         }
         acc_i = x2::add(acc_i, x2::select(u1, u2, hi, 0.f));
         if (!self) {
@@ -605,15 +607,13 @@ __global__ void __launch_bounds__(128) gb_descreen_x2(const GbArgs a) {
         // minus the radial force: D_i g(rho_i, s_j) + D_j g(rho_j, s_i)
         float2 fo = x2::mul(x2::mul(x2::mul(di, x2::bc(qj.w)), far_gradient(ti)), uu);
         fo = x2::mul(x2::fma(x2::mul(x2::mul(s3i, x2::bc(dj)), far_gradient(tj)), uu, fo), u);
-        if (near1) {
-          const float inv = rsqrt_r(r2.x), r = r2.x * inv;
-          fo.x = di.x * descreening_gradient_fast(q1.x, qj.y, r, inv) +
-                 dj * descreening_gradient_fast(qj.x, q1.y, r, inv);
-        }
-        if (near_2) {
-          const float inv = rsqrt_r(r2.y), r = r2.y * inv;
-          fo.y = di.y * descreening_gradient_fast(q2.x, qj.y, r, inv) +
-                 dj * descreening_gradient_fast(qj.x, q2.y, r, inv);
+        if (near1 || near_2) {
+          const float2 inv = x2::rsqrt_approx(r2), r = x2::mul(r2, inv);
+          const float f1 = di.x * descreening_gradient_fast(q1.x, qj.y, r.x, inv.x) +
+                           dj * descreening_gradient_fast(qj.x, q1.y, r.x, inv.x);
+          const float f2 = di.y * descreening_gradient_fast(q2.x, qj.y, r.y, inv.y) +
+                           dj * descreening_gradient_fast(qj.x, q2.y, r.y, inv.y);
+          fo = make_float2(near1 ? f1 : fo.x, near_2 ? f2 : fo.y);
         }
         fo = x2::select(u1, u2, fo, 0.f);
         const float2 gx = x2::mul(fo, dx), gy = x2::mul(fo, dy), gz = x2::mul(fo, dz);

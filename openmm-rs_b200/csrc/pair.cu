@@ -191,21 +191,166 @@ __global__ void __launch_bounds__(32 * kPairWarps) pair_kernel(const PairArgs<Re
   if (kTerms && !a.block_segment) commit_cta<kTerms>(a.energy, e_fixed, w_fixed);
 }
 
-// The FP32 form with two i-particles per lane and packed (f32x2) arithmetic.  The warp splits
-// into groups of G lanes (G = 8 for halves tiles, 16 otherwise); a group owns G consecutive
-// entries and the 2G i-slots that meet them, lane m of the group holding i-slots m and m + G
-// of its half (halves) or of the block.  In G steps the lane meets each of the group's entries
-// once, evaluating the pairs with both of its i-particles in the two lanes of the packed
-// values; the entry's force (both pairs summed) rotates one lane per step within the group and
-// is back at the entry's own lane after G steps.  Every i-slot is met by two groups, whose
-// partial forces are summed at the end (lane ^ G), so each lane commits the i-slot equal to
-// its lane index and the entry it loaded.  A warp evaluates 64 pair slots per step, against 32
-// in the one-particle-per-lane form, with half the shuffles and shared-memory reads per pair.
-// Entry data sit in shared memory already duplicated into both lanes of each packed value, so
-// a step moves no register.  The cutoff (and with it the exact decision band) applies to the
-// Ewald and reaction-field forms; the bare-Coulomb form is the no-cutoff method.
-template <int kElec, int kTerms, bool kDump, bool kSwitch>
-__global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairArgs<float> a) {
+// The 2 P i-particles of a lane, packed two by two, and their forces.
+template <int P>
+struct ISlots {
+  float2 npx[P], npy[P], npz[P], q[P], sg[P], ep[P];  // negated positions
+};
+template <int P>
+struct IForces {
+  float2 x[P], y[P], z[P];
+};
+template <int P>
+__device__ __forceinline__ ISlots<P> load_slots(const float4* pos, const float2* lj, int stride) {
+  ISlots<P> v;
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    const float4 p1 = pos[2 * s * stride], p2 = pos[(2 * s + 1) * stride];
+    const float2 l1 = lj[2 * s * stride], l2 = lj[(2 * s + 1) * stride];
+    v.npx[s] = make_float2(-p1.x, -p2.x);
+    v.npy[s] = make_float2(-p1.y, -p2.y);
+    v.npz[s] = make_float2(-p1.z, -p2.z);
+    v.q[s] = make_float2(p1.w, p2.w);
+    v.sg[s] = make_float2(l1.x, l2.x);
+    v.ep[s] = make_float2(l1.y, l2.y);
+  }
+  return v;
+}
+
+// The sums over the 2 P groups of G lanes that met the same i-slots: the lane of group c keeps
+// i-slot c of its 2 P.  The order of the additions is fixed.
+template <int P>
+__device__ __forceinline__ float3 reduce_groups(const IForces<P>& f, int lane, int G) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const bool hi = (lane & (2 * G)) != 0, odd = (lane & G) != 0;
+  auto sum = [&](const float2(&v)[P]) {
+    float2 t = v[0];
+    if constexpr (P == 2) {
+      const float2 keep = hi ? v[1] : v[0], give = hi ? v[0] : v[1];
+      t = x2::add(keep, make_float2(__shfl_xor_sync(FULL, give.x, 2 * G),
+                                    __shfl_xor_sync(FULL, give.y, 2 * G)));
+    }
+    return (odd ? t.y : t.x) + __shfl_xor_sync(FULL, odd ? t.x : t.y, G);
+  };
+  return make_float3(sum(f.x), sum(f.y), sum(f.z));
+}
+
+// One entry (its values duplicated into both lanes of each packed value, so a step moves no
+// register) against the lane's i-particles: adds to their forces, the entry's force and the sums.
+// Bit c * shift of `excluded` drops the pair with i-particle c, whose number is iatom[c * stride].
+template <int P, int kElec, int kTerms, bool kDump, bool kSwitch, bool kCutoff>
+__device__ __forceinline__ void pair_step(const PairArgs<float>& a, const float4 jxy, const float4 jzq,
+                                          const float4 jse, uint32_t excluded, int shift, bool image,
+                                          bool self, const int* jatom, const int* iatom, int stride,
+                                          const ISlots<P>& q, IForces<P>& f, float& fjx, float& fjy,
+                                          float& fjz, double& e_acc, double (&w_acc)[6]) {
+  float2 dx[P], dy[P], dz[P], r2[P];
+  bool u[2 * P];
+#pragma unroll
+  for (int t = 0; t < 2 * P; ++t) u[t] = ((excluded >> (t * shift)) & 1u) == 0u;
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    dx[s] = x2::add(make_float2(jxy.x, jxy.y), q.npx[s]);
+    dy[s] = x2::add(make_float2(jxy.z, jxy.w), q.npy[s]);
+    dz[s] = x2::add(make_float2(jzq.x, jzq.y), q.npz[s]);
+    if (image) {
+      min_image_fast(dx[s].x, dy[s].x, dz[s].x, a.box);
+      min_image_fast(dx[s].y, dy[s].y, dz[s].y, a.box);
+    }
+    r2[s] = x2::fma(dz[s], dz[s], x2::fma(dy[s], dy[s], x2::mul(dx[s], dx[s])));
+  }
+  if (kCutoff) {
+    const float lo = a.cutoff2 - a.band, hi = a.cutoff2 + a.band;
+    bool near_cutoff = false, c[2 * P];
+#pragma unroll
+    for (int t = 0; t < 2 * P; ++t) {
+      const float r = (t & 1) ? r2[t >> 1].y : r2[t >> 1].x;
+      u[t] = u[t] && r < hi;
+      c[t] = u[t] && r >= lo;
+      near_cutoff = near_cutoff || c[t];
+    }
+    if (near_cutoff) {  // within the band: the reference's decision from the f64 positions
+      const int b = *jatom;
+#pragma unroll
+      for (int t = 0; t < 2 * P; ++t)
+        if (c[t]) {
+          const int ia = iatom[t * stride];
+          u[t] = ia >= 0 && b >= 0 &&
+                 exact_inside(a.pos, ia, b, a.periodic, a.box_exact, a.cutoff2_exact);
+        }
+    }
+  }
+  if (kDump) {
+    const int b = *jatom;
+    for (int t = 0; t < 2 * P; ++t) {
+      const int ia = iatom[t * stride];
+      if (u[t] && ia >= 0 && b >= 0 && (!self || ia < b)) {
+        const unsigned long long slot = atomicAdd(a.pair_count, 1ull);
+        if ((long long)slot < a.pair_capacity) {
+          a.pair_dump[2 * slot] = ia < b ? ia : b;
+          a.pair_dump[2 * slot + 1] = ia < b ? b : ia;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < P; ++s) {
+    const bool u1 = u[2 * s], u2 = u[2 * s + 1];
+    float2 fo, en;
+    pair_terms_x2<kElec, kTerms, kSwitch>(
+        a, x2::select(u1, u2, r2[s], 1.f), x2::mul(make_float2(jzq.z, jzq.w), q.q[s]),
+        x2::add(make_float2(jse.x, jse.y), q.sg[s]), x2::mul(make_float2(jse.z, jse.w), q.ep[s]), fo, en);
+    fo = x2::select(u1, u2, fo, 0.f);
+    f.x[s] = x2::fma(fo, dx[s], f.x[s]);
+    f.y[s] = x2::fma(fo, dy[s], f.y[s]);
+    f.z[s] = x2::fma(fo, dz[s], f.z[s]);
+    if (kTerms) {
+      const double scale = self ? 0.5 : 1.0;
+      if (u1) e_acc += scale * (double)en.x;
+      if (u2) e_acc += scale * (double)en.y;
+      if (kTerms > kTermsEnergy) {
+        const float2 fdx = x2::mul(fo, dx[s]), fdy = x2::mul(fo, dy[s]), fdz = x2::mul(fo, dz[s]);
+        const float2 w[6] = {x2::mul(fdx, dx[s]), x2::mul(fdy, dy[s]), x2::mul(fdz, dz[s]),
+                             x2::mul(fdx, dy[s]), x2::mul(fdx, dz[s]), x2::mul(fdy, dz[s])};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+          if (u1) w_acc[c] -= scale * (double)w[c].x;
+          if (u2) w_acc[c] -= scale * (double)w[c].y;
+        }
+      }
+    }
+    if (!self) {
+      fjx = fmaf(-fo.x, dx[s].x, fjx);
+      fjy = fmaf(-fo.x, dy[s].x, fjy);
+      fjz = fmaf(-fo.x, dz[s].x, fjz);
+      fjx = fmaf(-fo.y, dx[s].y, fjx);
+      fjy = fmaf(-fo.y, dy[s].y, fjy);
+      fjz = fmaf(-fo.y, dz[s].y, fjz);
+    }
+  }
+}
+
+// The FP32 form with 2 P i-particles per lane in packed (f32x2) arithmetic.  The warp splits into
+// groups of G lanes (G = 8 / P for halves tiles, 16 / P otherwise); a group owns G consecutive
+// entries and the i-slots that meet them, lane m of the group holding i-slots m + c G, c < 2 P, of
+// its half (halves) or of the block.  In G steps the lane meets each of the group's entries once,
+// evaluating the pairs with its i-particles two by two in the lanes of packed values; the entry's
+// force (all its pairs summed) rotates one lane per step within the group and is back at the
+// entry's own lane after G steps.  Every i-slot is met by 2 P groups, whose partial forces are
+// summed at the end, so each lane commits the i-slot equal to its lane index and the entry it
+// loaded.  The cutoff (and with it the exact decision band) applies to the Ewald and
+// reaction-field forms; the bare-Coulomb form is the no-cutoff method.
+//
+// The warps of an SM issue two instructions in three cycles; what a step does once for all its
+// pairs (entry reads, force shuffles, constants moved into register pairs, the loop) is a quarter
+// of it with P = 1.  P = 2 halves that share per pair and gives each warp two independent chains,
+// at 120 registers (4 CTAs per SM) against 96 (5): the 23,958-particle box takes 92.5 against
+// 94.3 us per step, 8,217 particles with a barostat 99 against 104.  It serves the periodic lists.
+// Tiles of the whole blocks of non-periodic systems keep P = 1: with a cutoff most of them are
+// skipped, which more warps in flight do faster (4,999 particles: 180 us per evaluation against
+// 182).
+template <int P, int kElec, int kTerms, bool kDump, bool kSwitch>
+__global__ void __launch_bounds__(32 * kPairWarps, P == 2 ? 4 : 5) pair_kernel_x2(const PairArgs<float> a) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr bool kCutoff = kElec != kElecCoulomb;
   __shared__ float4 s_j[kPairWarps][3][32];  // per entry (x, x, y, y), (z, z, q, q), (s, s, e, e)
@@ -261,27 +406,23 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
     s_ilj[w][lane] = li;
     s_iatom[w][lane] = ai;
     __syncwarp();
-    const int G = halves ? 8 : 16, gm = G - 1;
+    const int G = (halves ? 8 : 16) / P, gm = G - 1;
     const int m = lane & gm, eb = lane & ~gm;
-    const int i1 = (halves ? (lane & 16) : 0) + m, i2 = i1 + G;
-    // exclusion/padding bits of the two i-slots in step order: bit k (i1) and bit 16 + k (i2)
-    // stand for entry eb + ((m + k) mod G); a self tile also drops the diagonal
-    uint32_t steps_mask;
-    {
+    const int i0 = (halves ? (lane & 16) : 0) + m;
+    // exclusion/padding bits of the i-slots in step order: bit (16 / P) c + k of i-slot i0 + c G
+    // stands for entry eb + ((m + k) mod G); a self tile also drops the diagonal
+    uint32_t steps_mask = 0u;
+    if (self || (tile.y & kTileHasMask)) {
       const uint32_t gmask = (1u << G) - 1u;
-      const uint32_t x1 = ((__shfl_sync(FULL, excl, i1) | (self ? 1u << i1 : 0u)) >> eb) & gmask;
-      const uint32_t x2v = ((__shfl_sync(FULL, excl, i2) | (self ? 1u << i2 : 0u)) >> eb) & gmask;
-      const uint32_t r1 = ((x1 >> m) | (x1 << (G - m))) & gmask;
-      const uint32_t r2v = ((x2v >> m) | (x2v << (G - m))) & gmask;
-      steps_mask = r1 | (r2v << 16);
+#pragma unroll
+      for (int c = 0; c < 2 * P; ++c) {
+        const int i = i0 + c * G;
+        const uint32_t x = ((__shfl_sync(FULL, excl, i) | (self ? 1u << i : 0u)) >> eb) & gmask;
+        steps_mask |= (((x >> m) | (x << (G - m))) & gmask) << (16 / P * c);
+      }
     }
-    const float4 p1 = s_ipos[w][i1], p2 = s_ipos[w][i2];
-    const float2 l1 = s_ilj[w][i1], l2 = s_ilj[w][i2];
-    const float2 npx = make_float2(-p1.x, -p2.x), npy = make_float2(-p1.y, -p2.y),
-                 npz = make_float2(-p1.z, -p2.z);
-    const float2 qi = make_float2(p1.w, p2.w), sgi = make_float2(l1.x, l2.x),
-                 epi = make_float2(l1.y, l2.y);
-    float2 fx = x2::bc(0.f), fy = x2::bc(0.f), fz = x2::bc(0.f);
+    const ISlots<P> islots = load_slots<P>(s_ipos[w] + i0, s_ilj[w] + i0, G);
+    IForces<P> f = {};
     float fjx = 0.f, fjy = 0.f, fjz = 0.f;
     double e_tile = 0.0;
     double w_tile[6] = {0, 0, 0, 0, 0, 0};
@@ -289,96 +430,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
     auto steps = [&](auto image_tag) {
       constexpr bool kImage = decltype(image_tag)::value;
       uint32_t sm = steps_mask;
-      // 96 registers and no unrolling: at 80 registers the compiler re-read constants and
-      // lane-dependent values inside the loop (23,958-atom box: 62.9 -> 58.8 us)
-#pragma unroll 1
+#pragma unroll 1  // unrolled, the constants no longer stay in registers
       for (int k = 0; k < G; ++k) {
         const int jl = eb | ((m + k) & gm);
-        const float4 jxy = s_j[w][0][jl], jzq = s_j[w][1][jl], jse = s_j[w][2][jl];
-        float2 dx = x2::add(make_float2(jxy.x, jxy.y), npx);
-        float2 dy = x2::add(make_float2(jxy.z, jxy.w), npy);
-        float2 dz = x2::add(make_float2(jzq.x, jzq.y), npz);
-        if (kImage) {
-          min_image_fast(dx.x, dy.x, dz.x, a.box);
-          min_image_fast(dx.y, dy.y, dz.y, a.box);
-        }
-        const float2 r2 = x2::fma(dz, dz, x2::fma(dy, dy, x2::mul(dx, dx)));
-        bool u1 = (sm & 1u) == 0u, u2 = (sm & 0x10000u) == 0u;
+        pair_step<P, kElec, kTerms, kDump, kSwitch, kCutoff>(
+            a, s_j[w][0][jl], s_j[w][1][jl], s_j[w][2][jl], sm, 16 / P, kImage, self, s_atom[w] + jl,
+            s_iatom[w] + i0, G, islots, f, fjx, fjy, fjz, e_tile, w_tile);
         sm >>= 1;
-        if (kCutoff) {
-          bool in1 = r2.x < a.cutoff2, in2 = r2.y < a.cutoff2;
-          const float2 d = x2::add(r2, x2::bc(-a.cutoff2));
-          const bool b1 = fabsf(d.x) < a.band && u1, b2 = fabsf(d.y) < a.band && u2;
-          if (b1 | b2) {  // within the band: the reference's decision from the f64 positions
-            const int b = s_atom[w][jl];
-            if (b1) {
-              const int ia = s_iatom[w][i1];
-              in1 = ia >= 0 && b >= 0 &&
-                    exact_inside(a.pos, ia, b, a.periodic, a.box_exact, a.cutoff2_exact);
-            }
-            if (b2) {
-              const int ia = s_iatom[w][i2];
-              in2 = ia >= 0 && b >= 0 &&
-                    exact_inside(a.pos, ia, b, a.periodic, a.box_exact, a.cutoff2_exact);
-            }
-          }
-          u1 = u1 && in1;
-          u2 = u2 && in2;
-        }
-        if (kDump) {
-          const int b = s_atom[w][jl];
-          for (int h = 0; h < 2; ++h) {
-            const int ia = s_iatom[w][h ? i2 : i1];
-            if ((h ? u2 : u1) && ia >= 0 && b >= 0 && (!self || ia < b)) {
-              const unsigned long long slot = atomicAdd(a.pair_count, 1ull);
-              if ((long long)slot < a.pair_capacity) {
-                a.pair_dump[2 * slot] = ia < b ? ia : b;
-                a.pair_dump[2 * slot + 1] = ia < b ? b : ia;
-              }
-            }
-          }
-        }
-        float2 fo, en;
-        pair_terms_x2<kElec, kTerms, kSwitch>(
-            a, x2::select(u1, u2, r2, 1.f), x2::mul(make_float2(jzq.z, jzq.w), qi),
-            x2::add(make_float2(jse.x, jse.y), sgi), x2::mul(make_float2(jse.z, jse.w), epi), fo, en);
-        fo = x2::select(u1, u2, fo, 0.f);
-        fx = x2::fma(fo, dx, fx);
-        fy = x2::fma(fo, dy, fy);
-        fz = x2::fma(fo, dz, fz);
-        if (kTerms) {
-          const double scale = self ? 0.5 : 1.0;
-          if (u1) e_tile += scale * (double)en.x;
-          if (u2) e_tile += scale * (double)en.y;
-          if (kTerms > kTermsEnergy) {
-            const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
-            const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
-                         wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
-            if (u1) {
-              w_tile[0] -= scale * (double)wxx.x;
-              w_tile[1] -= scale * (double)wyy.x;
-              w_tile[2] -= scale * (double)wzz.x;
-              w_tile[3] -= scale * (double)wxy.x;
-              w_tile[4] -= scale * (double)wxz.x;
-              w_tile[5] -= scale * (double)wyz.x;
-            }
-            if (u2) {
-              w_tile[0] -= scale * (double)wxx.y;
-              w_tile[1] -= scale * (double)wyy.y;
-              w_tile[2] -= scale * (double)wzz.y;
-              w_tile[3] -= scale * (double)wxy.y;
-              w_tile[4] -= scale * (double)wxz.y;
-              w_tile[5] -= scale * (double)wyz.y;
-            }
-          }
-        }
         if (!self) {
-          fjx = fmaf(-fo.x, dx.x, fjx);
-          fjy = fmaf(-fo.x, dy.x, fjy);
-          fjz = fmaf(-fo.x, dz.x, fjz);
-          fjx = fmaf(-fo.y, dx.y, fjx);
-          fjy = fmaf(-fo.y, dy.y, fjy);
-          fjz = fmaf(-fo.y, dz.y, fjz);
           fjx = __shfl_sync(FULL, fjx, src);
           fjy = __shfl_sync(FULL, fjy, src);
           fjz = __shfl_sync(FULL, fjz, src);
@@ -389,19 +448,13 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
       steps(std::true_type{});
     else
       steps(std::false_type{});
-    // the two groups that met this lane's i-slots combine; the lane commits i-slot `lane`
-    fx.x += __shfl_xor_sync(FULL, fx.x, G);
-    fx.y += __shfl_xor_sync(FULL, fx.y, G);
-    fy.x += __shfl_xor_sync(FULL, fy.x, G);
-    fy.y += __shfl_xor_sync(FULL, fy.y, G);
-    fz.x += __shfl_xor_sync(FULL, fz.x, G);
-    fz.y += __shfl_xor_sync(FULL, fz.y, G);
-    const bool second = (lane & G) != 0;
+    // the groups that met the same i-slots combine; the lane commits i-slot `lane`
+    const float3 fi = reduce_groups(f, lane, G);
     const float fs = float(kForceScale);
     if (ai >= 0) {
-      add_fixed(a.force + ai, to_fixed(second ? fx.y : fx.x, fs));
-      add_fixed(a.force + a.n_atoms + ai, to_fixed(second ? fy.y : fy.x, fs));
-      add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(second ? fz.y : fz.x, fs));
+      add_fixed(a.force + ai, to_fixed(fi.x, fs));
+      add_fixed(a.force + a.n_atoms + ai, to_fixed(fi.y, fs));
+      add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(fi.z, fs));
     }
     if (!self && aj >= 0) {
       add_fixed(a.force + aj, to_fixed(fjx, fs));
@@ -440,7 +493,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_x2(const PairA
 // bounding box of the current positions of its half of I: no pair of such an entry can be
 // inside the cutoff, so the pair set is unchanged.  The surviving entries of each half queue in
 // a ring in shared memory; whenever both halves hold 16, a round runs the halves-tile steps
-// (groups of 8 lanes, two i-slots per lane) over 16 queued entries per half, and at the end of
+// (groups of 4 lanes, four i-slots per lane) over 16 queued entries per half, and at the end of
 // the sub-chunk the rest runs with dummy entries (masked for every i-slot) topping the rounds
 // up.  Each round commits its entries' forces; the i-forces accumulate over the sub-chunk and
 // are committed once.  Sub-chunks are fixed runs of a block's own tiles, whose order the
@@ -498,106 +551,24 @@ enum CullRound : int {
   kRoundSelf1 = 3,  // ... then with the other half
 };
 
-// One round: lane m of a group of 8 lanes meets the group's 8 entries, at ring slots
-// base + ((m + k) mod 8), with its i-slots i1 and i2, in 8 steps.  The entry's force rotates
+// One round: lane m of a group of 4 lanes meets the group's 4 entries, at ring slots
+// base + ((m + k) mod 4), with its four i-slots i + 4 c, in 4 steps.  The entry's force rotates
 // one lane per step and ends in the lane whose m is the entry's position (self rounds keep no
-// entry forces: every pair is met from both sides, at half energy).
+// entry forces: every pair is met from both sides, at half energy).  Four i-slots per lane for the
+// reasons given at the tile kernel; 255,477 particles: 398 us per launch with two, 390 with four.
 template <int kElec, int kTerms, bool kDump, bool kSwitch>
 __device__ __forceinline__ void cull_steps(const PairArgs<float>& a, const CullRing& r, int base,
-                                           int m, int src, int i1, int i2, bool image, bool self,
-                                           float2 npx, float2 npy, float2 npz, float2 qi,
-                                           float2 sgi, float2 epi, float2& fx, float2& fy,
-                                           float2& fz, float& fjx, float& fjy, float& fjz,
-                                           double& e_acc, double (&w_acc)[6]) {
+                                           int m, int src, int i, bool image, bool self,
+                                           const ISlots<2>& q, IForces<2>& f, float& fjx,
+                                           float& fjy, float& fjz, double& e_acc, double (&w_acc)[6]) {
   constexpr unsigned FULL = 0xffffffffu;
 #pragma unroll 1
-  for (int k = 0; k < 8; ++k) {
-    const int jf = base + ((m + k) & 7);
-    const float4 jxy = r.j[0][jf], jzq = r.j[1][jf], jse = r.j[2][jf];
-    const uint32_t em = r.em[jf];
-    float2 dx = x2::add(make_float2(jxy.x, jxy.y), npx);
-    float2 dy = x2::add(make_float2(jxy.z, jxy.w), npy);
-    float2 dz = x2::add(make_float2(jzq.x, jzq.y), npz);
-    if (image) {
-      min_image_fast(dx.x, dy.x, dz.x, a.box);
-      min_image_fast(dx.y, dy.y, dz.y, a.box);
-    }
-    const float2 r2 = x2::fma(dz, dz, x2::fma(dy, dy, x2::mul(dx, dx)));
-    bool u1 = ((em >> i1) & 1u) == 0u, u2 = ((em >> i2) & 1u) == 0u;
-    {
-      bool in1 = r2.x < a.cutoff2, in2 = r2.y < a.cutoff2;
-      const float2 d = x2::add(r2, x2::bc(-a.cutoff2));
-      const bool c1 = fabsf(d.x) < a.band && u1, c2 = fabsf(d.y) < a.band && u2;
-      if (c1 | c2) {  // within the band: the reference's decision from the f64 positions
-        const int b = r.at[jf];
-        if (c1) {
-          const int ia = r.iatom[i1];
-          in1 = ia >= 0 && b >= 0 &&
-                exact_inside(a.pos, ia, b, a.periodic, a.box_exact, a.cutoff2_exact);
-        }
-        if (c2) {
-          const int ia = r.iatom[i2];
-          in2 = ia >= 0 && b >= 0 &&
-                exact_inside(a.pos, ia, b, a.periodic, a.box_exact, a.cutoff2_exact);
-        }
-      }
-      u1 = u1 && in1;
-      u2 = u2 && in2;
-    }
-    if (kDump) {
-      const int b = r.at[jf];
-      for (int hh = 0; hh < 2; ++hh) {
-        const int ia = r.iatom[hh ? i2 : i1];
-        if ((hh ? u2 : u1) && ia >= 0 && b >= 0 && (!self || ia < b)) {
-          const unsigned long long slot = atomicAdd(a.pair_count, 1ull);
-          if ((long long)slot < a.pair_capacity) {
-            a.pair_dump[2 * slot] = ia < b ? ia : b;
-            a.pair_dump[2 * slot + 1] = ia < b ? b : ia;
-          }
-        }
-      }
-    }
-    float2 fo, en;
-    pair_terms_x2<kElec, kTerms, kSwitch>(
-        a, x2::select(u1, u2, r2, 1.f), x2::mul(make_float2(jzq.z, jzq.w), qi),
-        x2::add(make_float2(jse.x, jse.y), sgi), x2::mul(make_float2(jse.z, jse.w), epi), fo, en);
-    fo = x2::select(u1, u2, fo, 0.f);
-    fx = x2::fma(fo, dx, fx);
-    fy = x2::fma(fo, dy, fy);
-    fz = x2::fma(fo, dz, fz);
-    if (kTerms) {
-      const double scale = self ? 0.5 : 1.0;
-      if (u1) e_acc += scale * (double)en.x;
-      if (u2) e_acc += scale * (double)en.y;
-      if (kTerms > kTermsEnergy) {
-        const float2 fdx = x2::mul(fo, dx), fdy = x2::mul(fo, dy), fdz = x2::mul(fo, dz);
-        const float2 wxx = x2::mul(fdx, dx), wyy = x2::mul(fdy, dy), wzz = x2::mul(fdz, dz),
-                     wxy = x2::mul(fdx, dy), wxz = x2::mul(fdx, dz), wyz = x2::mul(fdy, dz);
-        if (u1) {
-          w_acc[0] -= scale * (double)wxx.x;
-          w_acc[1] -= scale * (double)wyy.x;
-          w_acc[2] -= scale * (double)wzz.x;
-          w_acc[3] -= scale * (double)wxy.x;
-          w_acc[4] -= scale * (double)wxz.x;
-          w_acc[5] -= scale * (double)wyz.x;
-        }
-        if (u2) {
-          w_acc[0] -= scale * (double)wxx.y;
-          w_acc[1] -= scale * (double)wyy.y;
-          w_acc[2] -= scale * (double)wzz.y;
-          w_acc[3] -= scale * (double)wxy.y;
-          w_acc[4] -= scale * (double)wxz.y;
-          w_acc[5] -= scale * (double)wyz.y;
-        }
-      }
-    }
+  for (int k = 0; k < 4; ++k) {
+    const int jf = base + ((m + k) & 3);
+    pair_step<2, kElec, kTerms, kDump, kSwitch, true>(
+        a, r.j[0][jf], r.j[1][jf], r.j[2][jf], r.em[jf] >> i, 4, image, self, r.at + jf, r.iatom + i,
+        4, q, f, fjx, fjy, fjz, e_acc, w_acc);
     if (!self) {
-      fjx = fmaf(-fo.x, dx.x, fjx);
-      fjy = fmaf(-fo.x, dy.x, fjy);
-      fjz = fmaf(-fo.x, dz.x, fjz);
-      fjx = fmaf(-fo.y, dx.y, fjx);
-      fjy = fmaf(-fo.y, dy.y, fjy);
-      fjz = fmaf(-fo.y, dz.y, fjz);
       fjx = __shfl_sync(FULL, fjx, src);
       fjy = __shfl_sync(FULL, fjy, src);
       fjz = __shfl_sync(FULL, fjz, src);
@@ -606,7 +577,7 @@ __device__ __forceinline__ void cull_steps(const PairArgs<float>& a, const CullR
 }
 
 template <int kElec, int kTerms, bool kDump, bool kSwitch>
-__global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const PairArgs<float> a) {
+__global__ void __launch_bounds__(32 * kPairWarps, 4) pair_kernel_cull(const PairArgs<float> a) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ CullRing s_ring[kPairWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -619,11 +590,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
   const float4* posq = reinterpret_cast<const float4*>(a.posq);
   const float2* ljp = reinterpret_cast<const float2*>(a.ljp);
   const float4* entries = reinterpret_cast<const float4*>(a.entries);
-  // rounds: groups of 8 lanes (gsub: the group's first entry within its half's 16); lane m of
-  // a group meets i-slots i1 = 16 h + m and i2 = i1 + 8 of its half h
-  const int h = lane >> 4, m = lane & 7, gsub = lane & 8;
-  const int i1 = (lane & 16) + m, i2 = i1 + 8;
-  const int src8 = (lane & ~7) | ((m + 1) & 7);
+  // rounds: groups of 4 lanes (gsub: the group's first entry within its half's 16); lane m of
+  // a group meets i-slots i0 + 4 c, i0 = 16 h + m, of its half h
+  const int h = lane >> 4, m = lane & 3, gsub = lane & 12;
+  const int i0 = (lane & 16) + m;
+  const int src4 = (lane & ~3) | ((m + 1) & 3);
   const float fs = float(kForceScale);
   long long e_fixed = 0;
   long long w_fixed[6] = {0, 0, 0, 0, 0, 0};
@@ -645,17 +616,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
       rg.iatom[lane] = a.sorted_atom[si];
     }
     __syncwarp();
-    float2 npx, npy, npz, qi, sgi, epi;
-    {
-      const float4 p1 = rg.ipos[i1], p2 = rg.ipos[i2];
-      const float2 l1 = rg.ilj[i1], l2 = rg.ilj[i2];
-      npx = make_float2(-p1.x, -p2.x);
-      npy = make_float2(-p1.y, -p2.y);
-      npz = make_float2(-p1.z, -p2.z);
-      qi = make_float2(p1.w, p2.w);
-      sgi = make_float2(l1.x, l2.x);
-      epi = make_float2(l1.y, l2.y);
-    }
+    const ISlots<2> islots = load_slots<2>(rg.ipos + i0, rg.ilj + i0, 4);
     {  // bounding box of the real particles of each half (empty: nothing is kept)
       const float4 pi = rg.ipos[lane];
       const bool real = rg.iatom[lane] >= 0;
@@ -678,7 +639,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
       }
       __syncwarp();
     }
-    float2 fx = x2::bc(0.f), fy = x2::bc(0.f), fz = x2::bc(0.f);
+    IForces<2> f = {};
     double e_acc = 0.0;
     double w_acc[6] = {0, 0, 0, 0, 0, 0};
     int hd0 = 0, tl0 = 0, hd1 = 0, tl1 = 0;  // ring cursors per half (heads: multiples of 16)
@@ -716,8 +677,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
                                              : kRing * (h ^ (mode == kRoundSelf1)) + gsub;
         float fjx = 0.f, fjy = 0.f, fjz = 0.f;
         cull_steps<kElec, kTerms, kDump, kSwitch>(
-            a, rg, base, m, src8, i1, i2, mode == kRoundImage || (self && staged_image), self,
-            npx, npy, npz, qi, sgi, epi, fx, fy, fz, fjx, fjy, fjz, e_acc, w_acc);
+            a, rg, base, m, src4, i0, mode == kRoundImage || (self && staged_image), self, islots, f,
+            fjx, fjy, fjz, e_acc, w_acc);
         ++n_rounds;
         if (!self) {
           const int aj = rg.at[base + m];
@@ -802,20 +763,14 @@ __global__ void __launch_bounds__(32 * kPairWarps, 5) pair_kernel_cull(const Pai
       ent = ent_n;
       xw = xw_n;
     }
-    // the two groups of each half met the same i-slots; the lane commits i-slot `lane`
-    fx.x += __shfl_xor_sync(FULL, fx.x, 8);
-    fx.y += __shfl_xor_sync(FULL, fx.y, 8);
-    fy.x += __shfl_xor_sync(FULL, fy.x, 8);
-    fy.y += __shfl_xor_sync(FULL, fy.y, 8);
-    fz.x += __shfl_xor_sync(FULL, fz.x, 8);
-    fz.y += __shfl_xor_sync(FULL, fz.y, 8);
+    // the four groups of each half met the same i-slots; the lane commits i-slot `lane`
+    const float3 fi = reduce_groups(f, lane, 4);
     if (lane == 0) atomicAdd(a.cull_rounds, (unsigned long long)n_rounds);
     const int ai = rg.iatom[lane];
     if (ai >= 0) {
-      const bool second = gsub != 0;
-      add_fixed(a.force + ai, to_fixed(second ? fx.y : fx.x, fs));
-      add_fixed(a.force + a.n_atoms + ai, to_fixed(second ? fy.y : fy.x, fs));
-      add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(second ? fz.y : fz.x, fs));
+      add_fixed(a.force + ai, to_fixed(fi.x, fs));
+      add_fixed(a.force + a.n_atoms + ai, to_fixed(fi.y, fs));
+      add_fixed(a.force + 2 * a.n_atoms + ai, to_fixed(fi.z, fs));
     }
     if (kTerms) {
       for (int off = 16; off > 0; off >>= 1) {
@@ -904,7 +859,10 @@ void launch_pair(const PairArgs<Real>& a, int elec, int terms, bool dump, int gr
         return;                                                                     \
       }                                                                             \
     }                                                                               \
-    pair_kernel_x2<E, EN, D, SW><<<kPairWaves * grid, 32 * kPairWarps, 0, s>>>(a);  \
+    if (a.periodic)                                                                 \
+      pair_kernel_x2<2, E, EN, D, SW><<<kPairWaves * grid, 32 * kPairWarps, 0, s>>>(a); \
+    else                                                                            \
+      pair_kernel_x2<1, E, EN, D, SW><<<kPairWaves * grid, 32 * kPairWarps, 0, s>>>(a); \
   } else                                                                            \
     pair_kernel<Real, E, EN, D, SW><<<kPairWaves * grid, 32 * kPairWarps, 0, s>>>(a)
 #define OMMB200_PAIR_SW(E, EN, D)     \

@@ -18,7 +18,6 @@
 // follow unless the network's error is already within half the tolerance.  Until the next
 // judge the network's radii are used only if it passed (error below `tolerance`); otherwise
 // the exact passes run.
-#include "f32x2.cuh"
 #include "gb_math.cuh"
 #include "kernels.h"
 #include "pair_math.cuh"
@@ -29,15 +28,7 @@ namespace {
 using namespace gb;
 
 constexpr int kNF = kRadiiFeatures;
-constexpr int kFeatureWarps = 8;  // warps of a CTA of lr_features
-constexpr int kForceWarps = 4;    // ... of lr_forces
-// CTAs that share a block's neighbour list in lr_forces (list entries taken in turn).  With one,
-// three chains of 5,000 particles give 471 CTAs of 4 warps to 148 SMs, and the launch lasts as long
-// as the CTA of the block with the most neighbours: 92 us, and 65 with two CTAs, block pairs shared
-// evenly and packed arithmetic.  Four take 57 there, but 195 against 156 on sixteen chains, where
-// one CTA per block fills the SMs.  The number is fixed, so that a system's sums do not depend on
-// what is batched beside it.
-constexpr int kForceSplit = 2;
+constexpr int kWarps = 4;
 constexpr float kMu0 = 0.1f;               // first Gaussian centre (nm)
 constexpr float kDmu = 1.1f / 31.0f;       // centre spacing: 0.1 .. 1.2 nm
 constexpr float kEta = 1.0f / (2.0f * 0.07f * 0.07f);  // Gaussian width 0.07 nm
@@ -191,89 +182,63 @@ __device__ __forceinline__ void gauss_seeds(float r, float* ec, float* up, float
   *down = __expf(-a - b);
 }
 
-// Sums over pairs of scale e_f / Q_{|f - c|}: the side above the centre in pairs (c + 1 + 2 p,
-// c + 2 + 2 p), the side below in pairs (c - 1 - 2 p, c - 2 - 2 p); the constants Q join at the end.
-// Packed products and sums (two per pair of features) halve the instructions of the scalar form.
-struct GaussSums {
-  float centre = 0.f;
-  float2 up[8], down[8];
-};
-static_assert(kNF == 32 && kCentre == 15, "16 features above the centre, 15 below");
-
-__device__ __forceinline__ void add_gaussians(float r, float scale, GaussSums& G) {
+// G_f += scale e_f for all f.  Each side runs two products (odd and even steps, ratio U^2), which
+// halves the dependent chain.
+__device__ __forceinline__ void add_gaussians(float r, float scale, float* G) {
   float ec, up, down;
   gauss_seeds(r, &ec, &up, &down);
   const float v0 = ec * scale;
-  G.centre += v0;
+  G[kCentre] += v0;
   const float up2 = up * up, down2 = down * down;
-  float2 u = make_float2(v0 * up, v0 * up2), d = make_float2(v0 * down, v0 * down2);
+  float va = v0 * up, vb = v0 * up2;
 #pragma unroll
-  for (int p = 0; p < 8; ++p) {
-    G.up[p] = x2::add(G.up[p], u);
-    G.down[p] = x2::add(G.down[p], d);  // the last one's second lane is no feature
-    if (p < 7) {
-      u = x2::mul(u, x2::bc(up2));
-      d = x2::mul(d, x2::bc(down2));
-    }
+  for (int k = 1; kCentre + k < kNF; k += 2) {
+    G[kCentre + k] = fmaf(va, c_gauss_q[kCentre + k], G[kCentre + k]);
+    if (kCentre + k + 1 < kNF)
+      G[kCentre + k + 1] = fmaf(vb, c_gauss_q[kCentre + k + 1], G[kCentre + k + 1]);
+    va *= up2;
+    vb *= up2;
   }
-}
-// Feature f of the sums.
-__device__ __forceinline__ float gauss_sum(const GaussSums& G, int f) {
-  if (f == kCentre) return G.centre;
-  const int k = f > kCentre ? f - kCentre - 1 : kCentre - 1 - f;
-  const float2 v = f > kCentre ? G.up[k >> 1] : G.down[k >> 1];
-  return ((k & 1) ? v.y : v.x) * c_gauss_q[f];
+  va = v0 * down;
+  vb = v0 * down2;
+#pragma unroll
+  for (int k = 1; kCentre - k >= 0; k += 2) {
+    G[kCentre - k] = fmaf(va, c_gauss_q[kCentre - k], G[kCentre - k]);
+    if (kCentre - k - 1 >= 0)
+      G[kCentre - k - 1] = fmaf(vb, c_gauss_q[kCentre - k - 1], G[kCentre - k - 1]);
+    va *= down2;
+    vb *= down2;
+  }
 }
 
-// Weights A_f in the order weighted_gaussians reads them: pair k < 15 holds (A_{c + 1 + k},
-// A_{c - 1 - k}), pair 15 (A_31, A_c).
-__device__ __forceinline__ constexpr int weight_feature(int at) {
-  const int k = at >> 1;
-  return k == 15 ? ((at & 1) ? kCentre : kNF - 1) : ((at & 1) ? kCentre - 1 - k : kCentre + 1 + k);
-}
-// A_f = scale dtail_f Q_{|f - c|} of a particle's row, four in that order at a time.
-template <class Store>
-__device__ __forceinline__ void load_weights(const float* dtail, float scale, Store store) {
-  const float4* row = reinterpret_cast<const float4*>(dtail);
-  float v[kNF];
-#pragma unroll
-  for (int q = 0; q < kNF / 4; ++q) {
-    const float4 x = row[q];
-    v[4 * q] = x.x;
-    v[4 * q + 1] = x.y;
-    v[4 * q + 2] = x.z;
-    v[4 * q + 3] = x.w;
-  }
-  auto weight = [&](int at) { return scale * v[weight_feature(at)] * c_gauss_q[weight_feature(at)]; };
-#pragma unroll
-  for (int q = 0; q < kNF / 4; ++q)
-    store(q, make_float4(weight(4 * q), weight(4 * q + 1), weight(4 * q + 2), weight(4 * q + 3)));
+__device__ __forceinline__ float component(const float4& v, int c) {
+  return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
 }
 
 // s0 = sum_f W_f e_f and t = sum_f W_f e_f mu_f for the pair weights W_f = W_if + W_jf, given
-// premultiplied as A_f = W_f Q_{|f - c|} in load_weights' order (own part wq in registers, the
-// partner's sq as a 16-byte aligned shared row).  With e_{c +- k} = e_c U_+-^k Q_k, U = U_+, D = U_-:
+// premultiplied as A_f = W_f Q_{|f - c|} (own part wq in registers, the partner's sq as 16-byte
+// aligned shared rows).  With e_{c +- k} = e_c U_+-^k Q_k, U = U_+, D = U_-:
 //   s0 = e_c S,  S = A_c + U P_+(U) + D P_-(D),  P_+(U) = sum_{k>=1} A_{c+k} U^(k-1)  (likewise P_-),
 //   t  = e_c (mu_c S + dmu (U (P_+ + U P_+') - D (P_- + D P_-'))),
-// the two polynomials and their derivatives by Horner's rule in the lanes of packed values: three
-// instructions per two features, half of the scalar form's.
-__device__ __forceinline__ void weighted_gaussians(float r, const float2* wq, const float4* sq,
+// the polynomials and their derivatives by Horner's rule: three operations per feature.
+__device__ __forceinline__ void weighted_gaussians(float r, const float* wq, const float4* sq,
                                                    float* s0, float* t) {
   float ec, up, down;
   gauss_seeds(r, &ec, &up, &down);
-  const float2 u = make_float2(up, down);
-  const float4 last = sq[7];
-  const float2 ends = x2::add(wq[15], make_float2(last.z, last.w));  // A_31, A_c
-  float2 p = make_float2(ends.x, 0.f), d = x2::bc(0.f);
+  float pu = wq[kNF - 1] + component(sq[(kNF - 1) >> 2], (kNF - 1) & 3), du = 0.f;
 #pragma unroll
-  for (int k = 14; k >= 0; --k) {
-    const float4 row = sq[k >> 1];
-    const float2 c = x2::add(wq[k], (k & 1) ? make_float2(row.z, row.w) : make_float2(row.x, row.y));
-    d = x2::fma(d, u, p);
-    p = x2::fma(p, u, c);
+  for (int f = kNF - 2; f > kCentre; --f) {
+    du = fmaf(du, up, pu);
+    pu = fmaf(pu, up, wq[f] + component(sq[f >> 2], f & 3));
   }
-  const float sum = ends.y + up * p.x + down * p.y;
-  const float moment = up * fmaf(up, d.x, p.x) - down * fmaf(down, d.y, p.y);
+  float pd = wq[0] + component(sq[0], 0), dd = 0.f;
+#pragma unroll
+  for (int f = 1; f < kCentre; ++f) {
+    dd = fmaf(dd, down, pd);
+    pd = fmaf(pd, down, wq[f] + component(sq[f >> 2], f & 3));
+  }
+  const float sum = wq[kCentre] + component(sq[kCentre >> 2], kCentre & 3) + up * pu + down * pd;
+  const float moment = up * fmaf(up, du, pu) - down * fmaf(down, dd, pd);
   *s0 = ec * sum;
   *t = ec * fmaf(kMuC, sum, kDmu * moment);
 }
@@ -297,7 +262,6 @@ __device__ __forceinline__ float2 slot_par(const void* params, int s) {
 // filled in block order by a prefix over the chunk, so every run visits the same pairs in the
 // same order.
 constexpr int kChunk = 16;             // blocks of I's list per chunk
-constexpr int kWindow = 128;           // entries per half staged at a time by lr_features
 constexpr int kListCap = 32 * kChunk;  // entries per list per chunk
 enum : int { kNearA, kNearB, kFarA, kFarB };
 constexpr float kListMargin = 1e-4f;   // nm added to both cutoffs for the box tests
@@ -349,28 +313,20 @@ __device__ __forceinline__ float box_gap2(float3 p, float3 c, float3 h) {
   return gx * gx + gy * gy + gz * gz;
 }
 
-template <int kParts>
-__device__ __forceinline__ int part_size(int nn, int part) {
-  return (nn - part + kParts - 1) / kParts;
-}
-
-// Fills L with the entries of the blocks at q0 .. q0 + kChunk - 1 of this CTA's `part` of I's list
-// (every kParts-th block) and returns the number of blocks taken.  With `half` each pair of blocks is in the list of one of the two: of the lower
-// when I + J is even, of the higher when it is odd, so that every block has about half of its
-// neighbours (all pairs in the lower block's list left the first blocks' CTAs with twice the mean
-// and the last with none).  Ends with the CTA synchronised.
-template <class Real, int kWarps, int kParts>
-__device__ int build_entry_lists(const LearnedGbArgs& a, const GbArgs& g, int I, int part,
-                                 int q0, int nn, int n_near, bool half, EntryLists& L) {
+// Fills L with the entries of blocks q0 .. q0 + kChunk - 1 of I's list (blocks below I skipped
+// when `upper`) and returns the number of blocks taken.  Ends with the CTA synchronised.
+template <class Real>
+__device__ int build_entry_lists(const LearnedGbArgs& a, const GbArgs& g, int I, int q0, int nn,
+                                 int n_near, bool upper, EntryLists& L) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nq = min(kChunk, part_size<kParts>(nn, part) - q0);
+  const int nq = min(kChunk, nn - q0);
   const float rc_m = a.rc + kListMargin, rf_m = a.rf + kListMargin;
   const float rc2 = rc_m * rc_m, rf2 = rf_m * rf_m;
   for (int qq = w; qq < nq; qq += kWarps) {
     bool unused;
-    const int J = list_block(a, I, kParts * (q0 + qq) + part, n_near, &unused);
+    const int J = list_block(a, I, q0 + qq, n_near, &unused);
     bool in[4] = {false, false, false, false};
-    if (!(half && J != I && (J < I) != ((I + J) & 1))) {
+    if (!(upper && J < I)) {
       const int aj = g.slot_atom[32 * J + lane];
       const float4 p4 = slot_pos<Real>(g.posq, 32 * J + lane);
       if (aj >= 0) {
@@ -424,25 +380,19 @@ __device__ int build_entry_lists(const LearnedGbArgs& a, const GbArgs& g, int I,
   return nq;
 }
 
-// One CTA per block I, lane = particle i.  I's entries pass through shared memory a window at a time;
-// each warp takes every kWarps-th of them (whole tiles of 16 to a warp leave some warps with twice
-// the entries of others, where a half block has a few dozen), and the warps' partial sums meet in
-// shared memory in a fixed order.  Radial features (near entries, r < rf) and the switched
-// short-range integral (r < rc) over every particle j != i.
-//
-// The launch lasts as long as the CTA of the block with the most neighbours (twice the mean in a
-// loose chain): three chains of 5,000 particles took 71 us with four warps to a CTA and a tile of
-// entries to a warp, 45 us with eight and windows (six: 54).  Two CTAs to a block as a cluster took
-// 66 us and clusters of four 163: the launch of many small clusters is slow.
+// One CTA per block I, lane = particle i; the CTA's warps share I's entry lists (one tile of 16
+// entries per half at a time) and their partial sums meet in shared memory in a fixed order.
+// Radial features (near entries, r < rf) and the switched short-range integral (r < rc) over
+// every particle j != i.
 template <class Real>
-__global__ void __launch_bounds__(32 * kFeatureWarps, 3) lr_features(LearnedGbArgs a, GbArgs g) {
+__global__ void __launch_bounds__(32 * kWarps) lr_features(LearnedGbArgs a, GbArgs g) {
   if (!a.state->need) return;
-  constexpr int kWarps = kFeatureWarps;
   __shared__ EntryLists s_lists;
-  __shared__ float4 s_pos[2][kWindow];  // per half: xyz, slot as int bits (-1: no entry)
-  __shared__ float s_scaled[2][kWindow];
+  __shared__ float4 s_pos[kWarps][32];  // xyz, slot as int bits (-1: no entry)
+  __shared__ float s_scaled[kWarps][32];
   __shared__ float s_red[kWarps][32][kNF + 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int hbase = lane & 16;
   const float rc2 = a.rc * a.rc, rf2 = a.rf * a.rf;
   const float fc_k = kPiF / a.rf;
   for (int I = blockIdx.x; I < a.n_blocks; I += gridDim.x) {
@@ -456,86 +406,86 @@ __global__ void __launch_bounds__(32 * kFeatureWarps, 3) lr_features(LearnedGbAr
       if (threadIdx.x == 0) s_lists.box = boxes;
     }
     __syncthreads();
-    GaussSums G;
+    float G[kNF];
 #pragma unroll
-    for (int p = 0; p < 8; ++p) G.up[p] = G.down[p] = x2::bc(0.f);
+    for (int f = 0; f < kNF; ++f) G[f] = 0.f;
     float ishort = 0.f;
     const int n_near = a.nbr_count[2 * I], nn = n_near + a.nbr_count[2 * I + 1];
     for (int q0 = 0; q0 < nn; q0 += kChunk) {
-      const int nq = build_entry_lists<Real, kWarps, 1>(a, g, I, 0, q0, nn, n_near, false, s_lists);
-      for (int near = 1; near >= 0; --near) {
-        const int list = near ? kNearA : kFarA;
-        const int n_a = s_lists.pre[list][nq], n_b = s_lists.pre[list + 1][nq];
-        for (int e0 = 0; e0 < max(n_a, n_b); e0 += kWindow) {
-          const int n_window = min(kWindow, max(n_a, n_b) - e0);
-          for (int t = threadIdx.x; t < 2 * kWindow; t += 32 * kWarps) {
-            const int h = t / kWindow, e = t % kWindow;
-            const int slot = e0 + e < (h ? n_b : n_a) ? s_lists.slot[list + h][e0 + e] : -1;
-            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (slot >= 0) {
-              p = slot_pos<Real>(g.posq, slot);
-              s_scaled[h][e] = slot_par<Real>(g.params, slot).y;
-            }
-            p.w = __int_as_float(slot);
-            s_pos[h][e] = p;
-          }
-          __syncthreads();
-          if (ai >= 0) {
-#pragma unroll 2
-            for (int e = w; e < n_window; e += kWarps) {
-              const float4 pj = s_pos[lane >> 4][e];
-              const int sj = __float_as_int(pj.w);
-              if (sj < 0 || sj == si) continue;
-              const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-              const float r2 = dx * dx + dy * dy + dz * dz;
-              if (r2 >= rc2) continue;
-              const float inv_r = rsqrt_r(r2), r = r2 * inv_r;
-              float ds;
-              const float sw = switch_value(r, a.rs, a.rc, &ds);
-              const float h = descreening_fast(off_i, s_scaled[lane >> 4][e], r, inv_r);
-              ishort = fmaf(h, sw, ishort);
-              if (!near || r2 >= rf2) continue;
-              const float fc = 0.5f * (__cosf(fc_k * r) + 1.f);  // SFU cosine
-              add_gaussians(r, fc, G);
-            }
-          }
-          __syncthreads();  // the next window
+      const int nq = build_entry_lists<Real>(a, g, I, q0, nn, n_near, false, s_lists);
+      const int n_na = s_lists.pre[kNearA][nq], n_nb = s_lists.pre[kNearB][nq];
+      const int n_fa = s_lists.pre[kFarA][nq], n_fb = s_lists.pre[kFarB][nq];
+      const int t_near = (max(n_na, n_nb) + 15) >> 4, t_far = (max(n_fa, n_fb) + 15) >> 4;
+      for (int t = w; t < t_near + t_far; t += kWarps) {
+        const bool near = t < t_near;  // uniform over the warp
+        const int list = (near ? kNearA : kFarA) + (lane >> 4);
+        const int e = 16 * (near ? t : t - t_near) + (lane & 15);
+        const int slot = e < s_lists.pre[list][nq] ? s_lists.slot[list][e] : -1;
+        if (slot >= 0) {
+          const float4 p = slot_pos<Real>(g.posq, slot);
+          s_pos[w][lane] = make_float4(p.x, p.y, p.z, __int_as_float(slot));
+          s_scaled[w][lane] = slot_par<Real>(g.params, slot).y;
+        } else {
+          s_pos[w][lane] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+          s_scaled[w][lane] = 0.f;
         }
+        __syncwarp();
+        if (ai >= 0) {
+#pragma unroll 2
+          for (int k = 0; k < 16; ++k) {
+            const int jl = hbase | ((lane + k) & 15);
+            const float4 pj = s_pos[w][jl];
+            const int sj = __float_as_int(pj.w);
+            if (sj < 0 || sj == si) continue;
+            const float dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            if (r2 >= rc2) continue;
+            const float inv_r = rsqrt_r(r2), r = r2 * inv_r;
+            float ds, h, gr;
+            const float sw = switch_value(r, a.rs, a.rc, &ds);
+            descreening_fast(off_i, s_scaled[w][jl], r, inv_r, &h, &gr);
+            ishort = fmaf(h, sw, ishort);
+            if (!near || r2 >= rf2) continue;
+            const float fc = 0.5f * (__cosf(fc_k * r) + 1.f);  // SFU cosine
+            add_gaussians(r, fc, G);
+          }
+        }
+        __syncwarp();
       }
+      __syncthreads();  // the next chunk refills the lists
     }
 #pragma unroll
-    for (int f = 0; f < kNF; ++f) s_red[w][lane][f] = gauss_sum(G, f);
+    for (int f = 0; f < kNF; ++f) s_red[w][lane][f] = G[f];
     s_red[w][lane][kNF] = ishort;
     __syncthreads();
-    if (ai >= 0) {  // the features in groups of four, a group to a warp
-      auto total = [&](int f) {
-        float t = s_red[0][lane][f];
-#pragma unroll
-        for (int u = 1; u < kWarps; ++u) t += s_red[u][lane][f];
-        return t;
-      };
+    if (w == 0 && ai >= 0) {
       float4* out = reinterpret_cast<float4*>(a.features + (size_t)ai * kNF);
-      for (int q = w; q < kNF / 4; q += kWarps)
-        out[q] = make_float4(total(4 * q), total(4 * q + 1), total(4 * q + 2), total(4 * q + 3));
-      if (w == kWarps - 1) a.short_sum[ai] = to_fixed((double)total(kNF), kBornScale);
+      float v[kNF + 1];
+#pragma unroll
+      for (int f = 0; f <= kNF; ++f) {
+        float t = s_red[0][lane][f];
+        for (int u = 1; u < kWarps; ++u) t += s_red[u][lane][f];
+        v[f] = t;
+      }
+#pragma unroll
+      for (int f = 0; f < kNF / 4; ++f)
+        out[f] = make_float4(v[4 * f], v[4 * f + 1], v[4 * f + 2], v[4 * f + 3]);
+      a.short_sum[ai] = to_fixed((double)v[kNF], kBornScale);
     }
     __syncthreads();
   }
 }
 
-// kForceSplit CTAs per block I, each committing its own sums; lane = particle i, and the warps share
-// I's entries (one tile of 16 per half at a time):
-//   F_i = sum_j (D_i Phi'_ij + D_j Phi'_ji) / r d_ij,
+// One CTA per block I as above: F_i = sum_j (D_i Phi'_ij + D_j Phi'_ji) / r d_ij,
 // Phi_ij = H(r; i, j) S(r) + sum_f (d tail_i / d G_if) g_f(r), D = dE/dI (half the chain
 // value the GB chain kernel leaves per slot).  The pair term is symmetric in i and j, so each
-// pair is done once, from one of the two blocks (build_entry_lists): the force on each
+// pair is done once, from the lower block (entries of blocks J >= I only): the force on each
 // entry travels with it one lane per warp shuffle within its half and is committed in fixed
 // point after the 16 steps; pairs inside block I are visited from both sides and keep their
 // i-forces only.
 template <class Real>
-__global__ void __launch_bounds__(32 * kForceWarps, 5) lr_forces(LearnedGbArgs a, GbArgs g) {
+__global__ void __launch_bounds__(32 * kWarps, 5) lr_forces(LearnedGbArgs a, GbArgs g) {
   if (!a.state->use_learned) return;
-  constexpr int kWarps = kForceWarps;
   __shared__ EntryLists s_lists;
   __shared__ float4 s_pos[kWarps][32];        // xyz, slot as int bits (-1: no entry)
   __shared__ float4 s_par[kWarps][32];        // offset radius, scaled radius, D
@@ -549,25 +499,29 @@ __global__ void __launch_bounds__(32 * kForceWarps, 5) lr_forces(LearnedGbArgs a
   const Real* chain = reinterpret_cast<const Real*>(g.dedr_slot);
   const float fc_k = kPiF / a.rf;
   const float fscale = (float)kForceScale;
-  const int part = blockIdx.x % kForceSplit;
-  for (int I = blockIdx.x / kForceSplit; I < a.n_blocks; I += gridDim.x / kForceSplit) {
+  for (int I = blockIdx.x; I < a.n_blocks; I += gridDim.x) {
     const int si = 32 * I + lane;
     const int ai = g.slot_atom[si];
     const float4 p4 = slot_pos<Real>(g.posq, si);
     const float3 pi = make_float3(p4.x, p4.y, p4.z);
     float off_i = 1.f, sc_i = 0.f, d_i = 0.f;
-    float2 wi[kNF / 2];  // D_i d tail_i / d G_if, times Q_{|f - c|}
+    float wi[kNF];  // D_i d tail_i / d G_if, times Q_{|f - c|}
 #pragma unroll
-    for (int k = 0; k < kNF / 2; ++k) wi[k] = x2::bc(0.f);
+    for (int f = 0; f < kNF; ++f) wi[f] = 0.f;
     if (ai >= 0) {
       const float2 par = slot_par<Real>(g.params, si);
       off_i = par.x;
       sc_i = par.y;
       d_i = 0.5f * (float)chain[si];
-      load_weights(a.dtail + (size_t)ai * kNF, d_i, [&](int q, float4 v) {
-        wi[2 * q] = make_float2(v.x, v.y);
-        wi[2 * q + 1] = make_float2(v.z, v.w);
-      });
+      const float4* dt = reinterpret_cast<const float4*>(a.dtail + (size_t)ai * kNF);
+#pragma unroll
+      for (int qq = 0; qq < kNF / 4; ++qq) {
+        const float4 v = dt[qq];
+        wi[4 * qq] = d_i * v.x * c_gauss_q[4 * qq];
+        wi[4 * qq + 1] = d_i * v.y * c_gauss_q[4 * qq + 1];
+        wi[4 * qq + 2] = d_i * v.z * c_gauss_q[4 * qq + 2];
+        wi[4 * qq + 3] = d_i * v.w * c_gauss_q[4 * qq + 3];
+      }
     }
     {
       const HalfBoxes boxes = half_boxes(pi, ai >= 0);
@@ -576,8 +530,8 @@ __global__ void __launch_bounds__(32 * kForceWarps, 5) lr_forces(LearnedGbArgs a
     __syncthreads();
     float fx = 0.f, fy = 0.f, fz = 0.f;
     const int n_near = a.nbr_count[2 * I], nn = n_near + a.nbr_count[2 * I + 1];
-    for (int q0 = 0; q0 < part_size<kForceSplit>(nn, part); q0 += kChunk) {
-      const int nq = build_entry_lists<Real, kWarps, kForceSplit>(a, g, I, part, q0, nn, n_near, true, s_lists);
+    for (int q0 = 0; q0 < nn; q0 += kChunk) {
+      const int nq = build_entry_lists<Real>(a, g, I, q0, nn, n_near, true, s_lists);
       const int n_na = s_lists.pre[kNearA][nq], n_nb = s_lists.pre[kNearB][nq];
       const int n_fa = s_lists.pre[kFarA][nq], n_fb = s_lists.pre[kFarB][nq];
       const int t_near = (max(n_na, n_nb) + 15) >> 4, t_far = (max(n_fa, n_fb) + 15) >> 4;
@@ -595,8 +549,14 @@ __global__ void __launch_bounds__(32 * kForceWarps, 5) lr_forces(LearnedGbArgs a
           s_pos[w][lane] = make_float4(p.x, p.y, p.z, __int_as_float(slot));
           s_par[w][lane] = make_float4(par.x, par.y, dj, 0.f);
           if (near) {
+            const float4* dt = reinterpret_cast<const float4*>(a.dtail + (size_t)aj * kNF);
             float4* row = reinterpret_cast<float4*>(s_w[w][lane]);
-            load_weights(a.dtail + (size_t)aj * kNF, dj, [&](int q, float4 v) { row[q] = v; });
+#pragma unroll
+            for (int qq = 0; qq < kNF / 4; ++qq) {
+              const float4 v = dt[qq];
+              row[qq] = make_float4(dj * v.x * c_gauss_q[4 * qq], dj * v.y * c_gauss_q[4 * qq + 1],
+                                    dj * v.z * c_gauss_q[4 * qq + 2], dj * v.w * c_gauss_q[4 * qq + 3]);
+            }
           }
         } else {
           s_pos[w][lane] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
@@ -797,21 +757,21 @@ template <class Real>
 void launch_learned_phase(const LearnedGbArgs& a, const GbArgs& g, int phase, int sm_count,
                           cudaStream_t s) {
   const int wb = ceil_div(a.n_blocks * 32, 128);
-  const int ctas = std::max(1, a.n_blocks);  // per part: the scheduler balances uneven lists
+  const int ctas = std::max(1, a.n_blocks);  // one CTA per block: the scheduler balances uneven lists
   switch (phase) {
     case kLrLists:
       lr_boxes<<<wb, 128, 0, s>>>(a, g);
       lr_neighbors<<<wb, 128, 0, s>>>(a);
       break;
     case kLrFeatures:
-      lr_features<Real><<<ctas, 32 * kFeatureWarps, 0, s>>>(a, g);
+      lr_features<Real><<<ctas, 32 * kWarps, 0, s>>>(a, g);
       break;
     case kLrInfer:
       launch_mlp_infer(a.n_atoms, a.features, a.params, a.tail, a.dtail, a.status, sm_count, s,
                        &a.state->need);
       break;
     case kLrForces:
-      lr_forces<Real><<<kForceSplit * ctas, 32 * kForceWarps, 0, s>>>(a, g);
+      lr_forces<Real><<<ctas, 32 * kWarps, 0, s>>>(a, g);
       break;
     case kLrJudge:
       lr_judge<<<ceil_div(a.n_atoms, 256), 256, 0, s>>>(a, g);
